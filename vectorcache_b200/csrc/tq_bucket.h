@@ -183,7 +183,7 @@ struct BucketScanArgs {
 // `grid`: a bound of the item count; the launch runs min(grid, resident CTAs).
 cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStream_t stream);
 // floor[q] = the k-th largest score (above -inf) among the first count[q]
-// candidates of query q's region (cand + q * stride), -inf when there are
+// (count null: all `stride`) candidates of query q's region (cand + q * stride), -inf when there are
 // fewer than k: the k-th score of their merged top k, a lower bound of the
 // k-th best over all probes.
 cudaError_t launch_kth_floor(const float* cand, long long stride, const uint32_t* count, long long nq, int k,

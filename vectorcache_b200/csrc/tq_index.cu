@@ -197,7 +197,7 @@ int tq_index_create(size_t dim, size_t bits, uint32_t flags, int device, tq_inde
     h->d_perm_sign.reserve(dim * 4);
     h->d_bnd.reserve(64);
     h->d_cen.reserve(64);
-    h->d_counter.reserve(8);
+    h->d_counter.reserve(16);  // replay count, wait status
     h->upload(h->d_perm_sign.get(), ps.data(), dim * 4);
     h->upload(h->d_bnd.get(), bnd.data(), 64);
     h->upload(h->d_cen.get(), cen.data(), 64);
@@ -211,7 +211,7 @@ int tq_index_create(size_t dim, size_t bits, uint32_t flags, int device, tq_inde
       h->upload(h->d_grid.get(), cells.data(), cells.size() * 4);
       h->has_grid = true;
     }
-    vcb::check(cudaMemsetAsync(h->d_counter.get(), 0, 8, h->stream), "cudaMemsetAsync");
+    vcb::check(cudaMemsetAsync(h->d_counter.get(), 0, 16, h->stream), "cudaMemsetAsync");
     h->sync();
     *out = h.release();
   });

@@ -14,6 +14,7 @@
 #include "../../include/vectorcache_b200.h"
 #include "tq_abi.h"
 #include "tq_host_math.h"
+#include "tq_bucket.h"
 #include "tq_kernels.h"
 
 namespace vcb {
@@ -138,15 +139,18 @@ struct FlatScratch {
   DeviceBuffer* cand_i;
   DeviceBuffer* partial = nullptr;  // nullptr: the scan does not split
   long long range_cap = 0;          // > 0: at most this many vectors per scan CTA
+  DeviceBuffer* onehot = nullptr;   // nullptr: batches stay on the lookup scan
 };
 
 // Owning variant for callers that run searches concurrently (one per stream).
 struct FlatScratchStore {
-  DeviceBuffer luts, qf, cand_s, cand_i, partial;
+  DeviceBuffer luts, qf, cand_s, cand_i, partial, onehot;
   long long range_cap = 0;  // see FlatScratch::range_cap
-  FlatScratch ref() { return {&luts, &qf, &cand_s, &cand_i, &partial, range_cap}; }
+  // Searches that bound a CTA's vectors (the server's) keep the lookup scan:
+  // the one-hot kernel holds its SMs for the whole search.
+  FlatScratch ref() { return {&luts, &qf, &cand_s, &cand_i, &partial, range_cap, range_cap > 0 ? nullptr : &onehot}; }
   void bind(ScratchArena* a) {
-    for (DeviceBuffer* b : {&luts, &qf, &cand_s, &cand_i, &partial}) b->bind(a);
+    for (DeviceBuffer* b : {&luts, &qf, &cand_s, &cand_i, &partial, &onehot}) b->bind(a);
   }
 };
 
@@ -178,7 +182,11 @@ struct tq_index {
   vcb::DeviceBuffer d_perm_sign, d_bnd, d_cen, d_grid, d_shift, d_scale, d_inv_scale;
   vcb::DeviceBuffer d_codes, d_alpha, d_staged, d_flat, d_counter;
   // search scratch
-  vcb::DeviceBuffer d_queries, d_luts, d_qf, d_cand_s, d_cand_i, d_out_s, d_out_i, d_qrot, d_partial;
+  vcb::DeviceBuffer d_queries, d_luts, d_qf, d_cand_s, d_cand_i, d_out_s, d_out_i, d_qrot, d_partial, d_onehot;
+  // Set once a search ran a kernel with bounded waits: sync() then looks at the
+  // word such a kernel sets when a wait gave up (behind d_counter's count).
+  // A search on another stream may still be running then: it keeps the flag set.
+  bool check_status = false, status_foreign = false;
 
   // Optional per-launch timing (tq_index_set_profiling).
   enum Kind { kPrep = 0, kScan = 1, kMerge = 2, kEncode = 3 };
@@ -239,7 +247,20 @@ struct tq_index {
     timed_launches.push_back(t);
   }
 
-  void sync() { vcb::check(cudaStreamSynchronize(stream), "cudaStreamSynchronize"); }
+  void sync() {
+    vcb::check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+    if (check_status) {
+      unsigned status = 0;
+      vcb::check(cudaMemcpyAsync(&status, device_status(), 4, cudaMemcpyDeviceToHost, stream), "D2H");
+      vcb::check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+      check_status = status_foreign;
+      if (status) {
+        vcb::check(cudaMemsetAsync(device_status(), 0, 4, stream), "cudaMemsetAsync");
+        vcb::fail(TQ_ERR_CUDA, "a scan kernel gave up waiting on its own pipeline; its results are not valid");
+      }
+    }
+  }
+  unsigned* device_status() const { return d_counter.as<unsigned>() + 2; }
 
   cudaStream_t pick(void* s) const { return s ? static_cast<cudaStream_t>(s) : stream; }
 
@@ -325,7 +346,7 @@ struct tq_index {
   }
 
   // The index's own search scratch (one search at a time on one stream).
-  vcb::FlatScratch own_scratch() { return {&d_luts, &d_qf, &d_cand_s, &d_cand_i, &d_partial}; }
+  vcb::FlatScratch own_scratch() { return {&d_luts, &d_qf, &d_cand_s, &d_cand_i, &d_partial, 0, &d_onehot}; }
 
   // LUTs and per-query constants for nq device rows.
   void prep_queries(const float* d_q, size_t nq, cudaStream_t s, float* q_rot_out) {
@@ -373,6 +394,12 @@ struct tq_index {
     for (size_t q0 = 0; q0 < nq; q0 += max_pass) {
       const size_t m = std::min(max_pass, nq - q0);
       prep_queries(d_q + q0 * dim, m, s, nullptr, sc);
+      vcb::OneHotPlan oh;
+      if (sc.onehot && vcb::plan_onehot(static_cast<long long>(n), static_cast<long long>(m), static_cast<int>(nbg),
+                                        static_cast<int>(bits), static_cast<int>(k_eff), sms, &oh)) {
+        search_onehot(oh, m, k_eff, d_scores + q0 * k_eff, d_ids + q0 * k_eff, s, sc);
+        continue;
+      }
       vcb::ScanPlan plan;
       if (!vcb::plan_scan(static_cast<long long>(n), static_cast<long long>(m), static_cast<int>(nbg),
                           static_cast<int>(k_eff), sms, &plan, sc.range_cap, static_cast<int>(bits))) {
@@ -431,6 +458,59 @@ struct tq_index {
       launch(kMerge, s, "merge kernel", [&] { return vcb::launch_merge(mg, s); });
     }
     (void)k;
+  }
+
+  // A batch of m prepared queries on the tensor cores: thresholds from a
+  // sample of the index, the scan above them, the merge of its lists.
+  void search_onehot(const vcb::OneHotPlan& p, size_t m, size_t k_eff, float* d_scores, uint64_t* d_ids, cudaStream_t s,
+                     vcb::FlatScratch sc) {
+    const size_t lists = 2 * static_cast<size_t>(p.n_ranges);
+    sc.cand_s->reserve(m * lists * p.list_len * 4);
+    sc.cand_i->reserve(m * lists * p.list_len * 4);
+    // The sample's scores and the scan's running lists share one region.
+    const size_t region = vcb::round_up(
+        std::max(vcb::onehot_list_bytes(p), vcb::onehot_sample_bytes(p, static_cast<long long>(m))), 256);
+    sc.onehot->reserve(region + m * 4);
+    float* floor = reinterpret_cast<float*>(sc.onehot->as<unsigned char>() + region);
+    const float* qf = sc.qf->as<float>();
+    vcb::OneHotArgs a{};
+    a.codes = d_codes.as<uint32_t>();
+    a.alpha = d_alpha.as<float>();
+    a.luts = sc.luts->as<uint8_t>();
+    a.lut_scale = qf;
+    a.fa_init = qf + 3 * m;
+    a.n = static_cast<long long>(n);
+    a.nbg = static_cast<int>(nbg);
+    a.nq = static_cast<long long>(m);
+    a.k = static_cast<int>(k_eff);
+    a.lists = sc.onehot->as<unsigned long long>();
+    a.cand_score = sc.cand_s->as<float>();
+    a.cand_id = sc.cand_i->as<uint32_t>();
+    a.floor = floor;
+    a.dense = sc.onehot->as<float>();
+    a.status = device_status();
+    check_status = true;
+    status_foreign |= s != stream;
+    launch(kPrep, s, "threshold sample kernel", [&] { return vcb::launch_onehot_sample(a, p, sms, s); });
+    launch(kPrep, s, "threshold kernel", [&] {
+      return vcb::launch_kth_floor(a.dense, static_cast<long long>(p.sample_tiles) * 256, nullptr,
+                                   static_cast<long long>(m), static_cast<int>(k_eff), floor, s);
+    });
+    launch(kScan, s, "scan kernel", [&] { return vcb::launch_onehot_scan(a, p, s); });
+    if (!vcb::dry_run_flag()) {
+      scan_stream_bytes += static_cast<uint64_t>(p.q_tiles) * n * (nbg + 4);
+      scan_queries += m;
+    }
+    vcb::MergeArgs mg{};
+    mg.cand_score = a.cand_score;
+    mg.cand_id = a.cand_id;
+    mg.nq = static_cast<long long>(m);
+    mg.n_lists = static_cast<int>(lists);
+    mg.k = p.list_len;
+    mg.k_out = static_cast<int>(k_eff);
+    mg.out_score = d_scores;
+    mg.out_id = d_ids;
+    launch(kMerge, s, "merge kernel", [&] { return vcb::launch_merge(mg, s); });
   }
 };
 

@@ -181,6 +181,61 @@ bool plan_scan(long long n, long long nq, int nbg, int k, int sms, ScanPlan* pla
 cudaError_t launch_scan(const ScanArgs& a, const ScanPlan& plan, cudaStream_t stream);
 cudaError_t launch_merge(const MergeArgs& a, cudaStream_t stream);
 
+// ---- batches of queries on the tensor cores (tq_onehot.cu) -------------------
+// The one-hot contraction costs the same up to about 64 queries, the lookup scan
+// grows with every four. Both measured (us per search, k = 10, lookup / one-hot):
+// 1M x 1536 4-bit 16 queries 1713 / 1642, 12 queries 1267 / 1641; 300k x 384
+// 2-bit 16 queries 141 / 134; 100k x 128 4-bit 32 queries 94 / 81, 24 queries
+// 69 / 80; 2M x 768 3-bit 32 queries 1987 / 1623, 24 queries 1430 / 1621 (3-bit
+// lookups take half the instructions). With k > 32 the lookup scan keeps its
+// lists in shared memory on one CTA per SM and loses from four queries on (1M x
+// 1536: 1716 / 1690; 100k x 128: 256 / 131).
+constexpr long long kOneHotMinQueries = 32;
+constexpr long long kOneHotMinQueriesWide = 16;        // 2- and 4-bit codes of at least ...
+constexpr long long kOneHotWideBytes = 20LL << 20;     // ... this many bytes
+constexpr long long kOneHotMinQueriesLists = 4;        // k > 32
+// Below this the launches (a sample, its thresholds) cost more than the scan.
+constexpr long long kOneHotMinVectors = 16384;
+
+struct OneHotPlan {
+  int tile_queries = 0;  // queries per tile (a multiple of 32, <= 256)
+  int q_tiles = 0;
+  int tiles = 0;         // 256-vector tiles of the index
+  int range_tiles = 0, n_ranges = 0;
+  int ctas = 0;
+  int cap = 256;         // entries per running list
+  int list_len = 0;      // entries per published list (>= k)
+  int sample_tiles = 0, sample_step = 1;
+};
+struct OneHotArgs {
+  const uint32_t* codes;
+  const float* alpha;
+  const uint8_t* luts;
+  const float* lut_scale;
+  const float* fa_init;
+  long long n;
+  int nbg;
+  long long nq;
+  int k;
+  // running lists: ctas x tile_queries x cap keys
+  unsigned long long* lists;
+  // candidate lists of plan.list_len: nq x (2 * n_ranges)
+  float* cand_score;
+  uint32_t* cand_id;
+  const float* floor;   // per query: no score below it reaches the top k
+  float* dense;         // sample: nq x dense_stride scores
+  long long dense_stride;
+  unsigned* status;     // device word, set to 1 when a wait gave up
+  // set by the launchers
+  int tile_queries, q_tiles, tiles, tile_step, range_tiles, n_ranges, list_len;
+};
+// False when the batch belongs to the lookup scan.
+bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, OneHotPlan* plan);
+size_t onehot_list_bytes(const OneHotPlan& p);
+size_t onehot_sample_bytes(const OneHotPlan& p, long long nq);
+cudaError_t launch_onehot_sample(const OneHotArgs& a, const OneHotPlan& p, int sms, cudaStream_t stream);
+cudaError_t launch_onehot_scan(const OneHotArgs& a, const OneHotPlan& p, cudaStream_t stream);
+
 // Parity/introspection: integer LUT sums and float scores for every
 // (query, vector) pair, computed straight from the scan layout.
 cudaError_t launch_dense_scores(const uint32_t* codes, const float* alpha, const uint8_t* luts,

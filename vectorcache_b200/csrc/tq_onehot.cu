@@ -1,0 +1,721 @@
+// The FastScan sums of a batch of queries as an integer contraction on the
+// tensor cores (sm_100a).
+//
+// A vector's LUT sum for a query is sum_g LUT[q][g][code(v, g)]: a row of the
+// one-hot matrix of its nibbles (16 columns per nibble, a single 1 each) times
+// the query's LUT bytes, which already lie K-major in the order [group][high
+// nibble's 16 entries, low nibble's 16]. u8 x u8 products with s32 accumulation
+// (tcgen05.mma kind::i8) give exactly the integers the lookup kernels add up,
+// and the epilogue flushes them into f32 every 256 byte groups with the same
+// fused multiply-add (search_avx2.cpp:24-48), so scores and top-k are equal bit
+// for bit to tq_scan.cu's.
+//
+// A pair of CTAs (cta_group::2) owns a tile of 256 vectors (128 per CTA) x N
+// queries (N <= 192). Per stage of 4 byte groups (128 bytes of K):
+//   * a TMA load per CTA brings its half of the N queries' LUT bytes to shared
+//     memory (K-major, 128-byte swizzle);
+//   * four of eight producer warps read the codes, build each vector's one-hot
+//     row in registers (its own TMEM lane) and store it to TMEM;
+//   * one thread of the pair issues four K = 32 MMAs (A in TMEM, B in shared
+//     memory).
+// The one-hot operand lives in TMEM because shared memory could not carry it as
+// well: writing and reading it there next to the LUT tiles takes all of the 128
+// bytes per clock at N = 256 (measured: 631 clocks per stage instead of 512).
+// Accumulators are double-buffered in TMEM per 256-group batch (2 x 192 columns,
+// the other 128 hold four one-hot stages); eight warps per CTA read them back,
+// keep the f32 sums in registers across batches (96 queries each), and append
+// scores at or above the query's threshold to a list, cut back to the top k when
+// it fills up.
+#include <cfloat>
+#include <algorithm>
+
+#include <cuda.h>
+
+#include "tq_device.cuh"
+#include "tq_kernels.h"
+#include "tq_tc.cuh"
+
+namespace vcb {
+namespace {
+
+// Byte groups per stage: 256 bytes of K. The issuing warp spends about 400 clocks
+// per stage on its waits and commits whatever the stage holds (measured), so a
+// stage has to be worth more than that: 8 MMAs are 768 clocks at N = 192.
+constexpr int kStageGroupsTc = 8;
+constexpr int kHalfGroups = 4;          // a producer set's share of a stage
+constexpr int kMaxN = 192;              // queries per tile
+constexpr int kHalfN = kMaxN / 2;       // LUT rows per CTA; queries per epilogue warp
+constexpr int kTileB = kHalfN * 128;    // LUT bytes per CTA and half stage (128 bytes of K)
+constexpr int kStagesB = 6;
+constexpr int kMaxStagesA = 4;
+constexpr int kHalfColsA = 32;          // TMEM columns of a half stage's one-hot rows
+constexpr int kStageColsA = 2 * kHalfColsA;
+// Codes: 32 byte groups (32 words of 128 vectors each) per chunk.
+constexpr int kChunkStages = 4;
+constexpr int kChunkGroups = kChunkStages * kStageGroupsTc;
+constexpr int kTileC = kChunkGroups * 128;
+constexpr int kStagesC = 4;
+constexpr int kTmemCols = 512;
+constexpr int kPairVectors = 256;
+constexpr int kBatchStages = kFlushGroups / kStageGroupsTc;
+// Warps 0-7 build one-hot rows (two sets of four, a TMEM quadrant each), 8-15
+// are the epilogue, 16 loads LUT tiles, 17 issues MMAs, 18 loads codes (19 fills
+// up the warpgroup). Registers: 640 x 96 at launch >= 256 x 64 + 256 x 152 + 128 x 40.
+constexpr int kThreads = 640;
+constexpr int kRegsLaunch = 96, kRegsProducer = 64, kRegsEpilogue = 152, kRegsIssue = 40;
+static_assert(256 * (kRegsProducer + kRegsEpilogue) + 128 * kRegsIssue <= kThreads * kRegsLaunch,
+              "the register split must fit what the block is launched with");
+
+constexpr int kQueue = 24;
+
+struct Shared {
+  uint64_t full_b[kStagesB], empty_b[kStagesB];
+  uint64_t full_a[kMaxStagesA], empty_a[kMaxStagesA];
+  uint64_t full_c[kStagesC], empty_c[kStagesC];
+  uint64_t acc_full[2], acc_empty[2];
+  uint32_t tmem;
+  uint32_t pad[3];
+  float scale[kMaxN];
+  float init[kMaxN];
+  float thr[kMaxN];
+  int cnt[kMaxN];
+  // Scores at or above their query's threshold on their way to the query lists:
+  // (score, query column), kQueue entries per epilogue lane.
+  uint2 queue[8][kQueue][32];
+};
+constexpr size_t kSmemBytes = 1024 + static_cast<size_t>(kStagesB) * 2 * kTileB + kStagesC * kTileC + sizeof(Shared);
+
+__device__ __forceinline__ uint32_t order_key(float s) {
+  const uint32_t u = __float_as_uint(s);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float key_score(uint32_t k) {
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+// Descending bitonic sort of 32 * E keys of a warp, entry lane * E + e.
+template <int E>
+__device__ __forceinline__ void warp_sort_keys(unsigned long long (&key)[E], int lane) {
+#pragma unroll
+  for (int size = 2; size <= 32 * E; size <<= 1) {
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      if (stride >= E) {
+        const int m = stride / E;
+        const bool lower = (lane & m) == 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const unsigned long long o = __shfl_xor_sync(full_mask(), key[e], m);
+          const bool desc = ((lane * E + e) & size) == 0;
+          const bool take_max = lower == desc;
+          key[e] = ((key[e] > o) == take_max) ? key[e] : o;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          if ((e & stride) == 0) {
+            const bool desc = ((lane * E + e) & size) == 0;
+            const unsigned long long x = key[e], y = key[e | stride];
+            const bool keep = (x > y) == desc;
+            key[e] = keep ? x : y;
+            key[e | stride] = keep ? y : x;
+          }
+        }
+      }
+    }
+  }
+}
+
+// Cuts a list of n (<= 32 * E) entries to its best min(k, n), best first, in
+// place; returns the k-th key.
+template <int E>
+__device__ __noinline__ unsigned long long cut_list(unsigned long long* list, int n, int k, int lane) {
+  unsigned long long key[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = lane * E + e;
+    key[e] = i < n ? __ldcg(list + i) : 0ull;
+  }
+  warp_sort_keys<E>(key, lane);
+  unsigned long long kth = 0ull;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = lane * E + e;
+    if (i < k && i < n) list[i] = key[e];
+    const unsigned long long c = __shfl_sync(full_mask(), key[e], (k - 1) / E);
+    if ((k - 1) % E == e) kth = c;
+  }
+  return kth;
+}
+
+template <int CAP>
+__device__ __forceinline__ unsigned long long cut_any(unsigned long long* list, int n, int k, int lane) {
+  const int m = n > k ? n : k;
+  if (m <= 128) return cut_list<4>(list, n, k, lane);
+  if (CAP == 256 || m <= 256) return cut_list<8>(list, n, k, lane);
+  return cut_list<16>(list, n, k, lane);
+}
+
+// The 16 one-hot bytes of the nibble in bits 3..6 of x, as two 64-bit shifts of a
+// 1 by 8 * nibble and 8 * nibble - 64; a shift of 64 or more gives 0.
+__device__ __forceinline__ void onehot16(uint32_t x, uint32_t* out) {
+  uint64_t lo, hi;
+  asm("shl.b64 %0, %1, %2;" : "=l"(lo) : "l"(uint64_t{1}), "r"(x & 0x78u));
+  asm("shl.b64 %0, %1, %2;" : "=l"(hi) : "l"(uint64_t{1}), "r"((x & 0x78u) ^ 0x40u));
+  out[0] = static_cast<uint32_t>(lo);
+  out[1] = static_cast<uint32_t>(lo >> 32);
+  out[2] = static_cast<uint32_t>(hi);
+  out[3] = static_cast<uint32_t>(hi >> 32);
+}
+
+// SAMPLE: write every score of the sampled tiles (thresholds come from them).
+// Otherwise keep each query's top k of the range; CAP entries per list.
+template <bool SAMPLE, int CAP>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    onehot_scan_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap code_map,
+                       OneHotArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t{1023});
+  unsigned char* codes_smem = base + static_cast<size_t>(kStagesB) * 2 * kTileB;
+  Shared& sh = *reinterpret_cast<Shared*>(codes_smem + kStagesC * kTileC);
+  const uint32_t sB = tc::smem_u32(base), sC = tc::smem_u32(codes_smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = tc::cta_rank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int n_stages = (a.nbg + kStageGroupsTc - 1) / kStageGroupsTc;
+  const int n_batches = (a.nbg + kFlushGroups - 1) / kFlushGroups;
+  const int items = a.q_tiles * a.n_ranges;
+  // TMEM: two accumulators of acc_cols columns, then the one-hot stages.
+  const uint32_t acc_cols = a.tile_queries <= 128 ? 128 : kMaxN;
+  const int stages_a = acc_cols == 128 ? kMaxStagesA : 2;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStagesB; ++s) {
+      tc::mbar_init(tc::smem_u32(&sh.full_b[s]), 1);
+      tc::mbar_init(tc::smem_u32(&sh.empty_b[s]), 1);
+    }
+    for (int s = 0; s < kMaxStagesA; ++s) {
+      tc::mbar_init(tc::smem_u32(&sh.full_a[s]), 16);  // eight producer warps of each CTA
+      tc::mbar_init(tc::smem_u32(&sh.empty_a[s]), 1);
+    }
+    for (int s = 0; s < kStagesC; ++s) {
+      tc::mbar_init(tc::smem_u32(&sh.full_c[s]), 1);
+      tc::mbar_init(tc::smem_u32(&sh.empty_c[s]), 8);  // this CTA's producer warps
+    }
+    for (int b = 0; b < 2; ++b) {
+      tc::mbar_init(tc::smem_u32(&sh.acc_full[b]), 1);
+      tc::mbar_init(tc::smem_u32(&sh.acc_empty[b]), 16);  // eight epilogue warps of each CTA
+    }
+    tc::mbar_init_fence();
+    tc::prefetch_map(&lut_map);
+    tc::prefetch_map(&code_map);
+  }
+  if (warp == 17) {
+    tc::tmem_alloc2(tc::smem_u32(&sh.tmem), kTmemCols);
+    tc::tmem_relinquish2();
+    tc::fence_before();
+  }
+  __syncthreads();
+  tc::cluster_sync();
+  tc::fence_after();
+  const uint32_t tmem = sh.tmem;
+  bool alive = true;  // false: a wait gave up; this role stops
+
+  if (warp < 8) {
+    // ---- one-hot rows: set `set` builds its half of every stage; TMEM lane
+    // 32 quad + lane holds vector 4 lane + quad of this CTA's 128.
+    tc::reg_dec<kRegsProducer>();
+    const int quad = warp & 3, set = warp >> 2;
+    const uint32_t dst0 = tmem + 2 * acc_cols + set * kHalfColsA + (static_cast<uint32_t>(quad * 32) << 16);
+    const uint32_t src0 = sC + set * kHalfGroups * 128 + lane * 4;
+    const unsigned rot = (4 * quad + 29) & 31;  // brings the quad's nibbles to bits 3..6 and 19..22
+    int slot = 0, sc = 0;
+    uint32_t ph = 0, pc = 0;
+    for (int it = pair; it < items && alive; it += pairs) {
+      const int r = it % a.n_ranges;
+      const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
+      for (int t = t0; t < t1 && alive; ++t) {
+        for (int s0 = 0; s0 < n_stages && alive; s0 += kChunkStages) {
+          if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.full_c[sc]), pc))) {
+            alive = false;
+            break;
+          }
+          const int s1 = min(kChunkStages, n_stages - s0);
+          uint32_t src = src0 + sc * kTileC;
+          for (int s = 0; s < s1; ++s, src += kStageGroupsTc * 128) {
+            // The first look at the slot runs under the shifts, the first
+            // half's columns are stored while the second half is built.
+            const uint32_t bar = tc::smem_u32(&sh.empty_a[slot]);
+            const bool ready = tc::mbar_test(bar, ph ^ 1u);
+            uint32_t w[kHalfGroups], row[2][kHalfColsA / 2];
+#pragma unroll
+            for (int g = 0; g < kHalfGroups; ++g) {
+              asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[g]) : "r"(src + g * 128));
+            }
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              // high nibble (first half of the LUT row), then the low one
+              const uint32_t x = __funnelshift_r(w[g], w[g], rot);
+              onehot16(x >> 16, row[0] + 8 * g);
+              onehot16(x, row[0] + 8 * g + 4);
+            }
+            if (!__all_sync(full_mask(), ready || tc::mbar_wait(bar, ph ^ 1u))) {
+              alive = false;
+              break;
+            }
+            tc::fence_after();
+            tc::tmem_st16(dst0 + slot * kStageColsA, row[0]);
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              const uint32_t x = __funnelshift_r(w[2 + g], w[2 + g], rot);
+              onehot16(x >> 16, row[1] + 8 * g);
+              onehot16(x, row[1] + 8 * g + 4);
+            }
+            tc::tmem_st16(dst0 + slot * kStageColsA + kHalfColsA / 2, row[1]);
+            tc::tmem_wait_st();
+            tc::fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&sh.full_a[slot]), 0));
+            if (++slot == stages_a) {
+              slot = 0;
+              ph ^= 1u;
+            }
+          }
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(tc::smem_u32(&sh.empty_c[sc]));
+          if (++sc == kStagesC) {
+            sc = 0;
+            pc ^= 1u;
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp >= 16) {
+    tc::reg_dec<kRegsIssue>();
+    if (warp == 16) {
+      // ---- LUT tiles -------------------------------------------------------
+      int st = 0;
+      uint32_t ph = 0;
+      for (int it = pair; it < items && alive; it += pairs) {
+        const int qt = it / a.n_ranges, r = it % a.n_ranges;
+        const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
+        const int y = qt * a.tile_queries + static_cast<int>(rank) * (a.tile_queries / 2);
+        for (int t = t0; t < t1 && alive; ++t) {
+          for (int s = 0; s < n_stages; ++s) {
+            if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) {
+              alive = false;
+              break;
+            }
+            const uint32_t bar = tc::smem_u32(&sh.full_b[st]);
+            if (tc::elect_one()) {
+              if (rank == 0) tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(a.tile_queries) * 256u);
+              const uint32_t cbar = tc::mapa(bar, 0);
+              tc::tma_load_2d_pair(sB + st * 2 * kTileB, &lut_map, s * 256, y, cbar);
+              tc::tma_load_2d_pair(sB + (st * 2 + 1) * kTileB, &lut_map, s * 256 + 128, y, cbar);
+            }
+            __syncwarp();
+            if (++st == kStagesB) {
+              st = 0;
+              ph ^= 1u;
+            }
+          }
+        }
+      }
+    } else if (warp == 18) {
+      // ---- code chunks: 32 rows (byte groups) x 32 words of the scan layout.
+      // Rows past the tile's last byte group meet zero LUT bytes.
+      int sc = 0;
+      uint32_t ph = 0;
+      for (int it = pair; it < items && alive; it += pairs) {
+        const int r = it % a.n_ranges;
+        const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
+        for (int t = t0; t < t1 && alive; ++t) {
+          const int vt = a.tile_step > 0 ? t * a.tile_step : t;
+          for (int g0 = 0; g0 < a.nbg; g0 += kChunkGroups) {
+            if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_c[sc]), ph ^ 1u))) {
+              alive = false;
+              break;
+            }
+            const uint32_t bar = tc::smem_u32(&sh.full_c[sc]);
+            if (tc::elect_one()) {
+              tc::mbar_arrive_expect_tx(bar, kTileC);
+              tc::tma_load_2d(sC + sc * kTileC, &code_map, (vt & 1) * 64 + static_cast<int>(rank) * 32,
+                              (vt >> 1) * a.nbg + g0, bar);
+            }
+            __syncwarp();
+            if (++sc == kStagesC) {
+              sc = 0;
+              ph ^= 1u;
+            }
+          }
+        }
+      }
+    } else if (warp == 17 && rank == 0) {
+      // ---- MMA ---------------------------------------------------------------
+      const uint32_t idesc = (2u << 4) | (static_cast<uint32_t>(a.tile_queries >> 3) << 17) | (16u << 24);
+      int sa = 0, sb = 0;
+      uint32_t pa = 0, pb = 0, batch = 0;
+      for (int it = pair; it < items && alive; it += pairs) {
+        const int r = it % a.n_ranges;
+        const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
+        for (int t = t0; t < t1 && alive; ++t) {
+          for (int s0 = 0; s0 < n_stages && alive; s0 += kBatchStages, ++batch) {
+            const uint32_t buf = batch & 1u;
+            const uint32_t d = tmem + buf * acc_cols;
+            if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.acc_empty[buf]), ((batch >> 1) & 1u) ^ 1u))) {
+              alive = false;
+              break;
+            }
+            const int s1 = min(s0 + kBatchStages, n_stages);
+            for (int s = s0; s < s1; ++s) {
+              if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.full_b[sb]), pb) &&
+                                               tc::mbar_wait(tc::smem_u32(&sh.full_a[sa]), pa))) {
+                alive = false;
+                break;
+              }
+              tc::fence_after();
+              const uint32_t ta = tmem + 2 * acc_cols + sa * kStageColsA;
+              const uint64_t db = tc::desc_k128(sB + sb * 2 * kTileB);
+              const uint64_t db2 = tc::desc_k128(sB + (sb * 2 + 1) * kTileB);
+              const bool second = s * kStageGroupsTc + kHalfGroups < a.nbg;
+              if (tc::elect_one()) {
+#pragma unroll
+                for (int j = 0; j < kHalfGroups; ++j) {
+                  tc::mma_i8_pair_ta(d, ta + 8u * j, db + 2u * j, idesc, (s > s0 || j > 0) ? 1u : 0u);
+                }
+                if (second) {
+#pragma unroll
+                  for (int j = 0; j < kHalfGroups; ++j) {
+                    tc::mma_i8_pair_ta(d, ta + kHalfColsA + 8u * j, db2 + 2u * j, idesc, 1u);
+                  }
+                }
+                tc::commit2(tc::smem_u32(&sh.empty_a[sa]));
+                tc::commit2(tc::smem_u32(&sh.empty_b[sb]));
+                if (s + 1 == s1) tc::commit2(tc::smem_u32(&sh.acc_full[buf]));
+              }
+              __syncwarp();
+              if (++sa == stages_a) {
+                sa = 0;
+                pa ^= 1u;
+              }
+              if (++sb == kStagesB) {
+                sb = 0;
+                pb ^= 1u;
+              }
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue: warp quadrant = 32 vectors, half = N / 2 queries ------------
+    tc::reg_inc<kRegsEpilogue>();
+    const int quad = warp & 3, half = (warp - 8) >> 2;
+    const int cols = a.tile_queries / 2;       // this half's queries, a multiple of 16
+    const int c0 = half * cols;
+    const uint32_t t_base = tmem + (static_cast<uint32_t>(quad * 32) << 16) + c0;
+    unsigned long long* lists = a.lists + (static_cast<long long>(blockIdx.x) * a.tile_queries + c0) * CAP;
+    const float* s_scale = sh.scale + half * kHalfN;
+    const float* s_init = sh.init + half * kHalfN;
+    float* s_thr = sh.thr + half * kHalfN;
+    int* s_cnt = sh.cnt + half * kHalfN;
+    uint2* queue = &sh.queue[warp - 8][0][lane];
+    const int ht = (warp & 3) * 32 + lane;  // thread of the half
+    uint32_t batch = 0;
+    for (int it = pair; it < items; it += pairs) {
+      const int qt = it / a.n_ranges, r = it % a.n_ranges;
+      const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
+      const long long q0 = static_cast<long long>(qt) * a.tile_queries + c0;
+      tc::named_sync(1 + half, 128);
+      if (ht < cols) {
+        const bool ok = q0 + ht < a.nq;
+        sh.scale[half * kHalfN + ht] = ok ? a.lut_scale[q0 + ht] : 0.f;
+        sh.init[half * kHalfN + ht] = ok ? a.fa_init[q0 + ht] : 0.f;
+        // -FLT_MAX admits every score above -inf; NaN never compares >=.
+        float th = -FLT_MAX;
+        if (!SAMPLE && ok && a.floor) th = fmaxf(th, a.floor[q0 + ht]);
+        s_thr[ht] = ok ? th : INFINITY;
+        s_cnt[ht] = 0;
+      }
+      tc::named_sync(1 + half, 128);
+      for (int t = t0; t < t1; ++t) {
+        const long long vt = a.tile_step > 0 ? static_cast<long long>(t) * a.tile_step : t;
+        const long long v = vt * kPairVectors + rank * 128 + 4 * lane + quad;
+        const bool valid = v < a.n;
+        const float al = valid ? __ldg(a.alpha + v) : 0.f;
+        float fa[kHalfN];
+#pragma unroll
+        for (int c = 0; c < kHalfN / 16; ++c) {
+          if (c * 16 < cols) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 f = *reinterpret_cast<const float4*>(s_init + c * 16 + i);
+              fa[c * 16 + i] = f.x;
+              fa[c * 16 + i + 1] = f.y;
+              fa[c * 16 + i + 2] = f.z;
+              fa[c * 16 + i + 3] = f.w;
+            }
+          }
+        }
+        for (int b = 0; b < n_batches; ++b, ++batch) {
+          const uint32_t buf = batch & 1u;
+          // A warp whose wait gave up goes on through the barriers it shares.
+          if (alive) alive = __all_sync(full_mask(), tc::mbar_wait_long(tc::smem_u32(&sh.acc_full[buf]), (batch >> 1) & 1u));
+          tc::fence_after();
+#pragma unroll
+          for (int c = 0; c < kHalfN / 16; ++c) {
+            if (c * 16 < cols) {
+              uint32_t acc[16];
+              tc::tmem_ld16(t_base + buf * acc_cols + c * 16, acc);
+              tc::tmem_wait_ld16(acc);
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(s_scale + c * 16 + i);
+                fa[c * 16 + i] = __fmaf_rn(f.x, __uint2float_rn(acc[i]), fa[c * 16 + i]);
+                fa[c * 16 + i + 1] = __fmaf_rn(f.y, __uint2float_rn(acc[i + 1]), fa[c * 16 + i + 1]);
+                fa[c * 16 + i + 2] = __fmaf_rn(f.z, __uint2float_rn(acc[i + 2]), fa[c * 16 + i + 2]);
+                fa[c * 16 + i + 3] = __fmaf_rn(f.w, __uint2float_rn(acc[i + 3]), fa[c * 16 + i + 3]);
+              }
+            }
+          }
+          tc::fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&sh.acc_empty[buf]), 0));
+        }
+        if (SAMPLE) {
+          const long long at = static_cast<long long>(t) * kPairVectors + rank * 128 + quad * 32 + lane;
+#pragma unroll
+          for (int c = 0; c < kHalfN / 16; ++c) {
+            if (c * 16 < cols) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                if (q0 + c * 16 + i < a.nq) {
+                  a.dense[(q0 + c * 16 + i) * a.dense_stride + at] =
+                      valid ? __fadd_rn(__fmul_rn(fa[c * 16 + i], al), 0.f) : -INFINITY;
+                }
+              }
+            }
+          }
+        } else {
+          // Straight-line code per score (no branch, no vote): scores at or above
+          // the threshold go to the lane's own queue, and the queues to the lists
+          // once per tile (sooner only when one could overflow).
+          int queued = 0;
+          auto flush = [&]() {
+            for (int e = 0; __any_sync(full_mask(), e < queued); ++e) {
+              if (e < queued) {
+                const uint2 x = queue[e * 32];
+                const int pos = atomicAdd(&s_cnt[x.y], 1);
+                lists[static_cast<long long>(x.y) * CAP + pos] =
+                    (static_cast<unsigned long long>(order_key(__uint_as_float(x.x))) << 32) |
+                    static_cast<uint32_t>(~static_cast<uint32_t>(v));
+              }
+            }
+            queued = 0;
+          };
+          // NaN and lanes past the end of the index never compare >=.
+          const float al_top = valid ? al : NAN;
+#pragma unroll
+          for (int c = 0; c < kHalfN / 16; ++c) {
+            if (c * 16 < cols) {
+#pragma unroll
+              for (int i = c * 16; i < c * 16 + 16; i += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(s_thr + i);
+                const float th[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const float sc = __fadd_rn(__fmul_rn(fa[i + u], al_top), 0.f);
+                  if (sc >= th[u]) {
+                    queue[queued * 32] = make_uint2(__float_as_uint(sc), static_cast<unsigned>(i + u));
+                    ++queued;
+                  }
+                }
+              }
+              if (__any_sync(full_mask(), queued > kQueue - 16)) flush();
+            }
+          }
+          flush();
+          // A tile adds at most 128 entries per list: cut the lists that might
+          // overflow on the next one to their top k and raise the threshold.
+          tc::named_sync(1 + half, 128);
+          const int mine = lane * 4 + quad;
+          unsigned need = __ballot_sync(full_mask(), mine < cols && s_cnt[mine] > CAP - 128);
+          while (need) {
+            const int c = (__ffs(need) - 1) * 4 + quad;
+            need &= need - 1;
+            const int n = s_cnt[c];
+            const unsigned long long kth = cut_any<CAP>(lists + static_cast<long long>(c) * CAP, n, a.k, lane);
+            __syncwarp();
+            if (lane == 0) {
+              s_cnt[c] = min(n, a.k);
+              if (n >= a.k) s_thr[c] = key_score(static_cast<uint32_t>(kth >> 32));
+            }
+          }
+          tc::named_sync(1 + half, 128);
+        }
+      }
+      if (!SAMPLE && alive) {
+        // Publish: lists that fit go out as they are, longer ones cut to the top k.
+        for (int c = quad; c < cols; c += 4) {
+          if (q0 + c >= a.nq) break;
+          unsigned long long* list = lists + static_cast<long long>(c) * CAP;
+          const long long out = ((q0 + c) * (2LL * a.n_ranges) + 2 * r + rank) * a.list_len;
+          int n = s_cnt[c];
+          if (n > a.list_len) {
+            cut_any<CAP>(list, n, a.k, lane);
+            __syncwarp();
+            n = a.k;
+          }
+          for (int i = lane; i < a.list_len; i += kWarp) {
+            const unsigned long long key = i < n ? __ldcg(list + i) : 0ull;
+            a.cand_score[out + i] = i < n ? key_score(static_cast<uint32_t>(key >> 32)) : -INFINITY;
+            a.cand_id[out + i] = ~static_cast<uint32_t>(key);
+          }
+        }
+      }
+    }
+  }
+  if (!alive && a.status) atomicExch(a.status, 1u);
+  // A role that gave up waited about two seconds first, so no copy of this
+  // CTA is still in flight here; otherwise every load was consumed.
+  __syncwarp();
+  __syncthreads();
+  tc::cluster_sync();
+  if (warp == 17) tc::tmem_dealloc2(tmem, kTmemCols);
+}
+
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiled encode_tiled() {
+  static EncodeTiled fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      p = nullptr;
+    }
+    return reinterpret_cast<EncodeTiled>(p);
+  }();
+  return fn;
+}
+
+cudaError_t make_map(CUtensorMapDataType type, const void* p, uint64_t cols, uint64_t rows, uint64_t row_bytes,
+                     uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle swizzle, CUtensorMap* m) {
+  EncodeTiled fn = encode_tiled();
+  if (!fn) return cudaErrorNotSupported;
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {row_bytes};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  const cuuint32_t es[2] = {1, 1};
+  const CUresult r = fn(m, type, 2, const_cast<void*>(p), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+template <bool SAMPLE, int CAP>
+cudaError_t launch_t(const OneHotArgs& a, int ctas, cudaStream_t stream) {
+  auto kern = onehot_scan_kernel<SAMPLE, CAP>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
+  if (e != cudaSuccess) return e;
+  CUtensorMap luts, codes;
+  e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, a.luts, static_cast<uint64_t>(a.nbg) * 32, static_cast<uint64_t>(a.nq),
+               static_cast<uint64_t>(a.nbg) * 32, 128, static_cast<uint32_t>(a.tile_queries / 2),
+               CU_TENSOR_MAP_SWIZZLE_128B, &luts);
+  if (e != cudaSuccess) return e;
+  const uint64_t rows = static_cast<uint64_t>((a.n + kTileVectors - 1) / kTileVectors) * static_cast<uint64_t>(a.nbg);
+  e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT32, a.codes, kTileWords, rows, kTileWords * 4, 32, kChunkGroups,
+               CU_TENSOR_MAP_SWIZZLE_NONE, &codes);
+  if (e != cudaSuccess) return e;
+  kern<<<static_cast<unsigned>(ctas), kThreads, kSmemBytes, stream>>>(luts, codes, a);
+  return cudaGetLastError();
+}
+
+// Ranges per query tile so that the items fill whole waves of CTA pairs: the
+// fewest ranges within 1 % of the smallest longest-pair time, but at least a
+// third of the pairs each (at most three query tiles' LUTs live in L2 at once).
+int choose_ranges(long long q_tiles, long long tiles, int pairs) {
+  const long long most = std::min<long long>(tiles, 2LL * pairs);
+  auto cost = [&](long long r) {
+    const long long per = (tiles + r - 1) / r;
+    const long long rr = (tiles + per - 1) / per;
+    return ((q_tiles * rr + pairs - 1) / pairs) * per;
+  };
+  long long best = cost(1);
+  for (long long r = 2; r <= most; ++r) best = std::min(best, cost(r));
+  const long long from = std::min<long long>(most, (pairs + 2) / 3);
+  for (long long r = from; r <= most; ++r) {
+    if (cost(r) * 100 <= best * 101) return static_cast<int>(r);
+  }
+  for (long long r = 1; r <= most; ++r) {
+    if (cost(r) * 100 <= best * 101) return static_cast<int>(r);
+  }
+  return 1;
+}
+
+}  // namespace
+
+bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, OneHotPlan* plan) {
+  if (n < kOneHotMinVectors || n > 0x7fffffffLL || nq < 1 || k < 1 || k > kMaxK || sms < 2) return false;
+  const bool wide = bits != 3 && n * nbg >= kOneHotWideBytes;
+  if (nq < (k > 32 ? kOneHotMinQueriesLists : (wide ? kOneHotMinQueriesWide : kOneHotMinQueries))) return false;
+  const long long q_tiles = (nq + kMaxN - 1) / kMaxN;
+  const long long per = (nq + q_tiles - 1) / q_tiles;
+  plan->tile_queries = static_cast<int>((per + 31) / 32 * 32);
+  plan->q_tiles = static_cast<int>((nq + plan->tile_queries - 1) / plan->tile_queries);
+  plan->tiles = static_cast<int>((n + kPairVectors - 1) / kPairVectors);
+  const int pairs = sms / 2;
+  int r = choose_ranges(plan->q_tiles, plan->tiles, pairs);
+  plan->range_tiles = (plan->tiles + r - 1) / r;
+  plan->n_ranges = (plan->tiles + plan->range_tiles - 1) / plan->range_tiles;
+  const long long items = static_cast<long long>(plan->q_tiles) * plan->n_ranges;
+  plan->ctas = static_cast<int>(2 * std::min<long long>(pairs, items));
+  plan->cap = k <= 64 ? 256 : 512;
+  plan->list_len = k + 16;
+  // Thresholds: the k-th best of a sample of whole tiles spread over the index,
+  // 1/64 of it within [1024, 16384] vectors and 64 MiB of scores.
+  long long sample = n / 64;
+  sample = std::min<long long>(sample, 16384);
+  sample = std::min<long long>(sample, (64LL << 20) / 4 / nq);
+  sample = std::max<long long>(sample, 1024);
+  plan->sample_tiles = static_cast<int>(std::min<long long>(plan->tiles, sample / kPairVectors));
+  plan->sample_step = plan->tiles / plan->sample_tiles;
+  return true;
+}
+
+size_t onehot_list_bytes(const OneHotPlan& p) { return static_cast<size_t>(p.ctas) * p.tile_queries * p.cap * 8; }
+size_t onehot_sample_bytes(const OneHotPlan& p, long long nq) {
+  return static_cast<size_t>(nq) * p.sample_tiles * kPairVectors * 4;
+}
+
+cudaError_t launch_onehot_sample(const OneHotArgs& in, const OneHotPlan& p, int sms, cudaStream_t stream) {
+  OneHotArgs a = in;
+  a.tile_queries = p.tile_queries;
+  a.q_tiles = p.q_tiles;
+  a.tiles = p.sample_tiles;
+  a.tile_step = p.sample_step;
+  a.dense_stride = static_cast<long long>(p.sample_tiles) * kPairVectors;
+  const int r = choose_ranges(p.q_tiles, p.sample_tiles, sms / 2);
+  a.range_tiles = (a.tiles + r - 1) / r;
+  a.n_ranges = (a.tiles + a.range_tiles - 1) / a.range_tiles;
+  const long long items = static_cast<long long>(a.q_tiles) * a.n_ranges;
+  return launch_t<true, 256>(a, static_cast<int>(2 * std::min<long long>(sms / 2, items)), stream);
+}
+
+cudaError_t launch_onehot_scan(const OneHotArgs& in, const OneHotPlan& p, cudaStream_t stream) {
+  OneHotArgs a = in;
+  a.tile_queries = p.tile_queries;
+  a.q_tiles = p.q_tiles;
+  a.tiles = p.tiles;
+  a.tile_step = 0;
+  a.range_tiles = p.range_tiles;
+  a.n_ranges = p.n_ranges;
+  a.list_len = p.list_len;
+  return p.cap == 256 ? launch_t<false, 256>(a, p.ctas, stream) : launch_t<false, 512>(a, p.ctas, stream);
+}
+
+}  // namespace vcb
