@@ -66,8 +66,6 @@ constexpr int kRegsLaunch = 96, kRegsProducer = 64, kRegsEpilogue = 152, kRegsIs
 static_assert(256 * (kRegsProducer + kRegsEpilogue) + 128 * kRegsIssue <= kThreads * kRegsLaunch,
               "the register split must fit what the block is launched with");
 
-constexpr int kQueue = 24;
-
 struct Shared {
   uint64_t full_b[kStagesB], empty_b[kStagesB];
   uint64_t full_a[kMaxStagesA], empty_a[kMaxStagesA];
@@ -79,9 +77,8 @@ struct Shared {
   float init[kMaxN];
   float thr[kMaxN];
   int cnt[kMaxN];
-  // Scores at or above their query's threshold on their way to the query lists:
-  // (score, query column), kQueue entries per epilogue lane.
-  uint2 queue[8][kQueue][32];
+  // 32 queries' scores of an epilogue warp's 32 vectors.
+  float stage[8][32][32];
 };
 constexpr size_t kSmemBytes = 1024 + static_cast<size_t>(kStagesB) * 2 * kTileB + kStagesC * kTileC + sizeof(Shared);
 
@@ -421,7 +418,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const float* s_init = sh.init + half * kHalfN;
     float* s_thr = sh.thr + half * kHalfN;
     int* s_cnt = sh.cnt + half * kHalfN;
-    uint2* queue = &sh.queue[warp - 8][0][lane];
+    float* stage = &sh.stage[warp - 8][0][lane];
     const int ht = (warp & 3) * 32 + lane;  // thread of the half
     uint32_t batch = 0;
     for (int it = pair; it < items; it += pairs) {
@@ -465,18 +462,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           if (alive) alive = __all_sync(full_mask(), tc::mbar_wait_long(tc::smem_u32(&sh.acc_full[buf]), (batch >> 1) & 1u));
           tc::fence_after();
 #pragma unroll
-          for (int c = 0; c < kHalfN / 16; ++c) {
-            if (c * 16 < cols) {
-              uint32_t acc[16];
-              tc::tmem_ld16(t_base + buf * acc_cols + c * 16, acc);
-              tc::tmem_wait_ld16(acc);
+          for (int c = 0; c < kHalfN / 32; ++c) {
+            if (c * 32 < cols) {
+              uint32_t acc[32];  // past `cols` the columns belong to the other half or are unused
+              tc::tmem_ld32(t_base + buf * acc_cols + c * 32, acc);
+              tc::tmem_wait_ld32(acc);
 #pragma unroll
-              for (int i = 0; i < 16; i += 4) {
-                const float4 f = *reinterpret_cast<const float4*>(s_scale + c * 16 + i);
-                fa[c * 16 + i] = __fmaf_rn(f.x, __uint2float_rn(acc[i]), fa[c * 16 + i]);
-                fa[c * 16 + i + 1] = __fmaf_rn(f.y, __uint2float_rn(acc[i + 1]), fa[c * 16 + i + 1]);
-                fa[c * 16 + i + 2] = __fmaf_rn(f.z, __uint2float_rn(acc[i + 2]), fa[c * 16 + i + 2]);
-                fa[c * 16 + i + 3] = __fmaf_rn(f.w, __uint2float_rn(acc[i + 3]), fa[c * 16 + i + 3]);
+              for (int i = 0; i < 32; i += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(s_scale + c * 32 + i);
+                const float sc[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  // The batch sum is below 2^23: exact as 2^23 + sum.
+                  const float v = __fsub_rn(__uint_as_float(acc[i + u] | 0x4b000000u), 8388608.f);
+                  fa[c * 32 + i + u] = __fmaf_rn(sc[u], v, fa[c * 32 + i + u]);
+                }
               }
             }
           }
@@ -499,44 +499,43 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
           }
         } else {
-          // Straight-line code per score (no branch, no vote): scores at or above
-          // the threshold go to the lane's own queue, and the queues to the lists
-          // once per tile (sooner only when one could overflow).
-          int queued = 0;
-          auto flush = [&]() {
-            for (int e = 0; __any_sync(full_mask(), e < queued); ++e) {
-              if (e < queued) {
-                const uint2 x = queue[e * 32];
-                const int pos = atomicAdd(&s_cnt[x.y], 1);
-                lists[static_cast<long long>(x.y) * CAP + pos] =
-                    (static_cast<unsigned long long>(order_key(__uint_as_float(x.x))) << 32) |
-                    static_cast<uint32_t>(~static_cast<uint32_t>(v));
-              }
-            }
-            queued = 0;
-          };
+          // Per 32 queries: one mask bit per score at or above its threshold, by
+          // straight-line code. Only when some lane has one do the scores go
+          // through shared memory (registers cannot be indexed) to the lists.
           // NaN and lanes past the end of the index never compare >=.
           const float al_top = valid ? al : NAN;
 #pragma unroll
-          for (int c = 0; c < kHalfN / 16; ++c) {
-            if (c * 16 < cols) {
+          for (int c = 0; c < kHalfN / 32; ++c) {
+            if (c * 32 < cols) {
+              unsigned part[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-              for (int i = c * 16; i < c * 16 + 16; i += 4) {
-                const float4 f = *reinterpret_cast<const float4*>(s_thr + i);
+              for (int i = 0; i < 32; i += 4) {
+                const float4 f = *reinterpret_cast<const float4*>(s_thr + c * 32 + i);
                 const float th[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                  const float sc = __fadd_rn(__fmul_rn(fa[i + u], al_top), 0.f);
-                  if (sc >= th[u]) {
-                    queue[queued * 32] = make_uint2(__float_as_uint(sc), static_cast<unsigned>(i + u));
-                    ++queued;
-                  }
+                  fa[c * 32 + i + u] = __fmul_rn(fa[c * 32 + i + u], al_top);
+                  if (fa[c * 32 + i + u] >= th[u]) part[u] |= 1u << (i + u);
                 }
               }
-              if (__any_sync(full_mask(), queued > kQueue - 16)) flush();
+              unsigned hits = part[0] | part[1] | part[2] | part[3];
+              if (cols - c * 32 < 32) hits &= 0xffffu;  // the last 16 queries
+              if (__any_sync(full_mask(), hits != 0u)) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) stage[i * 32] = fa[c * 32 + i];
+                while (hits) {
+                  const int i = __ffs(hits) - 1;
+                  hits &= hits - 1;
+                  const float score = __fadd_rn(stage[i * 32], 0.f);
+                  const int pos = atomicAdd(&s_cnt[c * 32 + i], 1);
+                  lists[static_cast<long long>(c * 32 + i) * CAP + pos] =
+                      (static_cast<unsigned long long>(order_key(score)) << 32) |
+                      static_cast<uint32_t>(~static_cast<uint32_t>(v));
+                }
+                __syncwarp();
+              }
             }
           }
-          flush();
           // A tile adds at most 128 entries per list: cut the lists that might
           // overflow on the next one to their top k and raise the threshold.
           tc::named_sync(1 + half, 128);
@@ -557,21 +556,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
       }
       if (!SAMPLE && alive) {
-        // Publish: lists that fit go out as they are, longer ones cut to the top k.
-        for (int c = quad; c < cols; c += 4) {
-          if (q0 + c >= a.nq) break;
-          unsigned long long* list = lists + static_cast<long long>(c) * CAP;
-          const long long out = ((q0 + c) * (2LL * a.n_ranges) + 2 * r + rank) * a.list_len;
-          int n = s_cnt[c];
-          if (n > a.list_len) {
-            cut_any<CAP>(list, n, a.k, lane);
-            __syncwarp();
-            n = a.k;
+        // Publish: lists that fit go out as they are, longer ones cut to the top
+        // k; four lists at a time, so that their loads overlap.
+        constexpr int kAtOnce = 4;
+        for (int base_c = quad; base_c < cols; base_c += 4 * kAtOnce) {
+          int n[kAtOnce];
+#pragma unroll
+          for (int j = 0; j < kAtOnce; ++j) {
+            const int c = base_c + 4 * j;
+            n[j] = c < cols && q0 + c < a.nq ? s_cnt[c] : -1;
+            if (n[j] > a.list_len) {
+              cut_any<CAP>(lists + static_cast<long long>(c) * CAP, n[j], a.k, lane);
+              __syncwarp();
+              n[j] = a.k;
+            }
           }
           for (int i = lane; i < a.list_len; i += kWarp) {
-            const unsigned long long key = i < n ? __ldcg(list + i) : 0ull;
-            a.cand_score[out + i] = i < n ? key_score(static_cast<uint32_t>(key >> 32)) : -INFINITY;
-            a.cand_id[out + i] = ~static_cast<uint32_t>(key);
+            unsigned long long key[kAtOnce];
+#pragma unroll
+            for (int j = 0; j < kAtOnce; ++j) {
+              key[j] = i < n[j] ? __ldcg(lists + static_cast<long long>(base_c + 4 * j) * CAP + i) : 0ull;
+            }
+#pragma unroll
+            for (int j = 0; j < kAtOnce; ++j) {
+              if (n[j] >= 0) {
+                const long long out = ((q0 + base_c + 4 * j) * (2LL * a.n_ranges) + 2 * r + rank) * a.list_len;
+                a.cand_score[out + i] = i < n[j] ? key_score(static_cast<uint32_t>(key[j] >> 32)) : -INFINITY;
+                a.cand_id[out + i] = ~static_cast<uint32_t>(key[j]);
+              }
+            }
           }
         }
       }
@@ -675,15 +688,22 @@ bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, O
   const long long items = static_cast<long long>(plan->q_tiles) * plan->n_ranges;
   plan->ctas = static_cast<int>(2 * std::min<long long>(pairs, items));
   plan->cap = k <= 64 ? 256 : 512;
-  plan->list_len = k + 16;
-  // Thresholds: the k-th best of a sample of whole tiles spread over the index,
-  // 1/64 of it within [1024, 16384] vectors and 64 MiB of scores.
-  long long sample = n / 64;
-  sample = std::min<long long>(sample, 16384);
-  sample = std::min<long long>(sample, (64LL << 20) / 4 / nq);
+  // Thresholds: the k-th best of a sample of whole tiles spread over the index.
+  // About n k / sample scores per query then pass them and cost the epilogue
+  // some hundred clocks each per warp, which rows of few stages (768 clocks of
+  // MMA each) do not hide: at least 8192 k / stages vectors, 1/64 of the index,
+  // at most 1/16 of it, 32768 vectors and 128 MiB of scores. (1000 queries x
+  // 100k x 128, k = 10: scan + sample + selection 261 + 23 + 13 us with 1536
+  // vectors, 188 + 35 + 25 us with the rule's 6144.)
+  const long long n_stages = (nbg + kStageGroupsTc - 1) / kStageGroupsTc;
+  long long sample = std::max<long long>(n / 64, 8192LL * k / n_stages);
+  sample = std::min<long long>({sample, n / 16, 32768, (128LL << 20) / 4 / nq});
   sample = std::max<long long>(sample, 1024);
   plan->sample_tiles = static_cast<int>(std::min<long long>(plan->tiles, sample / kPairVectors));
   plan->sample_step = plan->tiles / plan->sample_tiles;
+  // Published lists: room for what usually passes, so that few need a cut.
+  const long long expect = n * k / (static_cast<long long>(plan->sample_tiles) * kPairVectors * 2 * plan->n_ranges);
+  plan->list_len = k + (2 * expect <= k ? 0 : 16);
   return true;
 }
 
