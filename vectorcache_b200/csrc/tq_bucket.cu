@@ -1012,9 +1012,14 @@ __global__ void item_build_kernel(PairArgs a) {
   if (b >= a.nb) return;
   const unsigned long long c = a.pair_start[b + 1] - a.pair_start[b];
   const unsigned long long i0 = a.item_start[b];
-  for (unsigned long long t = 0; t * kItemQueries < c; ++t) {
-    const unsigned long long first = a.pair_start[b] + t * kItemQueries;
-    const unsigned long long cnt = min(static_cast<unsigned long long>(kItemQueries), c - t * kItemQueries);
+  unsigned long long per = static_cast<unsigned long long>(a.item_queries);
+  if (a.even_items && c > per) {
+    const unsigned long long parts = (c + per - 1) / per;
+    per = (c + parts - 1) / parts;
+  }
+  for (unsigned long long t = 0; t * per < c; ++t) {
+    const unsigned long long first = a.pair_start[b] + t * per;
+    const unsigned long long cnt = min(per, c - t * per);
     a.items[i0 + t] = make_uint4(static_cast<unsigned>(b), static_cast<unsigned>(first),
                                  static_cast<unsigned>(cnt), 0u);
   }
@@ -1468,6 +1473,39 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5) bucket_scan_kernel(BucketSca
   }
 }
 
+// launch_bucket_redo: probe by probe with the same item code, so at most k
+// entries per probe are appended and the region holds them all.
+template <bool NIBBLE8, bool WHOLE>
+__global__ void __launch_bounds__(kBsWarps * 32, 5)
+    bucket_redo_kernel(BucketScanArgs a, const uint32_t* probes, int probe_stride, const uint32_t* n_probe, int fixed_probe) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ ItemQueries iq;
+  const int q = static_cast<int>(blockIdx.x);
+  const long long region = static_cast<long long>(a.max_probe) * kBsListsPerProbe * a.k;
+  if (a.append_count[q] <= region) return;  // the whole CTA
+  __syncthreads();
+  if (threadIdx.x == 0) a.append_count[q] = 0u;
+  const int np = n_probe ? min(static_cast<int>(n_probe[q]), a.max_probe) : fixed_probe;
+  for (int j = 0; j < np; ++j) {
+    const uint32_t b = probes[static_cast<long long>(q) * probe_stride + j];
+    if (b == 0xffffffffu) continue;
+    __syncthreads();  // the previous probe is done with iq and the LUT area
+    if (threadIdx.x < kItemQueries) {
+      const int t = threadIdx.x;
+      iq.q[t] = t == 0 ? q : -1;
+      iq.list[t] = t == 0 ? static_cast<long long>(q) * a.max_probe * kBsListsPerProbe : 0;
+      iq.scale[t] = t == 0 ? a.lut_scale[q] : 0.f;
+      iq.init[t] = t == 0 ? a.fa_init[q] : 0.f;
+      iq.off[t] = t == 0 ? a.offsets[static_cast<long long>(q) * a.max_probe + j] : 0.f;
+      iq.floor[t] = t == 0 && a.floor ? a.floor[q] : -INFINITY;
+    }
+    __syncthreads();
+    const ItemView v{a.codes, a.alpha, a.slot_ids, static_cast<long long>(a.slot_start[b]),
+                     static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, 1, a.cand_score, a.cand_id, a.append_count};
+    scan_item<NIBBLE8, kBsQueriesPerWarp, WHOLE>(v, iq, smem);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Multi-index persistent scan: a fixed grid of CTAs pulls work items — (flat
 // index, vector range, up to 8 of its queries) — from a global counter until
@@ -1714,7 +1752,7 @@ cudaError_t launch_build_pairs(const PairArgs& a, cudaStream_t stream) {
     pair_count_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  prefix_kernel<<<1, 1024, 0, stream>>>(a.counts, a.nb, a.pair_start, kItemQueries, a.item_start, a.n_items);
+  prefix_kernel<<<1, 1024, 0, stream>>>(a.counts, a.nb, a.pair_start, a.item_queries, a.item_start, a.n_items);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (total > 0) {
     pair_scatter_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a);
@@ -1838,14 +1876,30 @@ cudaError_t launch_multi_scan(const MultiScanArgs& a, int ctas, size_t smem_byte
   return cudaGetLastError();
 }
 
+static size_t bucket_scan_smem(int nbg, int k) {
+  const int chunk = nbg < kFlushGroups ? nbg : kFlushGroups;
+  return static_cast<size_t>(kItemQueries) * chunk * 32 +
+         static_cast<size_t>(kBsWarps) * (static_cast<size_t>(kBsQueriesPerWarp) * kmax_of(k) * 8 + kBsBuf * 8);
+}
+
+cudaError_t launch_bucket_redo(const BucketScanArgs& a, long long nq, const uint32_t* probes, int probe_stride,
+                               const uint32_t* n_probe, int fixed_probe, cudaStream_t stream) {
+  if (nq <= 0) return cudaSuccess;
+  if (a.k < 1 || a.k > kMaxK || !a.append_count) return cudaErrorInvalidValue;
+  const size_t smem = bucket_scan_smem(a.nbg, a.k);
+  const bool whole = a.nbg % kBsPrefetch == 0;
+  auto kern = a.bits == 3 ? (whole ? bucket_redo_kernel<true, true> : bucket_redo_kernel<true, false>)
+                          : (whole ? bucket_redo_kernel<false, true> : bucket_redo_kernel<false, false>);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e != cudaSuccess) return e;
+  kern<<<static_cast<unsigned>(nq), kBsWarps * 32, smem, stream>>>(a, probes, probe_stride, n_probe, fixed_probe);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStream_t stream) {
   if (grid <= 0) return cudaSuccess;
   if (a.k < 1 || a.k > kMaxK || a.next_item == nullptr) return cudaErrorInvalidValue;
-  const int chunk = a.nbg < kFlushGroups ? a.nbg : kFlushGroups;
-  const int kmax = kmax_of(a.k);
-  const size_t smem =
-      static_cast<size_t>(kItemQueries) * chunk * 32 +
-      static_cast<size_t>(kBsWarps) * (static_cast<size_t>(kBsQueriesPerWarp) * kmax * 8 + kBsBuf * 8);
+  const size_t smem = bucket_scan_smem(a.nbg, a.k);
   // Whole rings when nbg is a multiple of the ring (no bounds checks).
   const bool whole = a.nbg % kBsPrefetch == 0;
   auto kern = a.bits == 3 ? (whole ? bucket_scan_kernel<true, true> : bucket_scan_kernel<true, false>)

@@ -149,6 +149,9 @@ struct PairArgs {
   // probes, else kFloorProbes (at most its n_probe).
   int first_split = 0;
   int wide_from = kFloorWideFrom;
+  // Queries per work item; even_items: a bucket's pairs split evenly.
+  int item_queries = kItemQueries;
+  bool even_items = false;
 };
 // Groups the (query, probe) pairs by bucket and builds the scan work items.
 cudaError_t launch_build_pairs(const PairArgs& a, cudaStream_t stream);
@@ -182,6 +185,19 @@ struct BucketScanArgs {
 };
 // `grid`: a bound of the item count; the launch runs min(grid, resident CTAs).
 cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStream_t stream);
+// The same items (PairArgs::item_queries = kOneHotItemQueries, even_items) on the
+// tensor cores (tq_onehot.cu): every score at or above its query's floor is
+// appended to the query's region, without the lists of k; append_count may end
+// above the region's size, where the appends past its end are missing.
+constexpr int kOneHotItemQueries = 192;
+constexpr long long kOneHotPairsPerBucket = 48;
+cudaError_t launch_onehot_buckets(const BucketScanArgs& a, long long nq, long long n_slots, int sms, unsigned* status,
+                                  cudaStream_t stream);
+// Scans again, list by list, every query whose append_count passed its region:
+// all its probes (n_probe[q], or fixed_probe), from an empty region. One CTA per
+// query; the others return at once.
+cudaError_t launch_bucket_redo(const BucketScanArgs& a, long long nq, const uint32_t* probes, int probe_stride,
+                               const uint32_t* n_probe, int fixed_probe, cudaStream_t stream);
 // floor[q] = the k-th largest score (above -inf) among the first count[q]
 // (count null: all `stride`) candidates of query q's region (cand + q * stride), -inf when there are
 // fewer than k: the k-th score of their merged top k, a lower bound of the

@@ -568,9 +568,29 @@ struct tq_bucketed {
       }
       const long long last_items =
           two_phase ? std::min(items, vcb::max_items(static_cast<long long>(m), max_probe - 1, nb)) : items;
+      // The far probes hold most pairs: with enough of them per bucket they go
+      // to the tensor cores, above the floors.
+      const long long far_pairs = static_cast<long long>(m) * (max_probe - first);
+      const bool onehot = two_phase && far_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2;
+      if (onehot) {
+        pa.item_queries = vcb::kOneHotItemQueries;
+        pa.even_items = true;
+      }
       eng->launch(tq_index::kPrep, s, "pair kernels", [&] { return vcb::launch_build_pairs(pa, s); });
-      eng->launch(tq_index::kScan, s, "bucket scan kernel",
-                  [&] { return vcb::launch_bucket_scan(ba, last_items, s); });
+      if (onehot) {
+        eng->check_status = true;
+        eng->status_foreign |= s != eng->stream;
+        eng->launch(tq_index::kScan, s, "bucket scan kernel", [&] {
+          return vcb::launch_onehot_buckets(ba, static_cast<long long>(m), static_cast<long long>(n_slots), eng->sms,
+                                            eng->device_status(), s);
+        });
+        eng->launch(tq_index::kScan, s, "bucket redo kernel", [&] {
+          return vcb::launch_bucket_redo(ba, static_cast<long long>(m), pa.probes, ptop, np_pass, max_probe, s);
+        });
+      } else {
+        eng->launch(tq_index::kScan, s, "bucket scan kernel",
+                    [&] { return vcb::launch_bucket_scan(ba, last_items, s); });
+      }
       vcb::MergeArgs mg{};
       mg.cand_score = ba.cand_score;
       mg.cand_id = ba.cand_id;

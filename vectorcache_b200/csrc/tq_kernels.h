@@ -226,6 +226,17 @@ struct OneHotArgs {
   float* dense;         // sample: nq x dense_stride scores
   long long dense_stride;
   unsigned* status;     // device word, set to 1 when a wait gave up
+  // Bucket items (launch_onehot_buckets): see BucketScanArgs in tq_bucket.h.
+  const uint4* items;
+  const unsigned long long* n_items;
+  const uint32_t* pairs;
+  const float* offsets;
+  const uint32_t* slot_ids;
+  const unsigned long long* slot_start;
+  const uint32_t* bucket_size;
+  uint32_t* append_count;
+  uint32_t region;      // entries a query's candidate region holds
+  int max_probe;
   // set by the launchers
   int tile_queries, q_tiles, tiles, tile_step, range_tiles, n_ranges, list_len;
 };

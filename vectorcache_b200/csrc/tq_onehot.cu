@@ -31,6 +31,7 @@
 
 #include <cuda.h>
 
+#include "tq_bucket.h"
 #include "tq_device.cuh"
 #include "tq_kernels.h"
 #include "tq_tc.cuh"
@@ -66,16 +67,25 @@ constexpr int kRegsLaunch = 96, kRegsProducer = 64, kRegsEpilogue = 152, kRegsIs
 static_assert(256 * (kRegsProducer + kRegsEpilogue) + 128 * kRegsIssue <= kThreads * kRegsLaunch,
               "the register split must fit what the block is launched with");
 
+enum Mode { kSample, kTopK, kBucket };
+
+// One item's queries and vectors (bucket mode: three items in flight).
+constexpr int kParams = 3;
+struct Params {
+  float scale[kMaxN], init[kMaxN], thr[kMaxN], off[kMaxN];
+  int q[kMaxN];   // LUT rows
+  int tiles, cols, size, vt0;
+};
+
 struct Shared {
   uint64_t full_b[kStagesB], empty_b[kStagesB];
   uint64_t full_a[kMaxStagesA], empty_a[kMaxStagesA];
   uint64_t full_c[kStagesC], empty_c[kStagesC];
   uint64_t acc_full[2], acc_empty[2];
+  uint64_t full_p[kParams], empty_p[kParams];
   uint32_t tmem;
   uint32_t pad[3];
-  float scale[kMaxN];
-  float init[kMaxN];
-  float thr[kMaxN];
+  Params par[kParams];
   int cnt[kMaxN];
   // 32 queries' scores of an epilogue warp's 32 vectors.
   float stage[8][32][32];
@@ -165,12 +175,23 @@ __device__ __forceinline__ void onehot16(uint32_t x, uint32_t* out) {
   out[3] = static_cast<uint32_t>(hi >> 32);
 }
 
-// SAMPLE: write every score of the sampled tiles (thresholds come from them).
-// Otherwise keep each query's top k of the range; CAP entries per list.
-template <bool SAMPLE, int CAP>
+// One role's view of a work item.
+struct Item {
+  int tiles;    // 256-vector tiles
+  int vt0, step;
+  int cols;     // queries (a multiple of 32)
+  int y;        // first LUT row (consecutive rows; not in bucket mode)
+};
+
+// kSample: write every score of the sampled tiles (thresholds come from them).
+// kTopK: keep each query's top k of the item's range; CAP entries per list.
+// kBucket: items are (bucket, up to 192 of its probing queries); the LUT rows are
+// gathered, and scores at or above the query's floor are appended to its region.
+template <int MODE, int CAP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     onehot_scan_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap code_map,
-                       OneHotArgs a) {
+                       const __grid_constant__ OneHotArgs a) {
+  constexpr bool SAMPLE = MODE == kSample;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t{1023});
   unsigned char* codes_smem = base + static_cast<size_t>(kStagesB) * 2 * kTileB;
@@ -181,9 +202,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int n_stages = (a.nbg + kStageGroupsTc - 1) / kStageGroupsTc;
   const int n_batches = (a.nbg + kFlushGroups - 1) / kFlushGroups;
-  const int items = a.q_tiles * a.n_ranges;
+  const int items = MODE == kBucket ? static_cast<int>(*a.n_items) : a.q_tiles * a.n_ranges;
   // TMEM: two accumulators of acc_cols columns, then the one-hot stages.
-  const uint32_t acc_cols = a.tile_queries <= 128 ? 128 : kMaxN;
+  const uint32_t acc_cols = MODE != kBucket && a.tile_queries <= 128 ? 128 : kMaxN;
   const int stages_a = acc_cols == 128 ? kMaxStagesA : 2;
 
   if (threadIdx.x == 0) {
@@ -203,6 +224,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       tc::mbar_init(tc::smem_u32(&sh.acc_full[b]), 1);
       tc::mbar_init(tc::smem_u32(&sh.acc_empty[b]), 16);  // eight epilogue warps of each CTA
     }
+    for (int b = 0; b < kParams; ++b) {
+      tc::mbar_init(tc::smem_u32(&sh.full_p[b]), 1);
+      // producers, epilogue, LUT and code loaders (and the issuing warp)
+      tc::mbar_init(tc::smem_u32(&sh.empty_p[b]), rank == 0 ? 19 : 18);
+    }
     tc::mbar_init_fence();
     tc::prefetch_map(&lut_map);
     tc::prefetch_map(&code_map);
@@ -218,6 +244,42 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const uint32_t tmem = sh.tmem;
   bool alive = true;  // false: a wait gave up; this role stops
 
+  // Every role walks the same items: number pair, pair + pairs, ... In bucket mode
+  // their parameters come through shared memory (warp 19 fills them in).
+  int pb = 0;
+  uint32_t pp = 0;
+  auto open_item = [&](int it) -> Item {
+    Item x{};
+    if constexpr (MODE == kBucket) {
+      if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.full_p[pb]), pp))) {
+        alive = false;
+        return x;
+      }
+      x.tiles = sh.par[pb].tiles;
+      x.vt0 = sh.par[pb].vt0;
+      x.step = 1;
+      x.cols = sh.par[pb].cols;
+    } else {
+      const int qt = it / a.n_ranges, t0 = (it % a.n_ranges) * a.range_tiles;
+      x.tiles = min(a.range_tiles, a.tiles - t0);
+      x.step = a.tile_step > 0 ? a.tile_step : 1;
+      x.vt0 = t0 * x.step;
+      x.cols = a.tile_queries;
+      x.y = qt * a.tile_queries;
+    }
+    return x;
+  };
+  auto close_item = [&]() {
+    if constexpr (MODE == kBucket) {
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(tc::smem_u32(&sh.empty_p[pb]));
+      if (++pb == kParams) {
+        pb = 0;
+        pp ^= 1u;
+      }
+    }
+  };
+
   if (warp < 8) {
     // ---- one-hot rows: set `set` builds its half of every stage; TMEM lane
     // 32 quad + lane holds vector 4 lane + quad of this CTA's 128.
@@ -229,9 +291,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     int slot = 0, sc = 0;
     uint32_t ph = 0, pc = 0;
     for (int it = pair; it < items && alive; it += pairs) {
-      const int r = it % a.n_ranges;
-      const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
-      for (int t = t0; t < t1 && alive; ++t) {
+      const Item x = open_item(it);
+      for (int t = 0; t < x.tiles && alive; ++t) {
         for (int s0 = 0; s0 < n_stages && alive; s0 += kChunkStages) {
           if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.full_c[sc]), pc))) {
             alive = false;
@@ -252,9 +313,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
               // high nibble (first half of the LUT row), then the low one
-              const uint32_t x = __funnelshift_r(w[g], w[g], rot);
-              onehot16(x >> 16, row[0] + 8 * g);
-              onehot16(x, row[0] + 8 * g + 4);
+              const uint32_t v = __funnelshift_r(w[g], w[g], rot);
+              onehot16(v >> 16, row[0] + 8 * g);
+              onehot16(v, row[0] + 8 * g + 4);
             }
             if (!__all_sync(full_mask(), ready || tc::mbar_wait(bar, ph ^ 1u))) {
               alive = false;
@@ -264,9 +325,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             tc::tmem_st16(dst0 + slot * kStageColsA, row[0]);
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
-              const uint32_t x = __funnelshift_r(w[2 + g], w[2 + g], rot);
-              onehot16(x >> 16, row[1] + 8 * g);
-              onehot16(x, row[1] + 8 * g + 4);
+              const uint32_t v = __funnelshift_r(w[2 + g], w[2 + g], rot);
+              onehot16(v >> 16, row[1] + 8 * g);
+              onehot16(v, row[1] + 8 * g + 4);
             }
             tc::tmem_st16(dst0 + slot * kStageColsA + kHalfColsA / 2, row[1]);
             tc::tmem_wait_st();
@@ -286,6 +347,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           }
         }
       }
+      close_item();
     }
     __syncwarp();
   } else if (warp >= 16) {
@@ -295,21 +357,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       int st = 0;
       uint32_t ph = 0;
       for (int it = pair; it < items && alive; it += pairs) {
-        const int qt = it / a.n_ranges, r = it % a.n_ranges;
-        const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
-        const int y = qt * a.tile_queries + static_cast<int>(rank) * (a.tile_queries / 2);
-        for (int t = t0; t < t1 && alive; ++t) {
+        const Item x = open_item(it);
+        const int half_rows = x.cols / 2;
+        int4 rows = make_int4(0, 0, 0, 0);
+        const bool gathers = MODE == kBucket && lane * 4 < half_rows;
+        if (gathers) rows = *reinterpret_cast<const int4*>(&sh.par[pb].q[rank * kHalfN + lane * 4]);
+        for (int t = 0; t < x.tiles && alive; ++t) {
           for (int s = 0; s < n_stages; ++s) {
             if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) {
               alive = false;
               break;
             }
             const uint32_t bar = tc::smem_u32(&sh.full_b[st]);
-            if (tc::elect_one()) {
-              if (rank == 0) tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(a.tile_queries) * 256u);
-              const uint32_t cbar = tc::mapa(bar, 0);
-              tc::tma_load_2d_pair(sB + st * 2 * kTileB, &lut_map, s * 256, y, cbar);
-              tc::tma_load_2d_pair(sB + (st * 2 + 1) * kTileB, &lut_map, s * 256 + 128, y, cbar);
+            const uint32_t dst = sB + st * 2 * kTileB, cbar = tc::mapa(bar, 0);
+            if constexpr (MODE == kBucket) {
+              // The second half of the last stage may lie past the row.
+              const bool second = s * kStageGroupsTc + kHalfGroups < a.nbg;
+              if (rank == 0 && lane == 0) {
+                tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(x.cols) * (second ? 256u : 128u));
+              }
+              __syncwarp();
+              if (gathers) {
+                tc::tma_gather4_pair(dst + lane * 512, &lut_map, s * 256, rows, cbar);
+                if (second) tc::tma_gather4_pair(dst + kTileB + lane * 512, &lut_map, s * 256 + 128, rows, cbar);
+              }
+            } else if (tc::elect_one()) {
+              const int y = x.y + static_cast<int>(rank) * half_rows;
+              if (rank == 0) tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(x.cols) * 256u);
+              tc::tma_load_2d_pair(dst, &lut_map, s * 256, y, cbar);
+              tc::tma_load_2d_pair(dst + kTileB, &lut_map, s * 256 + 128, y, cbar);
             }
             __syncwarp();
             if (++st == kStagesB) {
@@ -318,6 +394,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
           }
         }
+        close_item();
       }
     } else if (warp == 18) {
       // ---- code chunks: 32 rows (byte groups) x 32 words of the scan layout.
@@ -325,10 +402,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       int sc = 0;
       uint32_t ph = 0;
       for (int it = pair; it < items && alive; it += pairs) {
-        const int r = it % a.n_ranges;
-        const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
-        for (int t = t0; t < t1 && alive; ++t) {
-          const int vt = a.tile_step > 0 ? t * a.tile_step : t;
+        const Item x = open_item(it);
+        for (int t = 0; t < x.tiles && alive; ++t) {
+          const int vt = x.vt0 + t * x.step;
           for (int g0 = 0; g0 < a.nbg; g0 += kChunkGroups) {
             if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_c[sc]), ph ^ 1u))) {
               alive = false;
@@ -347,16 +423,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
           }
         }
+        close_item();
       }
     } else if (warp == 17 && rank == 0) {
       // ---- MMA ---------------------------------------------------------------
-      const uint32_t idesc = (2u << 4) | (static_cast<uint32_t>(a.tile_queries >> 3) << 17) | (16u << 24);
       int sa = 0, sb = 0;
       uint32_t pa = 0, pb = 0, batch = 0;
       for (int it = pair; it < items && alive; it += pairs) {
-        const int r = it % a.n_ranges;
-        const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
-        for (int t = t0; t < t1 && alive; ++t) {
+        const Item x = open_item(it);
+        const uint32_t idesc = (2u << 4) | (static_cast<uint32_t>(x.cols >> 3) << 17) | (16u << 24);
+        for (int t = 0; t < x.tiles && alive; ++t) {
           for (int s0 = 0; s0 < n_stages && alive; s0 += kBatchStages, ++batch) {
             const uint32_t buf = batch & 1u;
             const uint32_t d = tmem + buf * acc_cols;
@@ -403,6 +479,48 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
           }
         }
+        close_item();
+      }
+    } else if (MODE == kBucket && warp == 19) {
+      // ---- bucket items: the queries' constants, up to three items ahead -------
+      for (int it = pair; it < items && alive; it += pairs) {
+        if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_p[pb]), pp ^ 1u))) {
+          alive = false;
+          break;
+        }
+        Params& p = sh.par[pb];
+        const uint4 e = a.items[it];  // bucket, first pair, pairs
+        const int count = static_cast<int>(e.z), cols = (count + 31) / 32 * 32;
+        for (int c = lane; c < cols; c += kWarp) {
+          const int at = c < cols / 2 ? c : kHalfN + c - cols / 2;
+          int q = 0;
+          float scale = 0.f, init = 0.f, off = 0.f, thr = INFINITY;  // a column of no query
+          if (c < count) {
+            const uint32_t pr = a.pairs[e.y + c];
+            q = static_cast<int>(pr / static_cast<uint32_t>(a.max_probe));
+            scale = a.lut_scale[q];
+            init = a.fa_init[q];
+            off = a.offsets[pr];
+            thr = fmaxf(-FLT_MAX, a.floor[q]);
+          }
+          p.q[at] = q;
+          p.scale[at] = scale;
+          p.init[at] = init;
+          p.off[at] = off;
+          p.thr[at] = thr;
+        }
+        if (lane == 0) {
+          p.size = static_cast<int>(a.bucket_size[e.x]);
+          p.tiles = (p.size + kPairVectors - 1) / kPairVectors;
+          p.vt0 = static_cast<int>(a.slot_start[e.x] / kPairVectors);
+          p.cols = cols;
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(tc::smem_u32(&sh.full_p[pb]));
+        if (++pb == kParams) {
+          pb = 0;
+          pp ^= 1u;
+        }
       }
     }
     __syncwarp();
@@ -410,37 +528,47 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     // ---- epilogue: warp quadrant = 32 vectors, half = N / 2 queries ------------
     tc::reg_inc<kRegsEpilogue>();
     const int quad = warp & 3, half = (warp - 8) >> 2;
-    const int cols = a.tile_queries / 2;       // this half's queries, a multiple of 16
-    const int c0 = half * cols;
-    const uint32_t t_base = tmem + (static_cast<uint32_t>(quad * 32) << 16) + c0;
-    unsigned long long* lists = a.lists + (static_cast<long long>(blockIdx.x) * a.tile_queries + c0) * CAP;
-    const float* s_scale = sh.scale + half * kHalfN;
-    const float* s_init = sh.init + half * kHalfN;
-    float* s_thr = sh.thr + half * kHalfN;
+    const long long list0 = (static_cast<long long>(blockIdx.x) * a.tile_queries + half * (a.tile_queries / 2)) * CAP;
+    unsigned long long* lists = MODE == kTopK ? a.lists + list0 : nullptr;
     int* s_cnt = sh.cnt + half * kHalfN;
     float* stage = &sh.stage[warp - 8][0][lane];
     const int ht = (warp & 3) * 32 + lane;  // thread of the half
     uint32_t batch = 0;
-    for (int it = pair; it < items; it += pairs) {
-      const int qt = it / a.n_ranges, r = it % a.n_ranges;
-      const int t0 = r * a.range_tiles, t1 = min(t0 + a.range_tiles, a.tiles);
-      const long long q0 = static_cast<long long>(qt) * a.tile_queries + c0;
-      tc::named_sync(1 + half, 128);
-      if (ht < cols) {
-        const bool ok = q0 + ht < a.nq;
-        sh.scale[half * kHalfN + ht] = ok ? a.lut_scale[q0 + ht] : 0.f;
-        sh.init[half * kHalfN + ht] = ok ? a.fa_init[q0 + ht] : 0.f;
-        // -FLT_MAX admits every score above -inf; NaN never compares >=.
-        float th = -FLT_MAX;
-        if (!SAMPLE && ok && a.floor) th = fmaxf(th, a.floor[q0 + ht]);
-        s_thr[ht] = ok ? th : INFINITY;
-        s_cnt[ht] = 0;
+    // A warp whose wait gave up goes on through the barriers it shares.
+    for (int it = pair; it < items && (alive || MODE != kBucket); it += pairs) {
+      const Item x = open_item(it);
+      const int cols = x.cols / 2;  // this half's queries, a multiple of 16
+      const int c0 = half * cols;
+      const uint32_t t_base = tmem + (static_cast<uint32_t>(quad * 32) << 16) + c0;
+      const Params& par = sh.par[pb];
+      const float* s_scale = par.scale + half * kHalfN;
+      const float* s_init = par.init + half * kHalfN;
+      float* s_thr = sh.par[pb].thr + half * kHalfN;
+      const long long q0 = x.y + c0;
+      if constexpr (MODE != kBucket) {
+        tc::named_sync(1 + half, 128);
+        if (ht < cols) {
+          const bool ok = q0 + ht < a.nq;
+          sh.par[0].scale[half * kHalfN + ht] = ok ? a.lut_scale[q0 + ht] : 0.f;
+          sh.par[0].init[half * kHalfN + ht] = ok ? a.fa_init[q0 + ht] : 0.f;
+          // -FLT_MAX admits every score above -inf; NaN never compares >=.
+          float th = -FLT_MAX;
+          if (!SAMPLE && ok && a.floor) th = fmaxf(th, a.floor[q0 + ht]);
+          s_thr[ht] = ok ? th : INFINITY;
+          s_cnt[ht] = 0;
+        }
+        tc::named_sync(1 + half, 128);
       }
-      tc::named_sync(1 + half, 128);
-      for (int t = t0; t < t1; ++t) {
-        const long long vt = a.tile_step > 0 ? static_cast<long long>(t) * a.tile_step : t;
-        const long long v = vt * kPairVectors + rank * 128 + 4 * lane + quad;
-        const bool valid = v < a.n;
+      for (int t = 0; t < x.tiles; ++t) {
+        const long long v = (static_cast<long long>(x.vt0) + t * x.step) * kPairVectors + rank * 128 + 4 * lane + quad;
+        bool valid;
+        uint32_t id = static_cast<uint32_t>(v);
+        if constexpr (MODE == kBucket) {
+          valid = v - static_cast<long long>(x.vt0) * kPairVectors < par.size;
+          if (valid) id = __ldg(a.slot_ids + v);
+        } else {
+          valid = v < a.n;
+        }
         const float al = valid ? __ldg(a.alpha + v) : 0.f;
         float fa[kHalfN];
 #pragma unroll
@@ -458,7 +586,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         for (int b = 0; b < n_batches; ++b, ++batch) {
           const uint32_t buf = batch & 1u;
-          // A warp whose wait gave up goes on through the barriers it shares.
           if (alive) alive = __all_sync(full_mask(), tc::mbar_wait_long(tc::smem_u32(&sh.acc_full[buf]), (batch >> 1) & 1u));
           tc::fence_after();
 #pragma unroll
@@ -485,7 +612,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&sh.acc_empty[buf]), 0));
         }
         if (SAMPLE) {
-          const long long at = static_cast<long long>(t) * kPairVectors + rank * 128 + quad * 32 + lane;
+          const long long at =
+              (static_cast<long long>(it % a.n_ranges) * a.range_tiles + t) * kPairVectors + rank * 128 + quad * 32 + lane;
 #pragma unroll
           for (int c = 0; c < kHalfN / 16; ++c) {
             if (c * 16 < cols) {
@@ -512,9 +640,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
               for (int i = 0; i < 32; i += 4) {
                 const float4 f = *reinterpret_cast<const float4*>(s_thr + c * 32 + i);
                 const float th[4] = {f.x, f.y, f.z, f.w};
+                [[maybe_unused]] float of[4];
+                if constexpr (MODE == kBucket) {
+                  const float4 o = *reinterpret_cast<const float4*>(par.off + half * kHalfN + c * 32 + i);
+                  of[0] = o.x;
+                  of[1] = o.y;
+                  of[2] = o.z;
+                  of[3] = o.w;
+                }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                   fa[c * 32 + i + u] = __fmul_rn(fa[c * 32 + i + u], al_top);
+                  if constexpr (MODE == kBucket) fa[c * 32 + i + u] = __fadd_rn(fa[c * 32 + i + u], of[u]);
                   if (fa[c * 32 + i + u] >= th[u]) part[u] |= 1u << (i + u);
                 }
               }
@@ -526,16 +663,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 while (hits) {
                   const int i = __ffs(hits) - 1;
                   hits &= hits - 1;
-                  const float score = __fadd_rn(stage[i * 32], 0.f);
-                  const int pos = atomicAdd(&s_cnt[c * 32 + i], 1);
-                  lists[static_cast<long long>(c * 32 + i) * CAP + pos] =
-                      (static_cast<unsigned long long>(order_key(score)) << 32) |
-                      static_cast<uint32_t>(~static_cast<uint32_t>(v));
+                  if constexpr (MODE == kBucket) {
+                    // Past the region's end nothing is written; the count says so.
+                    const int q = par.q[half * kHalfN + c * 32 + i];
+                    const uint32_t pos = atomicAdd(a.append_count + q, 1u);
+                    if (pos < a.region) {
+                      const long long at = static_cast<long long>(q) * a.region + pos;
+                      a.cand_score[at] = stage[i * 32];
+                      a.cand_id[at] = id;
+                    }
+                  } else {
+                    const float score = __fadd_rn(stage[i * 32], 0.f);
+                    const int pos = atomicAdd(&s_cnt[c * 32 + i], 1);
+                    lists[static_cast<long long>(c * 32 + i) * CAP + pos] =
+                        (static_cast<unsigned long long>(order_key(score)) << 32) | static_cast<uint32_t>(~id);
+                  }
                 }
                 __syncwarp();
               }
             }
           }
+          if constexpr (MODE == kTopK) {
           // A tile adds at most 128 entries per list: cut the lists that might
           // overflow on the next one to their top k and raise the threshold.
           tc::named_sync(1 + half, 128);
@@ -553,9 +701,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
           }
           tc::named_sync(1 + half, 128);
+          }
         }
       }
-      if (!SAMPLE && alive) {
+      if (MODE == kTopK && alive) {
+        const int r = it % a.n_ranges;
         // Publish: lists that fit go out as they are, longer ones cut to the top
         // k; four lists at a time, so that their loads overlap.
         constexpr int kAtOnce = 4;
@@ -588,6 +738,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           }
         }
       }
+      close_item();
     }
   }
   if (!alive && a.status) atomicExch(a.status, 1u);
@@ -629,15 +780,16 @@ cudaError_t make_map(CUtensorMapDataType type, const void* p, uint64_t cols, uin
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <bool SAMPLE, int CAP>
+template <int MODE, int CAP>
 cudaError_t launch_t(const OneHotArgs& a, int ctas, cudaStream_t stream) {
-  auto kern = onehot_scan_kernel<SAMPLE, CAP>;
+  auto kern = onehot_scan_kernel<MODE, CAP>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
   if (e != cudaSuccess) return e;
   CUtensorMap luts, codes;
   e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, a.luts, static_cast<uint64_t>(a.nbg) * 32, static_cast<uint64_t>(a.nq),
-               static_cast<uint64_t>(a.nbg) * 32, 128, static_cast<uint32_t>(a.tile_queries / 2),
+               static_cast<uint64_t>(a.nbg) * 32, 128,
+               MODE == kBucket ? 1u : static_cast<uint32_t>(a.tile_queries / 2),  // gathers take one-row boxes
                CU_TENSOR_MAP_SWIZZLE_128B, &luts);
   if (e != cudaSuccess) return e;
   const uint64_t rows = static_cast<uint64_t>((a.n + kTileVectors - 1) / kTileVectors) * static_cast<uint64_t>(a.nbg);
@@ -723,7 +875,7 @@ cudaError_t launch_onehot_sample(const OneHotArgs& in, const OneHotPlan& p, int 
   a.range_tiles = (a.tiles + r - 1) / r;
   a.n_ranges = (a.tiles + a.range_tiles - 1) / a.range_tiles;
   const long long items = static_cast<long long>(a.q_tiles) * a.n_ranges;
-  return launch_t<true, 256>(a, static_cast<int>(2 * std::min<long long>(sms / 2, items)), stream);
+  return launch_t<kSample, 256>(a, static_cast<int>(2 * std::min<long long>(sms / 2, items)), stream);
 }
 
 cudaError_t launch_onehot_scan(const OneHotArgs& in, const OneHotPlan& p, cudaStream_t stream) {
@@ -735,7 +887,38 @@ cudaError_t launch_onehot_scan(const OneHotArgs& in, const OneHotPlan& p, cudaSt
   a.range_tiles = p.range_tiles;
   a.n_ranges = p.n_ranges;
   a.list_len = p.list_len;
-  return p.cap == 256 ? launch_t<false, 256>(a, p.ctas, stream) : launch_t<false, 512>(a, p.ctas, stream);
+  return p.cap == 256 ? launch_t<kTopK, 256>(a, p.ctas, stream) : launch_t<kTopK, 512>(a, p.ctas, stream);
+}
+
+cudaError_t launch_onehot_buckets(const BucketScanArgs& b, long long nq, long long n_slots, int sms, unsigned* status,
+                                  cudaStream_t stream) {
+  if (!b.append_count || !b.floor || b.n_items == nullptr || n_slots > 0x7fffffffLL) return cudaErrorInvalidValue;
+  OneHotArgs a{};
+  a.codes = b.codes;
+  a.alpha = b.alpha;
+  a.luts = b.luts;
+  a.lut_scale = b.lut_scale;
+  a.fa_init = b.fa_init;
+  a.n = n_slots;
+  a.nbg = b.nbg;
+  a.nq = nq;
+  a.k = b.k;
+  a.cand_score = b.cand_score;
+  a.cand_id = b.cand_id;
+  a.floor = b.floor;
+  a.status = status;
+  a.tile_queries = kMaxN;
+  a.items = b.items;
+  a.n_items = b.n_items;
+  a.pairs = b.pairs;
+  a.offsets = b.offsets;
+  a.slot_ids = b.slot_ids;
+  a.slot_start = b.slot_start;
+  a.bucket_size = b.bucket_size;
+  a.append_count = b.append_count;
+  a.region = static_cast<uint32_t>(static_cast<long long>(b.max_probe) * kBsListsPerProbe * b.k);
+  a.max_probe = b.max_probe;
+  return launch_t<kBucket, 256>(a, sms / 2 * 2, stream);
 }
 
 }  // namespace vcb

@@ -126,6 +126,16 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       : "memory");
 }
 
+// Four rows (one-row boxes of the map), 128 bytes each, to consecutive rows of a
+// tile; otherwise as tma_load_2d_pair.
+__device__ __forceinline__ void tma_gather4_pair(uint32_t dst, const CUtensorMap* m, int x, int4 rows, uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+      "l"(m), "r"(cluster_bar), "r"(x), "r"(rows.x), "r"(rows.y), "r"(rows.z), "r"(rows.w)
+      : "memory");
+}
+
 // ---- tcgen05, CTA pairs (cta_group::2) ---------------------------------------
 __device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(columns)
