@@ -60,12 +60,19 @@ constexpr int kTmemCols = 512;
 constexpr int kPairVectors = 256;
 constexpr int kBatchStages = kFlushGroups / kStageGroupsTc;
 // Warps 0-7 build one-hot rows (two sets of four, a TMEM quadrant each), 8-15
-// are the epilogue, 16 loads LUT tiles, 17 issues MMAs, 18 loads codes (19 fills
-// up the warpgroup). Registers: 640 x 96 at launch >= 256 x 64 + 256 x 152 + 128 x 40.
-constexpr int kThreads = 640;
-constexpr int kRegsLaunch = 96, kRegsProducer = 64, kRegsEpilogue = 152, kRegsIssue = 40;
-static_assert(256 * (kRegsProducer + kRegsEpilogue) + 128 * kRegsIssue <= kThreads * kRegsLaunch,
-              "the register split must fit what the block is launched with");
+// are the epilogue, 16 loads LUT tiles, 17 issues MMAs, 18 loads codes (in bucket
+// mode 16, 18, 20 and 21 gather LUT rows and 19 prepares items). ONE: rows of a
+// single 256-group batch, whose sums need no registers between batches: fewer
+// registers per epilogue warp, and four more warps.
+template <bool ONE>
+struct Config {
+  static constexpr int kThreads = ONE ? 768 : 640;
+  static constexpr int kRegsLaunch = ONE ? 80 : 96;
+  static constexpr int kRegsProducer = 64, kRegsEpilogue = ONE ? 128 : 152, kRegsIssue = ONE ? 48 : 40;
+  static_assert(256 * (kRegsProducer + kRegsEpilogue) + (kThreads - 512) * kRegsIssue <= kThreads * kRegsLaunch,
+                "the register split must fit what the block is launched with");
+  static constexpr int kGatherTeams = ONE ? 2 : 1;  // pairs of warps that gather LUT rows
+};
 
 enum Mode { kSample, kTopK, kBucket };
 
@@ -73,7 +80,8 @@ enum Mode { kSample, kTopK, kBucket };
 constexpr int kParams = 3;
 struct Params {
   float scale[kMaxN], init[kMaxN], thr[kMaxN], off[kMaxN];
-  int q[kMaxN];   // LUT rows
+  int q[kMaxN];
+  uint32_t row[kMaxN];  // byte offset of the query's LUT row
   int tiles, cols, size, vt0;
 };
 
@@ -83,6 +91,7 @@ struct Shared {
   uint64_t full_c[kStagesC], empty_c[kStagesC];
   uint64_t acc_full[2], acc_empty[2];
   uint64_t full_p[kParams], empty_p[kParams];
+  uint64_t landed_b[kStagesB];
   uint32_t tmem;
   uint32_t pad[3];
   Params par[kParams];
@@ -186,9 +195,9 @@ struct Item {
 // kSample: write every score of the sampled tiles (thresholds come from them).
 // kTopK: keep each query's top k of the item's range; CAP entries per list.
 // kBucket: items are (bucket, up to 192 of its probing queries); the LUT rows are
-// gathered, and scores at or above the query's floor are appended to its region.
-template <int MODE, int CAP>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+// gathered by cp.async, and scores at or above the query's floor are appended to its region.
+template <int MODE, int CAP, bool ONE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThreads, 1)
     onehot_scan_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap code_map,
                        const __grid_constant__ OneHotArgs a) {
   constexpr bool SAMPLE = MODE == kSample;
@@ -209,7 +218,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStagesB; ++s) {
-      tc::mbar_init(tc::smem_u32(&sh.full_b[s]), 1);
+      tc::mbar_init(tc::smem_u32(&sh.full_b[s]), MODE == kBucket ? 2 : 1);  // bucket mode: each CTA's relay
+      tc::mbar_init(tc::smem_u32(&sh.landed_b[s]), 64);  // two gathering warps
       tc::mbar_init(tc::smem_u32(&sh.empty_b[s]), 1);
     }
     for (int s = 0; s < kMaxStagesA; ++s) {
@@ -226,8 +236,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < kParams; ++b) {
       tc::mbar_init(tc::smem_u32(&sh.full_p[b]), 1);
-      // producers, epilogue, LUT and code loaders (and the issuing warp)
-      tc::mbar_init(tc::smem_u32(&sh.empty_p[b]), rank == 0 ? 19 : 18);
+      // eight producer, eight epilogue and the gathering warps, and the issuing one
+      tc::mbar_init(tc::smem_u32(&sh.empty_p[b]), 16 + 2 * Config<ONE>::kGatherTeams + (rank == 0 ? 1 : 0));
     }
     tc::mbar_init_fence();
     tc::prefetch_map(&lut_map);
@@ -283,7 +293,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   if (warp < 8) {
     // ---- one-hot rows: set `set` builds its half of every stage; TMEM lane
     // 32 quad + lane holds vector 4 lane + quad of this CTA's 128.
-    tc::reg_dec<kRegsProducer>();
+    tc::reg_dec<Config<ONE>::kRegsProducer>();
     const int quad = warp & 3, set = warp >> 2;
     const uint32_t dst0 = tmem + 2 * acc_cols + set * kHalfColsA + (static_cast<uint32_t>(quad * 32) << 16);
     const uint32_t src0 = sC + set * kHalfGroups * 128 + lane * 4;
@@ -351,17 +361,73 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     __syncwarp();
   } else if (warp >= 16) {
-    tc::reg_dec<kRegsIssue>();
-    if (warp == 16) {
+    tc::reg_dec<Config<ONE>::kRegsIssue>();
+    if (MODE == kBucket && (warp == 16 || warp == 18 || (ONE && (warp == 20 || warp == 21)))) {
+      // ---- LUT rows of the item's queries: warp 16 copies the first 128 bytes
+      // of K of every stage, warp 18 the second, 16 bytes a lane, eight lanes a
+      // row, in the 128-byte swizzle (16-byte chunk c of row r at c ^ (r % 8)); the
+      // copies arrive at landed_b themselves and warp 19 passes them on.
+      // A one-row-box TMA gather (tile::gather4) took about 77 clocks per four
+      // rows and bound the kernel (10k queries x 464 probes of 1.2M x 100: 8.8 ms
+      // against GATHER_MS). Warp 16 also loads the code chunks.
+      // Two pairs of warps (ONE) take the stages in turn.
+      const int which = warp == 18 || warp == 21;
+      const int team = warp >= 20;
+      const uint32_t rl = lane >> 3, cl = lane & 7;
+      const uint32_t dst_even = rl * 128 + ((cl ^ rl) << 4), dst_odd = rl * 128 + ((cl ^ (rl + 4)) << 4);
+      const uint32_t row_bytes = static_cast<uint32_t>(a.nbg) * 32;
+      int st = 0, sc = 0;
+      uint32_t ph = 0, pc = 0;
+      for (int it = pair; it < items && alive; it += pairs) {
+        const Item x = open_item(it);
+        const int groups4 = x.cols / 8;  // four rows at a time
+        const uint32_t* row = &sh.par[pb].row[rank * kHalfN + rl];
+        for (int t = 0; t < x.tiles && alive; ++t) {
+          for (int s = 0; s < n_stages && alive; ++s) {
+            if (warp == 16 && s % kChunkStages == 0) {
+              if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_c[sc]), pc ^ 1u))) alive = false;
+              if (alive && tc::elect_one()) {
+                const uint32_t bar = tc::smem_u32(&sh.full_c[sc]);
+                tc::mbar_arrive_expect_tx(bar, kTileC);
+                tc::tma_load_2d(sC + sc * kTileC, &code_map, ((x.vt0 + t) & 1) * 64 + static_cast<int>(rank) * 32,
+                                ((x.vt0 + t) >> 1) * a.nbg + s * kStageGroupsTc, bar);
+              }
+              __syncwarp();
+              if (++sc == kStagesC) {
+                sc = 0;
+                pc ^= 1u;
+              }
+            }
+            if (!alive) break;
+            if (st % Config<ONE>::kGatherTeams == team) {
+            if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) alive = false;
+            if (!alive) break;
+            const uint32_t at = static_cast<uint32_t>(s) * 256 + which * 128 + cl * 16;
+            const uint32_t bytes = at < row_bytes ? 16u : 0u;  // zero past the row's end
+            const uint8_t* src = a.luts + (bytes ? at : 0u);
+            uint32_t dst = sB + (st * 2 + which) * kTileB;
+#pragma unroll 4
+            for (int i = 0; i < groups4; i += 2, dst += 1024) {
+              tc::cp_async16_zfill(dst + dst_even, src + row[4 * i], bytes);
+              tc::cp_async16_zfill(dst + 512 + dst_odd, src + row[4 * i + 4], bytes);
+            }
+            tc::cp_async_arrive(tc::smem_u32(&sh.landed_b[st]));
+            }
+            if (++st == kStagesB) {
+              st = 0;
+              ph ^= 1u;
+            }
+          }
+        }
+        close_item();
+      }
+    } else if (warp == 16) {
       // ---- LUT tiles -------------------------------------------------------
       int st = 0;
       uint32_t ph = 0;
       for (int it = pair; it < items && alive; it += pairs) {
         const Item x = open_item(it);
         const int half_rows = x.cols / 2;
-        int4 rows = make_int4(0, 0, 0, 0);
-        const bool gathers = MODE == kBucket && lane * 4 < half_rows;
-        if (gathers) rows = *reinterpret_cast<const int4*>(&sh.par[pb].q[rank * kHalfN + lane * 4]);
         for (int t = 0; t < x.tiles && alive; ++t) {
           for (int s = 0; s < n_stages; ++s) {
             if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) {
@@ -370,18 +436,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
             const uint32_t bar = tc::smem_u32(&sh.full_b[st]);
             const uint32_t dst = sB + st * 2 * kTileB, cbar = tc::mapa(bar, 0);
-            if constexpr (MODE == kBucket) {
-              // The second half of the last stage may lie past the row.
-              const bool second = s * kStageGroupsTc + kHalfGroups < a.nbg;
-              if (rank == 0 && lane == 0) {
-                tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(x.cols) * (second ? 256u : 128u));
-              }
-              __syncwarp();
-              if (gathers) {
-                tc::tma_gather4_pair(dst + lane * 512, &lut_map, s * 256, rows, cbar);
-                if (second) tc::tma_gather4_pair(dst + kTileB + lane * 512, &lut_map, s * 256 + 128, rows, cbar);
-              }
-            } else if (tc::elect_one()) {
+            if (tc::elect_one()) {
               const int y = x.y + static_cast<int>(rank) * half_rows;
               if (rank == 0) tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(x.cols) * 256u);
               tc::tma_load_2d_pair(dst, &lut_map, s * 256, y, cbar);
@@ -482,14 +537,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         close_item();
       }
     } else if (MODE == kBucket && warp == 19) {
-      // ---- bucket items: the queries' constants, up to three items ahead -------
-      for (int it = pair; it < items && alive; it += pairs) {
-        if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_p[pb]), pp ^ 1u))) {
-          alive = false;
-          break;
-        }
+      // ---- bucket items: the queries' constants, up to three items ahead, and
+      // the relay of landed LUT stages: fenced to the async proxy here (a fence in
+      // the gathering warps waits for all their copies in flight), then passed to
+      // the issuing CTA.
+      int next = pair;  // the next item to prepare
+      auto prepare_item = [&]() {
         Params& p = sh.par[pb];
-        const uint4 e = a.items[it];  // bucket, first pair, pairs
+        const uint4 e = a.items[next];  // bucket, first pair, pairs
         const int count = static_cast<int>(e.z), cols = (count + 31) / 32 * 32;
         for (int c = lane; c < cols; c += kWarp) {
           const int at = c < cols / 2 ? c : kHalfN + c - cols / 2;
@@ -504,6 +559,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             thr = fmaxf(-FLT_MAX, a.floor[q]);
           }
           p.q[at] = q;
+          p.row[at] = static_cast<uint32_t>(q) * static_cast<uint32_t>(a.nbg) * 32u;
           p.scale[at] = scale;
           p.init[at] = init;
           p.off[at] = off;
@@ -517,16 +573,47 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(tc::smem_u32(&sh.full_p[pb]));
+        next += pairs;
         if (++pb == kParams) {
           pb = 0;
           pp ^= 1u;
         }
+      };
+      int rb = 0, st = 0;  // the relayed item's parameters, the next stage
+      uint32_t ph = 0;
+      for (int it = pair; it < items && alive; it += pairs) {
+        if (next == it) {
+          if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_p[pb]), pp ^ 1u))) {
+            alive = false;
+            break;
+          }
+          prepare_item();
+        }
+        const int stages = sh.par[rb].tiles * n_stages;
+        for (int s = 0; s < stages; ++s) {
+          if (next < items && next - it < kParams * pairs &&
+              __all_sync(full_mask(), tc::mbar_test(tc::smem_u32(&sh.empty_p[pb]), pp ^ 1u))) {
+            prepare_item();
+          }
+          if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.landed_b[st]), ph))) {
+            alive = false;
+            break;
+          }
+          tc::fence_async_shared();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive_release(tc::mapa(tc::smem_u32(&sh.full_b[st]), 0));
+          if (++st == kStagesB) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+        if (++rb == kParams) rb = 0;
       }
     }
     __syncwarp();
   } else {
     // ---- epilogue: warp quadrant = 32 vectors, half = N / 2 queries ------------
-    tc::reg_inc<kRegsEpilogue>();
+    tc::reg_inc<Config<ONE>::kRegsEpilogue>();
     const int quad = warp & 3, half = (warp - 8) >> 2;
     const long long list0 = (static_cast<long long>(blockIdx.x) * a.tile_queries + half * (a.tile_queries / 2)) * CAP;
     unsigned long long* lists = MODE == kTopK ? a.lists + list0 : nullptr;
@@ -559,130 +646,180 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         tc::named_sync(1 + half, 128);
       }
-      for (int t = 0; t < x.tiles; ++t) {
-        const long long v = (static_cast<long long>(x.vt0) + t * x.step) * kPairVectors + rank * 128 + 4 * lane + quad;
-        bool valid;
-        uint32_t id = static_cast<uint32_t>(v);
+      // A lane's vector of tile t: its alpha (NaN past the end: no score compares)
+      // and id, loaded one tile ahead.
+      auto slot_of = [&](int t) {
+        return (static_cast<long long>(x.vt0) + t * x.step) * kPairVectors + rank * 128 + 4 * lane + quad;
+      };
+      auto load_vector = [&](int t, float* al, uint32_t* id) {
+        const long long v = slot_of(t);
+        *al = NAN;
+        *id = static_cast<uint32_t>(v);
+        if (t >= x.tiles) return;
         if constexpr (MODE == kBucket) {
-          valid = v - static_cast<long long>(x.vt0) * kPairVectors < par.size;
-          if (valid) id = __ldg(a.slot_ids + v);
+          if (v - static_cast<long long>(x.vt0) * kPairVectors < par.size) {
+            *al = __ldg(a.alpha + v);
+            *id = __ldg(a.slot_ids + v);
+          }
         } else {
-          valid = v < a.n;
+          if (v < a.n) *al = __ldg(a.alpha + v);
         }
-        const float al = valid ? __ldg(a.alpha + v) : 0.f;
-        float fa[kHalfN];
+      };
+      float al, al_next;
+      uint32_t id, id_next;
+      load_vector(0, &al_next, &id_next);
+      for (int t = 0; t < x.tiles; ++t) {
+        al = al_next;
+        id = id_next;
+        load_vector(t + 1, &al_next, &id_next);
+        // fa of 32 queries (chunk c) -> scores: written out (sample), or one mask
+        // bit per score at or above its threshold, by straight-line code. Only
+        // when some lane has one do the scores go through shared memory
+        // (registers cannot be indexed) to the lists. NaN never compares >=.
+        auto take_scores = [&](int c, tc::F2 (&f)[16]) {
+          const tc::F2 al2{al, al};
+          if constexpr (SAMPLE) {
+            const long long at =
+                (static_cast<long long>(it % a.n_ranges) * a.range_tiles + t) * kPairVectors + rank * 128 + quad * 32 + lane;
+            const bool valid = slot_of(t) < a.n;
 #pragma unroll
-        for (int c = 0; c < kHalfN / 16; ++c) {
-          if (c * 16 < cols) {
+            for (int i = 0; i < 32; ++i) {
+              const float v = (i & 1) ? f[i / 2].y : f[i / 2].x;
+              if (c * 32 + i < cols && q0 + c * 32 + i < a.nq) {
+                a.dense[(q0 + c * 32 + i) * a.dense_stride + at] = valid ? __fadd_rn(__fmul_rn(v, al), 0.f) : -INFINITY;
+              }
+            }
+          } else {
+            unsigned part[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-              const float4 f = *reinterpret_cast<const float4*>(s_init + c * 16 + i);
-              fa[c * 16 + i] = f.x;
-              fa[c * 16 + i + 1] = f.y;
-              fa[c * 16 + i + 2] = f.z;
-              fa[c * 16 + i + 3] = f.w;
+            for (int i = 0; i < 32; i += 4) {
+              const float4 th = *reinterpret_cast<const float4*>(s_thr + c * 32 + i);
+              tc::F2 s0 = tc::mul2(f[i / 2], al2), s1 = tc::mul2(f[i / 2 + 1], al2);
+              if constexpr (MODE == kBucket) {
+                const float4 o = *reinterpret_cast<const float4*>(par.off + half * kHalfN + c * 32 + i);
+                // One by one: the packed add was fused with the packed multiply.
+                s0 = {__fadd_rn(s0.x, o.x), __fadd_rn(s0.y, o.y)};
+                s1 = {__fadd_rn(s1.x, o.z), __fadd_rn(s1.y, o.w)};
+              }
+              if (s0.x >= th.x) part[0] |= 1u << i;
+              if (s0.y >= th.y) part[1] |= 2u << i;
+              if (s1.x >= th.z) part[2] |= 4u << i;
+              if (s1.y >= th.w) part[3] |= 8u << i;
+              f[i / 2] = s0;
+              f[i / 2 + 1] = s1;
+            }
+            unsigned hits = part[0] | part[1] | part[2] | part[3];
+            if (cols - c * 32 < 32) hits &= 0xffffu;  // the last 16 queries
+            if (__any_sync(full_mask(), hits != 0u)) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                stage[2 * i * 32] = f[i].x;
+                stage[(2 * i + 1) * 32] = f[i].y;
+              }
+              while (hits) {
+                const int i = __ffs(hits) - 1;
+                hits &= hits - 1;
+                if constexpr (MODE == kBucket) {
+                  // Past the region's end nothing is written; the count says so.
+                  const int q = par.q[half * kHalfN + c * 32 + i];
+                  const uint32_t pos = atomicAdd(a.append_count + q, 1u);
+                  if (pos < a.region) {
+                    const long long at = static_cast<long long>(q) * a.region + pos;
+                    a.cand_score[at] = stage[i * 32];
+                    a.cand_id[at] = id;
+                  }
+                } else {
+                  const float score = __fadd_rn(stage[i * 32], 0.f);
+                  const int pos = atomicAdd(&s_cnt[c * 32 + i], 1);
+                  lists[static_cast<long long>(c * 32 + i) * CAP + pos] =
+                      (static_cast<unsigned long long>(order_key(score)) << 32) | static_cast<uint32_t>(~id);
+                }
+              }
+              __syncwarp();
             }
           }
-        }
-        for (int b = 0; b < n_batches; ++b, ++batch) {
+        };
+        // The batch sums are below 2^23: 2^23 + sum is exact in f32, and so is
+        // taking the 2^23 off again.
+        auto flush_sums = [&](int c, const uint32_t (&acc)[32], tc::F2 (&f)[16]) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            const float4 sc = *reinterpret_cast<const float4*>(s_scale + c * 32 + i);
+            const tc::F2 big{-8388608.f, -8388608.f};
+            const tc::F2 v0 = tc::add2({__uint_as_float(acc[i] | 0x4b000000u), __uint_as_float(acc[i + 1] | 0x4b000000u)}, big);
+            const tc::F2 v1 =
+                tc::add2({__uint_as_float(acc[i + 2] | 0x4b000000u), __uint_as_float(acc[i + 3] | 0x4b000000u)}, big);
+            f[i / 2] = tc::fma2({sc.x, sc.y}, v0, f[i / 2]);
+            f[i / 2 + 1] = tc::fma2({sc.z, sc.w}, v1, f[i / 2 + 1]);
+          }
+        };
+        auto load_init = [&](int c, tc::F2 (&f)[16]) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(s_init + c * 32 + i);
+            f[i / 2] = {v.x, v.y};
+            f[i / 2 + 1] = {v.z, v.w};
+          }
+        };
+        auto wait_acc = [&]() {
           const uint32_t buf = batch & 1u;
           if (alive) alive = __all_sync(full_mask(), tc::mbar_wait_long(tc::smem_u32(&sh.acc_full[buf]), (batch >> 1) & 1u));
           tc::fence_after();
+          return t_base + buf * acc_cols;
+        };
+        auto free_acc = [&]() {
+          tc::fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&sh.acc_empty[batch & 1u]), 0));
+          ++batch;
+        };
+        // TMEM columns past `cols` in a chunk belong to the other half or are unused.
+        if constexpr (ONE) {
+          // One batch: 32 queries at a time from sums to lists, the next 32 sums
+          // on their way.
+          const uint32_t acc_at = wait_acc();
+          uint32_t acc[2][32];
+          tc::tmem_ld32(acc_at, acc[0]);
 #pragma unroll
           for (int c = 0; c < kHalfN / 32; ++c) {
             if (c * 32 < cols) {
-              uint32_t acc[32];  // past `cols` the columns belong to the other half or are unused
-              tc::tmem_ld32(t_base + buf * acc_cols + c * 32, acc);
-              tc::tmem_wait_ld32(acc);
-#pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                const float4 f = *reinterpret_cast<const float4*>(s_scale + c * 32 + i);
-                const float sc[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                  // The batch sum is below 2^23: exact as 2^23 + sum.
-                  const float v = __fsub_rn(__uint_as_float(acc[i + u] | 0x4b000000u), 8388608.f);
-                  fa[c * 32 + i + u] = __fmaf_rn(sc[u], v, fa[c * 32 + i + u]);
-                }
+              tc::tmem_wait_ld32(acc[c & 1]);
+              if ((c + 1) * 32 < cols && c + 1 < kHalfN / 32) {
+                tc::tmem_ld32(acc_at + (c + 1) * 32, acc[(c + 1) & 1]);
+              } else {
+                free_acc();
               }
-            }
-          }
-          tc::fence_before();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive_cluster(tc::mapa(tc::smem_u32(&sh.acc_empty[buf]), 0));
-        }
-        if (SAMPLE) {
-          const long long at =
-              (static_cast<long long>(it % a.n_ranges) * a.range_tiles + t) * kPairVectors + rank * 128 + quad * 32 + lane;
-#pragma unroll
-          for (int c = 0; c < kHalfN / 16; ++c) {
-            if (c * 16 < cols) {
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                if (q0 + c * 16 + i < a.nq) {
-                  a.dense[(q0 + c * 16 + i) * a.dense_stride + at] =
-                      valid ? __fadd_rn(__fmul_rn(fa[c * 16 + i], al), 0.f) : -INFINITY;
-                }
-              }
+              tc::F2 f[16];
+              load_init(c, f);
+              flush_sums(c, acc[c & 1], f);
+              take_scores(c, f);
             }
           }
         } else {
-          // Per 32 queries: one mask bit per score at or above its threshold, by
-          // straight-line code. Only when some lane has one do the scores go
-          // through shared memory (registers cannot be indexed) to the lists.
-          // NaN and lanes past the end of the index never compare >=.
-          const float al_top = valid ? al : NAN;
+          tc::F2 fa[kHalfN / 32][16];
 #pragma unroll
           for (int c = 0; c < kHalfN / 32; ++c) {
-            if (c * 32 < cols) {
-              unsigned part[4] = {0u, 0u, 0u, 0u};
+            if (c * 32 < cols) load_init(c, fa[c]);
+          }
+          for (int b = 0; b < n_batches; ++b) {
+            const uint32_t acc_at = wait_acc();
 #pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                const float4 f = *reinterpret_cast<const float4*>(s_thr + c * 32 + i);
-                const float th[4] = {f.x, f.y, f.z, f.w};
-                [[maybe_unused]] float of[4];
-                if constexpr (MODE == kBucket) {
-                  const float4 o = *reinterpret_cast<const float4*>(par.off + half * kHalfN + c * 32 + i);
-                  of[0] = o.x;
-                  of[1] = o.y;
-                  of[2] = o.z;
-                  of[3] = o.w;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                  fa[c * 32 + i + u] = __fmul_rn(fa[c * 32 + i + u], al_top);
-                  if constexpr (MODE == kBucket) fa[c * 32 + i + u] = __fadd_rn(fa[c * 32 + i + u], of[u]);
-                  if (fa[c * 32 + i + u] >= th[u]) part[u] |= 1u << (i + u);
-                }
-              }
-              unsigned hits = part[0] | part[1] | part[2] | part[3];
-              if (cols - c * 32 < 32) hits &= 0xffffu;  // the last 16 queries
-              if (__any_sync(full_mask(), hits != 0u)) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) stage[i * 32] = fa[c * 32 + i];
-                while (hits) {
-                  const int i = __ffs(hits) - 1;
-                  hits &= hits - 1;
-                  if constexpr (MODE == kBucket) {
-                    // Past the region's end nothing is written; the count says so.
-                    const int q = par.q[half * kHalfN + c * 32 + i];
-                    const uint32_t pos = atomicAdd(a.append_count + q, 1u);
-                    if (pos < a.region) {
-                      const long long at = static_cast<long long>(q) * a.region + pos;
-                      a.cand_score[at] = stage[i * 32];
-                      a.cand_id[at] = id;
-                    }
-                  } else {
-                    const float score = __fadd_rn(stage[i * 32], 0.f);
-                    const int pos = atomicAdd(&s_cnt[c * 32 + i], 1);
-                    lists[static_cast<long long>(c * 32 + i) * CAP + pos] =
-                        (static_cast<unsigned long long>(order_key(score)) << 32) | static_cast<uint32_t>(~id);
-                  }
-                }
-                __syncwarp();
+            for (int c = 0; c < kHalfN / 32; ++c) {
+              if (c * 32 < cols) {
+                uint32_t acc[32];
+                tc::tmem_ld32(acc_at + c * 32, acc);
+                tc::tmem_wait_ld32(acc);
+                flush_sums(c, acc, fa[c]);
               }
             }
+            free_acc();
           }
+#pragma unroll
+          for (int c = 0; c < kHalfN / 32; ++c) {
+            if (c * 32 < cols) take_scores(c, fa[c]);
+          }
+        }
+        {
           if constexpr (MODE == kTopK) {
           // A tile adds at most 128 entries per list: cut the lists that might
           // overflow on the next one to their top k and raise the threshold.
@@ -780,24 +917,29 @@ cudaError_t make_map(CUtensorMapDataType type, const void* p, uint64_t cols, uin
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int MODE, int CAP>
-cudaError_t launch_t(const OneHotArgs& a, int ctas, cudaStream_t stream) {
-  auto kern = onehot_scan_kernel<MODE, CAP>;
+template <int MODE, int CAP, bool ONE>
+cudaError_t launch_one(const OneHotArgs& a, int ctas, cudaStream_t stream) {
+  auto kern = onehot_scan_kernel<MODE, CAP, ONE>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
   if (e != cudaSuccess) return e;
   CUtensorMap luts, codes;
   e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, a.luts, static_cast<uint64_t>(a.nbg) * 32, static_cast<uint64_t>(a.nq),
                static_cast<uint64_t>(a.nbg) * 32, 128,
-               MODE == kBucket ? 1u : static_cast<uint32_t>(a.tile_queries / 2),  // gathers take one-row boxes
+               static_cast<uint32_t>(a.tile_queries / 2),
                CU_TENSOR_MAP_SWIZZLE_128B, &luts);
   if (e != cudaSuccess) return e;
   const uint64_t rows = static_cast<uint64_t>((a.n + kTileVectors - 1) / kTileVectors) * static_cast<uint64_t>(a.nbg);
   e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT32, a.codes, kTileWords, rows, kTileWords * 4, 32, kChunkGroups,
                CU_TENSOR_MAP_SWIZZLE_NONE, &codes);
   if (e != cudaSuccess) return e;
-  kern<<<static_cast<unsigned>(ctas), kThreads, kSmemBytes, stream>>>(luts, codes, a);
+  kern<<<static_cast<unsigned>(ctas), Config<ONE>::kThreads, kSmemBytes, stream>>>(luts, codes, a);
   return cudaGetLastError();
+}
+
+template <int MODE, int CAP>
+cudaError_t launch_t(const OneHotArgs& a, int ctas, cudaStream_t stream) {
+  return a.nbg <= kFlushGroups ? launch_one<MODE, CAP, true>(a, ctas, stream) : launch_one<MODE, CAP, false>(a, ctas, stream);
 }
 
 // Ranges per query tile so that the items fill whole waves of CTA pairs: the
@@ -892,7 +1034,10 @@ cudaError_t launch_onehot_scan(const OneHotArgs& in, const OneHotPlan& p, cudaSt
 
 cudaError_t launch_onehot_buckets(const BucketScanArgs& b, long long nq, long long n_slots, int sms, unsigned* status,
                                   cudaStream_t stream) {
-  if (!b.append_count || !b.floor || b.n_items == nullptr || n_slots > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (!b.append_count || !b.floor || b.n_items == nullptr || n_slots > 0x7fffffffLL ||
+      nq * b.nbg * 32 > 0xffffffffLL) {
+    return cudaErrorInvalidValue;
+  }
   OneHotArgs a{};
   a.codes = b.codes;
   a.alpha = b.alpha;
