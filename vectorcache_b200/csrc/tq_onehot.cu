@@ -202,7 +202,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
                        const __grid_constant__ OneHotArgs a) {
   constexpr bool SAMPLE = MODE == kSample;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t{1023});
+  // An offset, not integer arithmetic on the pointer: the compiler has to see that
+  // everything below lies in shared memory.
+  unsigned char* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   unsigned char* codes_smem = base + static_cast<size_t>(kStagesB) * 2 * kTileB;
   Shared& sh = *reinterpret_cast<Shared*>(codes_smem + kStagesC * kTileC);
   const uint32_t sB = tc::smem_u32(base), sC = tc::smem_u32(codes_smem);
