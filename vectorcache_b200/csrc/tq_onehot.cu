@@ -81,7 +81,7 @@ constexpr int kParams = 3;
 struct Params {
   float scale[kMaxN], init[kMaxN], thr[kMaxN], off[kMaxN];
   int q[kMaxN];
-  uint32_t row[kMaxN];  // byte offset of the query's LUT row
+  uint32_t row[kMaxN + 32];  // byte offset of the query's LUT row (read in eights)
   int tiles, cols, size, vt0;
 };
 
@@ -408,10 +408,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             const uint32_t bytes = at < row_bytes ? 16u : 0u;  // zero past the row's end
             const uint8_t* src = a.luts + (bytes ? at : 0u);
             uint32_t dst = sB + (st * 2 + which) * kTileB;
-#pragma unroll 4
-            for (int i = 0; i < groups4; i += 2, dst += 1024) {
-              tc::cp_async16_zfill(dst + dst_even, src + row[4 * i], bytes);
-              tc::cp_async16_zfill(dst + 512 + dst_odd, src + row[4 * i + 4], bytes);
+            // Eight rows' offsets first: read one by one between the copies, their
+            // latency added up to 76 clocks a copy.
+            for (int i = 0; i < groups4; i += 8, dst += 4096) {
+              uint32_t off[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) off[u] = row[4 * (i + u)];
+#pragma unroll
+              for (int u = 0; u < 8; u += 2) {
+                if (i + u < groups4) {
+                  tc::cp_async16_zfill(dst + u * 512 + dst_even, src + off[u], bytes);
+                  tc::cp_async16_zfill(dst + u * 512 + 512 + dst_odd, src + off[u + 1], bytes);
+                }
+              }
             }
             tc::cp_async_arrive(tc::smem_u32(&sh.landed_b[st]));
             }
@@ -684,12 +693,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             const long long at =
                 (static_cast<long long>(it % a.n_ranges) * a.range_tiles + t) * kPairVectors + rank * 128 + quad * 32 + lane;
             const bool valid = slot_of(t) < a.n;
+            const int left = static_cast<int>(min(static_cast<long long>(cols), a.nq - q0)) - c * 32;
+            float* out = a.dense + (q0 + c * 32) * a.dense_stride + at;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const float v = (i & 1) ? f[i / 2].y : f[i / 2].x;
-              if (c * 32 + i < cols && q0 + c * 32 + i < a.nq) {
-                a.dense[(q0 + c * 32 + i) * a.dense_stride + at] = valid ? __fadd_rn(__fmul_rn(v, al), 0.f) : -INFINITY;
-              }
+              if (i < left) *out = valid ? __fadd_rn(__fmul_rn(v, al), 0.f) : -INFINITY;
+              out += a.dense_stride;
             }
           } else {
             unsigned part[4] = {0u, 0u, 0u, 0u};
@@ -699,7 +709,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
               tc::F2 s0 = tc::mul2(f[i / 2], al2), s1 = tc::mul2(f[i / 2 + 1], al2);
               if constexpr (MODE == kBucket) {
                 const float4 o = *reinterpret_cast<const float4*>(par.off + half * kHalfN + c * 32 + i);
-                // One by one: the packed add was fused with the packed multiply.
+                // One by one: ptxas 12.9 fused a packed add (.rn, -fmad=false) with the
+                // packed multiply before it, which rounds once instead of twice.
                 s0 = {__fadd_rn(s0.x, o.x), __fadd_rn(s0.y, o.y)};
                 s1 = {__fadd_rn(s1.x, o.z), __fadd_rn(s1.y, o.w)};
               }
