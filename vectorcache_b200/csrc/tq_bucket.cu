@@ -1777,7 +1777,9 @@ __global__ void __launch_bounds__(256) kth_floor_kernel(const float* __restrict_
   __shared__ uint32_t hist[256];
   __shared__ uint32_t s_digit, s_need, s_total;
   const long long q = blockIdx.x;
-  const long long n = count ? count[q] : stride;
+  // A count past the region (appends that found it full) means all of it: any
+  // subset's k-th best is a floor.
+  const long long n = count ? min(static_cast<long long>(count[q]), stride) : stride;
   const float* cs = cand + q * stride;
   uint32_t prefix = 0, mask = 0, need = static_cast<uint32_t>(k);
   for (int shift = 24; shift >= 0; shift -= 8) {

@@ -190,7 +190,7 @@ cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStre
 // appended to the query's region, without the lists of k; append_count may end
 // above the region's size, where the appends past its end are missing.
 constexpr int kOneHotItemQueries = 192;
-constexpr long long kOneHotPairsPerBucket = 48;
+constexpr long long kOneHotPairsPerBucket = 16;
 cudaError_t launch_onehot_buckets(const BucketScanArgs& a, long long nq, long long n_slots, int sms, unsigned* status,
                                   cudaStream_t stream);
 // Scans again, list by list, every query whose append_count passed its region:

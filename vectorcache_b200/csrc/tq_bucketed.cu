@@ -521,6 +521,26 @@ struct tq_bucketed {
       const int first =
           std::min(max_probe >= pa.wide_from ? vcb::kFloorProbesWide : vcb::kFloorProbes, max_probe);
       const bool two_phase = max_probe > vcb::kFloorProbes;
+      // Above a floor, steps with enough pairs per bucket go to the tensor cores.
+      bool any_onehot = false, onehot = false;
+      auto use_onehot = [&](long long step_pairs) {
+        onehot = ba.floor && step_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2;
+        pa.item_queries = onehot ? vcb::kOneHotItemQueries : vcb::kItemQueries;
+        pa.even_items = onehot;
+        any_onehot |= onehot;
+      };
+      auto scan = [&](const char* what, long long grid) {
+        if (!onehot) {
+          eng->launch(tq_index::kScan, s, what, [&] { return vcb::launch_bucket_scan(ba, grid, s); });
+          return;
+        }
+        eng->check_status = true;
+        eng->status_foreign |= s != eng->stream;
+        eng->launch(tq_index::kScan, s, what, [&] {
+          return vcb::launch_onehot_buckets(ba, static_cast<long long>(m), static_cast<long long>(n_slots), eng->sms,
+                                            eng->device_status(), s);
+        });
+      };
       if (two_phase) {
         // a query's candidate region: max_probe lists of kscan entries
         const long long region = static_cast<long long>(max_probe) * vcb::kBsListsPerProbe * kscan;
@@ -552,10 +572,11 @@ struct tq_bucketed {
           pa.first_split = st == 0 ? 0 : 1;
           const long long step_items =
               vcb::max_items(static_cast<long long>(m), steps[st + 1] - steps[st], nb);
+          use_onehot(static_cast<long long>(m) * (steps[st + 1] - steps[st]));
           eng->launch(tq_index::kPrep, s, "pair kernels (first probes)",
                       [&] { return vcb::launch_build_pairs(pa, s); });
-          eng->launch(tq_index::kScan, s, "bucket scan kernel (first probes)",
-                      [&] { return vcb::launch_bucket_scan(ba, std::min(items, step_items), s); });
+          scan(st == 0 ? "bucket scan kernel (probe 0)" : "bucket scan kernel (first probes)",
+               std::min(items, step_items));
           eng->launch(tq_index::kPrep, s, "floor kernel", [&] {
             return vcb::launch_kth_floor(ba.cand_score, region, ba.append_count, static_cast<long long>(m),
                                          static_cast<int>(kscan), sc.floor.as<float>(), s);
@@ -568,28 +589,13 @@ struct tq_bucketed {
       }
       const long long last_items =
           two_phase ? std::min(items, vcb::max_items(static_cast<long long>(m), max_probe - 1, nb)) : items;
-      // The far probes hold most pairs: with enough of them per bucket they go
-      // to the tensor cores, above the floors.
-      const long long far_pairs = static_cast<long long>(m) * (max_probe - first);
-      const bool onehot = two_phase && far_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2;
-      if (onehot) {
-        pa.item_queries = vcb::kOneHotItemQueries;
-        pa.even_items = true;
-      }
+      use_onehot(static_cast<long long>(m) * (max_probe - first));
       eng->launch(tq_index::kPrep, s, "pair kernels", [&] { return vcb::launch_build_pairs(pa, s); });
-      if (onehot) {
-        eng->check_status = true;
-        eng->status_foreign |= s != eng->stream;
-        eng->launch(tq_index::kScan, s, "bucket scan kernel", [&] {
-          return vcb::launch_onehot_buckets(ba, static_cast<long long>(m), static_cast<long long>(n_slots), eng->sms,
-                                            eng->device_status(), s);
-        });
+      scan("bucket scan kernel", last_items);
+      if (any_onehot) {
         eng->launch(tq_index::kScan, s, "bucket redo kernel", [&] {
           return vcb::launch_bucket_redo(ba, static_cast<long long>(m), pa.probes, ptop, np_pass, max_probe, s);
         });
-      } else {
-        eng->launch(tq_index::kScan, s, "bucket scan kernel",
-                    [&] { return vcb::launch_bucket_scan(ba, last_items, s); });
       }
       vcb::MergeArgs mg{};
       mg.cand_score = ba.cand_score;
