@@ -762,8 +762,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             const tc::F2 v0 = tc::add2({__uint_as_float(acc[i] | 0x4b000000u), __uint_as_float(acc[i + 1] | 0x4b000000u)}, big);
             const tc::F2 v1 =
                 tc::add2({__uint_as_float(acc[i + 2] | 0x4b000000u), __uint_as_float(acc[i + 3] | 0x4b000000u)}, big);
-            f[i / 2] = tc::fma2({sc.x, sc.y}, v0, f[i / 2]);
-            f[i / 2 + 1] = tc::fma2({sc.z, sc.w}, v1, f[i / 2 + 1]);
+            if constexpr (ONE) {  // the only batch: from the initial value
+              const float4 in = *reinterpret_cast<const float4*>(s_init + c * 32 + i);
+              f[i / 2] = tc::fma2({sc.x, sc.y}, v0, {in.x, in.y});
+              f[i / 2 + 1] = tc::fma2({sc.z, sc.w}, v1, {in.z, in.w});
+            } else {
+              f[i / 2] = tc::fma2({sc.x, sc.y}, v0, f[i / 2]);
+              f[i / 2 + 1] = tc::fma2({sc.z, sc.w}, v1, f[i / 2 + 1]);
+            }
           }
         };
         auto load_init = [&](int c, tc::F2 (&f)[16]) {
@@ -788,23 +794,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
         };
         // TMEM columns past `cols` in a chunk belong to the other half or are unused.
         if constexpr (ONE) {
-          // One batch: 32 queries at a time from sums to lists, the next 32 sums
-          // on their way.
+          // One batch: 32 queries at a time from sums to lists. (The next 32 sums
+          // loaded meanwhile: 224 bytes of spills per thread and tile, slower.)
           const uint32_t acc_at = wait_acc();
-          uint32_t acc[2][32];
-          tc::tmem_ld32(acc_at, acc[0]);
 #pragma unroll
           for (int c = 0; c < kHalfN / 32; ++c) {
             if (c * 32 < cols) {
-              tc::tmem_wait_ld32(acc[c & 1]);
-              if ((c + 1) * 32 < cols && c + 1 < kHalfN / 32) {
-                tc::tmem_ld32(acc_at + (c + 1) * 32, acc[(c + 1) & 1]);
-              } else {
-                free_acc();
-              }
+              uint32_t acc[32];
+              tc::tmem_ld32(acc_at + c * 32, acc);
+              tc::tmem_wait_ld32(acc);
+              if (c + 1 == kHalfN / 32 || (c + 1) * 32 >= cols) free_acc();
               tc::F2 f[16];
-              load_init(c, f);
-              flush_sums(c, acc[c & 1], f);
+              flush_sums(c, acc, f);
               take_scores(c, f);
             }
           }
