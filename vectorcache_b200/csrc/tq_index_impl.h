@@ -470,8 +470,10 @@ struct tq_index {
     // The sample's scores and the scan's running lists share one region.
     const size_t region = vcb::round_up(
         std::max(vcb::onehot_list_bytes(p), vcb::onehot_sample_bytes(p, static_cast<long long>(m))), 256);
-    sc.onehot->reserve(region + m * 4);
-    float* floor = reinterpret_cast<float*>(sc.onehot->as<unsigned char>() + region);
+    const size_t compact = p.compact ? m * nbg * 16 : 0;
+    sc.onehot->reserve(region + compact + m * 4);
+    uint8_t* compact_luts = sc.onehot->as<uint8_t>() + region;
+    float* floor = reinterpret_cast<float*>(compact_luts + compact);
     const float* qf = sc.qf->as<float>();
     vcb::OneHotArgs a{};
     a.codes = d_codes.as<uint32_t>();
@@ -488,6 +490,12 @@ struct tq_index {
     a.cand_id = sc.cand_i->as<uint32_t>();
     a.floor = floor;
     a.dense = sc.onehot->as<float>();
+    if (p.compact) {
+      launch(kPrep, s, "compact LUT kernel", [&] {
+        return vcb::launch_compact_luts(a.luts, static_cast<long long>(m), static_cast<int>(nbg), compact_luts, s);
+      });
+      a.luts = compact_luts;
+    }
     a.status = device_status();
     check_status = true;
     status_foreign |= s != stream;

@@ -206,11 +206,12 @@ struct OneHotPlan {
   int cap = 256;         // entries per running list
   int list_len = 0;      // entries per published list (>= k)
   int sample_tiles = 0, sample_step = 1;
+  bool compact = false;  // 3-bit codes: LUT rows of 16 bytes per byte group (launch_compact_luts)
 };
 struct OneHotArgs {
   const uint32_t* codes;
   const float* alpha;
-  const uint8_t* luts;
+  const uint8_t* luts;  // nq x nbg x 32 (compact plan: x 16)
   const float* lut_scale;
   const float* fa_init;
   long long n;
@@ -238,12 +239,15 @@ struct OneHotArgs {
   uint32_t region;      // entries a query's candidate region holds
   int max_probe;
   // set by the launchers
+  bool compact;
   int tile_queries, q_tiles, tiles, tile_step, range_tiles, n_ranges, list_len;
 };
 // False when the batch belongs to the lookup scan.
 bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, OneHotPlan* plan);
 size_t onehot_list_bytes(const OneHotPlan& p);
 size_t onehot_sample_bytes(const OneHotPlan& p, long long nq);
+// luts (nq x nbg x 32) -> out (nq x nbg x 16), the form a compact plan scans.
+cudaError_t launch_compact_luts(const uint8_t* luts, long long nq, int nbg, uint8_t* out, cudaStream_t stream);
 cudaError_t launch_onehot_sample(const OneHotArgs& a, const OneHotPlan& p, int sms, cudaStream_t stream);
 cudaError_t launch_onehot_scan(const OneHotArgs& a, const OneHotPlan& p, cudaStream_t stream);
 

@@ -42,8 +42,7 @@ namespace {
 // Byte groups per stage: 256 bytes of K. The issuing warp spends about 400 clocks
 // per stage on its waits and commits whatever the stage holds (measured), so a
 // stage has to be worth more than that: 8 MMAs are 768 clocks at N = 192.
-constexpr int kStageGroupsTc = 8;
-constexpr int kHalfGroups = 4;          // a producer set's share of a stage
+constexpr int kStageBytes = 256;
 constexpr int kMaxN = 192;              // queries per tile
 constexpr int kHalfN = kMaxN / 2;       // LUT rows per CTA; queries per epilogue warp
 constexpr int kTileB = kHalfN * 128;    // LUT bytes per CTA and half stage (128 bytes of K)
@@ -51,14 +50,23 @@ constexpr int kStagesB = 6;
 constexpr int kMaxStagesA = 4;
 constexpr int kHalfColsA = 32;          // TMEM columns of a half stage's one-hot rows
 constexpr int kStageColsA = 2 * kHalfColsA;
+// Byte groups of a stage. A byte group takes 32 bytes of K, or 16 with 3-bit
+// codes (N8): their nibbles are below 8, so half of a one-hot row and of the LUT
+// never meets a 1 and is left out (compact_luts_kernel).
+template <bool N8>
+struct Groups {
+  static constexpr int kBytes = N8 ? 16 : 32;
+  static constexpr int kStage = kStageBytes / kBytes;
+  static constexpr int kHalf = kStage / 2;  // a producer set's share
+  static constexpr int kBatchStages = kFlushGroups / kStage;
+  static constexpr int kChunkStages = 32 / kStage;
+};
 // Codes: 32 byte groups (32 words of 128 vectors each) per chunk.
-constexpr int kChunkStages = 4;
-constexpr int kChunkGroups = kChunkStages * kStageGroupsTc;
+constexpr int kChunkGroups = 32;
 constexpr int kTileC = kChunkGroups * 128;
 constexpr int kStagesC = 4;
 constexpr int kTmemCols = 512;
 constexpr int kPairVectors = 256;
-constexpr int kBatchStages = kFlushGroups / kStageGroupsTc;
 // Warps 0-7 build one-hot rows (two sets of four, a TMEM quadrant each), 8-15
 // are the epilogue, 16 loads LUT tiles, 17 issues MMAs, 18 loads codes (in bucket
 // mode 16, 18, 20 and 21 gather LUT rows and 19 prepares items). ONE: rows of a
@@ -172,6 +180,13 @@ __device__ __forceinline__ unsigned long long cut_any(unsigned long long* list, 
   return cut_list<16>(list, n, k, lane);
 }
 
+// The 8 one-hot bytes of a 3-bit code in bits 3..5 of x.
+__device__ __forceinline__ void onehot8(uint32_t x, uint32_t* out) {
+  uint64_t v;
+  asm("shl.b64 %0, %1, %2;" : "=l"(v) : "l"(uint64_t{1}), "r"(x & 0x38u));
+  out[0] = static_cast<uint32_t>(v);
+  out[1] = static_cast<uint32_t>(v >> 32);
+}
 // The 16 one-hot bytes of the nibble in bits 3..6 of x, as two 64-bit shifts of a
 // 1 by 8 * nibble and 8 * nibble - 64; a shift of 64 or more gives 0.
 __device__ __forceinline__ void onehot16(uint32_t x, uint32_t* out) {
@@ -196,11 +211,13 @@ struct Item {
 // kTopK: keep each query's top k of the item's range; CAP entries per list.
 // kBucket: items are (bucket, up to 192 of its probing queries); the LUT rows are
 // gathered by cp.async, and scores at or above the query's floor are appended to its region.
-template <int MODE, int CAP, bool ONE>
+template <int MODE, int CAP, bool ONE, bool N8>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThreads, 1)
     onehot_scan_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap code_map,
                        const __grid_constant__ OneHotArgs a) {
   constexpr bool SAMPLE = MODE == kSample;
+  constexpr int kStageGroupsTc = Groups<N8>::kStage, kHalfGroups = Groups<N8>::kHalf;
+  constexpr int kBatchStages = Groups<N8>::kBatchStages, kChunkStages = Groups<N8>::kChunkStages;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // An offset, not integer arithmetic on the pointer: the compiler has to see that
   // everything below lies in shared memory.
@@ -322,25 +339,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             for (int g = 0; g < kHalfGroups; ++g) {
               asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[g]) : "r"(src + g * 128));
             }
+            // Half of the set's groups: high nibble (first half of the LUT row),
+            // then the low one.
+            auto build = [&](int h, uint32_t* out) {
 #pragma unroll
-            for (int g = 0; g < 2; ++g) {
-              // high nibble (first half of the LUT row), then the low one
-              const uint32_t v = __funnelshift_r(w[g], w[g], rot);
-              onehot16(v >> 16, row[0] + 8 * g);
-              onehot16(v, row[0] + 8 * g + 4);
-            }
+              for (int g = 0; g < kHalfGroups / 2; ++g) {
+                const uint32_t word = w[h * (kHalfGroups / 2) + g];
+                const uint32_t v = __funnelshift_r(word, word, rot);
+                if constexpr (N8) {
+                  onehot8(v >> 16, out + 4 * g);
+                  onehot8(v, out + 4 * g + 2);
+                } else {
+                  onehot16(v >> 16, out + 8 * g);
+                  onehot16(v, out + 8 * g + 4);
+                }
+              }
+            };
+            build(0, row[0]);
             if (!__all_sync(full_mask(), ready || tc::mbar_wait(bar, ph ^ 1u))) {
               alive = false;
               break;
             }
             tc::fence_after();
             tc::tmem_st16(dst0 + slot * kStageColsA, row[0]);
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {
-              const uint32_t v = __funnelshift_r(w[2 + g], w[2 + g], rot);
-              onehot16(v >> 16, row[1] + 8 * g);
-              onehot16(v, row[1] + 8 * g + 4);
-            }
+            build(1, row[1]);
             tc::tmem_st16(dst0 + slot * kStageColsA + kHalfColsA / 2, row[1]);
             tc::tmem_wait_st();
             tc::fence_before();
@@ -377,7 +399,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
       const int team = warp >= 20;
       const uint32_t rl = lane >> 3, cl = lane & 7;
       const uint32_t dst_even = rl * 128 + ((cl ^ rl) << 4), dst_odd = rl * 128 + ((cl ^ (rl + 4)) << 4);
-      const uint32_t row_bytes = static_cast<uint32_t>(a.nbg) * 32;
+      const uint32_t row_bytes = static_cast<uint32_t>(a.nbg) * Groups<N8>::kBytes;
       int st = 0, sc = 0;
       uint32_t ph = 0, pc = 0;
       for (int it = pair; it < items && alive; it += pairs) {
@@ -520,12 +542,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
               const bool second = s * kStageGroupsTc + kHalfGroups < a.nbg;
               if (tc::elect_one()) {
 #pragma unroll
-                for (int j = 0; j < kHalfGroups; ++j) {
+                for (int j = 0; j < 4; ++j) {
                   tc::mma_i8_pair_ta(d, ta + 8u * j, db + 2u * j, idesc, (s > s0 || j > 0) ? 1u : 0u);
                 }
                 if (second) {
 #pragma unroll
-                  for (int j = 0; j < kHalfGroups; ++j) {
+                  for (int j = 0; j < 4; ++j) {
                     tc::mma_i8_pair_ta(d, ta + kHalfColsA + 8u * j, db2 + 2u * j, idesc, 1u);
                   }
                 }
@@ -570,7 +592,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             thr = fmaxf(-FLT_MAX, a.floor[q]);
           }
           p.q[at] = q;
-          p.row[at] = static_cast<uint32_t>(q) * static_cast<uint32_t>(a.nbg) * 32u;
+          p.row[at] = static_cast<uint32_t>(q) * static_cast<uint32_t>(a.nbg * Groups<N8>::kBytes);
           p.scale[at] = scale;
           p.init[at] = init;
           p.off[at] = off;
@@ -931,15 +953,24 @@ cudaError_t make_map(CUtensorMapDataType type, const void* p, uint64_t cols, uin
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int MODE, int CAP, bool ONE>
+// LUT rows of 3-bit codes without the entries no code selects: 16 bytes a byte
+// group, entries 0..7 of the high nibble, then of the low one.
+__global__ void compact_luts_kernel(const uint2* __restrict__ luts, long long groups, uint4* __restrict__ out) {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= groups) return;
+  const uint2 hi = luts[4 * i], lo = luts[4 * i + 2];
+  out[i] = make_uint4(hi.x, hi.y, lo.x, lo.y);
+}
+
+template <int MODE, int CAP, bool ONE, bool N8>
 cudaError_t launch_one(const OneHotArgs& a, int ctas, cudaStream_t stream) {
-  auto kern = onehot_scan_kernel<MODE, CAP, ONE>;
+  auto kern = onehot_scan_kernel<MODE, CAP, ONE, N8>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
   if (e != cudaSuccess) return e;
   CUtensorMap luts, codes;
-  e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, a.luts, static_cast<uint64_t>(a.nbg) * 32, static_cast<uint64_t>(a.nq),
-               static_cast<uint64_t>(a.nbg) * 32, 128,
+  const uint64_t row_bytes = static_cast<uint64_t>(a.nbg) * Groups<N8>::kBytes;
+  e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, a.luts, row_bytes, static_cast<uint64_t>(a.nq), row_bytes, 128,
                static_cast<uint32_t>(a.tile_queries / 2),
                CU_TENSOR_MAP_SWIZZLE_128B, &luts);
   if (e != cudaSuccess) return e;
@@ -953,7 +984,13 @@ cudaError_t launch_one(const OneHotArgs& a, int ctas, cudaStream_t stream) {
 
 template <int MODE, int CAP>
 cudaError_t launch_t(const OneHotArgs& a, int ctas, cudaStream_t stream) {
-  return a.nbg <= kFlushGroups ? launch_one<MODE, CAP, true>(a, ctas, stream) : launch_one<MODE, CAP, false>(a, ctas, stream);
+  const bool one = a.nbg <= kFlushGroups;
+  if constexpr (MODE != kBucket) {
+    if (a.compact) {
+      return one ? launch_one<MODE, CAP, true, true>(a, ctas, stream) : launch_one<MODE, CAP, false, true>(a, ctas, stream);
+    }
+  }
+  return one ? launch_one<MODE, CAP, true, false>(a, ctas, stream) : launch_one<MODE, CAP, false, false>(a, ctas, stream);
 }
 
 // Ranges per query tile so that the items fill whole waves of CTA pairs: the
@@ -1003,7 +1040,9 @@ bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, O
   // at most 1/16 of it, 32768 vectors and 128 MiB of scores. (1000 queries x
   // 100k x 128, k = 10: scan + sample + selection 261 + 23 + 13 us with 1536
   // vectors, 188 + 35 + 25 us with the rule's 6144.)
-  const long long n_stages = (nbg + kStageGroupsTc - 1) / kStageGroupsTc;
+  const int stage = bits == 3 ? Groups<true>::kStage : Groups<false>::kStage;
+  const long long n_stages = (nbg + stage - 1) / stage;
+  plan->compact = bits == 3;
   long long sample = std::max<long long>(n / 64, 8192LL * k / n_stages);
   sample = std::min<long long>({sample, n / 16, 32768, (128LL << 20) / 4 / nq});
   sample = std::max<long long>(sample, 1024);
@@ -1020,8 +1059,16 @@ size_t onehot_sample_bytes(const OneHotPlan& p, long long nq) {
   return static_cast<size_t>(nq) * p.sample_tiles * kPairVectors * 4;
 }
 
+cudaError_t launch_compact_luts(const uint8_t* luts, long long nq, int nbg, uint8_t* out, cudaStream_t stream) {
+  const long long groups = nq * nbg;
+  compact_luts_kernel<<<static_cast<unsigned>((groups + 255) / 256), 256, 0, stream>>>(
+      reinterpret_cast<const uint2*>(luts), groups, reinterpret_cast<uint4*>(out));
+  return cudaGetLastError();
+}
+
 cudaError_t launch_onehot_sample(const OneHotArgs& in, const OneHotPlan& p, int sms, cudaStream_t stream) {
   OneHotArgs a = in;
+  a.compact = p.compact;
   a.tile_queries = p.tile_queries;
   a.q_tiles = p.q_tiles;
   a.tiles = p.sample_tiles;
@@ -1036,6 +1083,7 @@ cudaError_t launch_onehot_sample(const OneHotArgs& in, const OneHotPlan& p, int 
 
 cudaError_t launch_onehot_scan(const OneHotArgs& in, const OneHotPlan& p, cudaStream_t stream) {
   OneHotArgs a = in;
+  a.compact = p.compact;
   a.tile_queries = p.tile_queries;
   a.q_tiles = p.q_tiles;
   a.tiles = p.tiles;
