@@ -39,28 +39,12 @@
 namespace vcb {
 namespace {
 
-// Byte groups per stage: 256 bytes of K. The issuing warp spends about 400 clocks
-// per stage on its waits and commits whatever the stage holds (measured), so a
-// stage has to be worth more than that: 8 MMAs are 768 clocks at N = 192.
-constexpr int kStageBytes = 256;
 constexpr int kMaxN = 192;              // queries per tile
 constexpr int kHalfN = kMaxN / 2;       // LUT rows per CTA; queries per epilogue warp
-constexpr int kTileB = kHalfN * 128;    // LUT bytes per CTA and half stage (128 bytes of K)
+constexpr int kTileB = kHalfN * 128;    // LUT bytes per CTA and 128 bytes of K
 constexpr int kStagesB = 6;
 constexpr int kMaxStagesA = 4;
-constexpr int kHalfColsA = 32;          // TMEM columns of a half stage's one-hot rows
-constexpr int kStageColsA = 2 * kHalfColsA;
-// Byte groups of a stage. A byte group takes 32 bytes of K, or 16 with 3-bit
-// codes (N8): their nibbles are below 8, so half of a one-hot row and of the LUT
-// never meets a 1 and is left out (compact_luts_kernel).
-template <bool N8>
-struct Groups {
-  static constexpr int kBytes = N8 ? 16 : 32;
-  static constexpr int kStage = kStageBytes / kBytes;
-  static constexpr int kHalf = kStage / 2;  // a producer set's share
-  static constexpr int kBatchStages = kFlushGroups / kStage;
-  static constexpr int kChunkStages = 32 / kStage;
-};
+constexpr int kPieceCols = 16;          // TMEM columns a producer stores at a time
 // Codes: 32 byte groups (32 words of 128 vectors each) per chunk.
 constexpr int kChunkGroups = 32;
 constexpr int kTileC = kChunkGroups * 128;
@@ -69,17 +53,47 @@ constexpr int kTmemCols = 512;
 constexpr int kPairVectors = 256;
 // Warps 0-7 build one-hot rows (two sets of four, a TMEM quadrant each), 8-15
 // are the epilogue, 16 loads LUT tiles, 17 issues MMAs, 18 loads codes (in bucket
-// mode 16, 18, 20 and 21 gather LUT rows and 19 prepares items). ONE: rows of a
-// single 256-group batch, whose sums need no registers between batches: fewer
-// registers per epilogue warp, and four more warps.
-template <bool ONE>
+// mode 16, 18, 20 and 21 gather LUT rows and 19 prepares items).
+//   kOne: rows of a single 256-group batch, whose sums need no registers between
+//     batches: fewer registers per epilogue warp, and four more warps.
+//   kSmall: at most 64 queries. The MMAs take a third of the time then and the
+//     hand-over of the stages bounds the kernel: 430 of 580 clocks per 256 bytes
+//     of K are left with a quarter of the MMAs and no one-hot stores. So stages
+//     hold 512 bytes of K, and the one-hot and LUT stages share one ring: one wait
+//     and one commit instead of two. (Twice the producer warps instead: 1M x 1536,
+//     16 queries 1625 -> 1792 us.)
+// A stage holds 256 bytes of K otherwise: the issuing warp spends about 400 clocks
+// per stage on its waits and commits whatever it holds, so it has to be worth more
+// than that (8 MMAs are 768 clocks at N = 192).
+enum Variant { kMulti, kOne, kSmall };
+template <int V>
 struct Config {
-  static constexpr int kThreads = ONE ? 768 : 640;
-  static constexpr int kRegsLaunch = ONE ? 80 : 96;
-  static constexpr int kRegsProducer = 64, kRegsEpilogue = ONE ? 128 : 152, kRegsIssue = ONE ? 48 : 40;
+  static constexpr int kThreads = V == kOne ? 768 : 640;
+  static constexpr int kRegsLaunch = V == kOne ? 80 : 96;
+  static constexpr int kRegsProducer = 64, kRegsEpilogue = V == kOne ? 128 : 152;
+  static constexpr int kRegsIssue = V == kOne ? 48 : 40;
   static_assert(256 * (kRegsProducer + kRegsEpilogue) + (kThreads - 512) * kRegsIssue <= kThreads * kRegsLaunch,
                 "the register split must fit what the block is launched with");
-  static constexpr int kGatherTeams = ONE ? 2 : 1;  // pairs of warps that gather LUT rows
+  static constexpr int kGatherTeams = V == kOne ? 2 : 1;    // pairs of warps that gather LUT rows
+  static constexpr int kCols = V == kSmall ? 64 : kMaxN;    // accumulator columns (queries)
+  static constexpr int kStageBytes = V == kSmall ? 512 : 256;
+  static constexpr int kTiles = kStageBytes / 128;          // LUT tiles of a stage
+  static constexpr int kTileBytes = V == kSmall ? 32 * 128 : kTileB;
+  static constexpr int kRingB = V == kSmall ? 3 : kStagesB; // kSmall: the one-hot ring as well
+  static constexpr int kStageCols = kStageBytes / 4;        // TMEM columns of a stage's one-hot rows
+};
+// Byte groups of a stage. A byte group takes 32 bytes of K, or 16 with 3-bit
+// codes (N8): their nibbles are below 8, so half of a one-hot row and of the LUT
+// never meets a 1 and is left out (compact_luts_kernel).
+template <bool N8, int V>
+struct Groups {
+  static constexpr int kBytes = N8 ? 16 : 32;
+  static constexpr int kStage = Config<V>::kStageBytes / kBytes;
+  static constexpr int kHalf = kStage / 2;        // a producer set's share
+  static constexpr int kTile = 128 / kBytes;      // per LUT tile
+  static constexpr int kPiece = 4 * kPieceCols / kBytes;
+  static constexpr int kBatchStages = kFlushGroups / kStage;
+  static constexpr int kChunkStages = kChunkGroups / kStage;
 };
 
 enum Mode { kSample, kTopK, kBucket };
@@ -211,13 +225,17 @@ struct Item {
 // kTopK: keep each query's top k of the item's range; CAP entries per list.
 // kBucket: items are (bucket, up to 192 of its probing queries); the LUT rows are
 // gathered by cp.async, and scores at or above the query's floor are appended to its region.
-template <int MODE, int CAP, bool ONE, bool N8>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThreads, 1)
+template <int MODE, int CAP, int V, bool N8>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<V>::kThreads, 1)
     onehot_scan_kernel(const __grid_constant__ CUtensorMap lut_map, const __grid_constant__ CUtensorMap code_map,
                        const __grid_constant__ OneHotArgs a) {
-  constexpr bool SAMPLE = MODE == kSample;
-  constexpr int kStageGroupsTc = Groups<N8>::kStage, kHalfGroups = Groups<N8>::kHalf;
-  constexpr int kBatchStages = Groups<N8>::kBatchStages, kChunkStages = Groups<N8>::kChunkStages;
+  constexpr bool SAMPLE = MODE == kSample, ONE = V == kOne;
+  constexpr int kChunks = Config<V>::kCols / 2 / 32;  // of 32 queries per epilogue warp
+  using G = Groups<N8, V>;
+  constexpr int kStageGroupsTc = G::kStage, kHalfGroups = G::kHalf;
+  constexpr int kBatchStages = G::kBatchStages, kChunkStages = G::kChunkStages;
+  constexpr int kTiles = Config<V>::kTiles, kTileBytes = Config<V>::kTileBytes, kRingB = Config<V>::kRingB;
+  constexpr int kStageColsA = Config<V>::kStageCols, kHalfColsA = kStageColsA / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // An offset, not integer arithmetic on the pointer: the compiler has to see that
   // everything below lies in shared memory.
@@ -232,8 +250,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
   const int n_batches = (a.nbg + kFlushGroups - 1) / kFlushGroups;
   const int items = MODE == kBucket ? static_cast<int>(*a.n_items) : a.q_tiles * a.n_ranges;
   // TMEM: two accumulators of acc_cols columns, then the one-hot stages.
-  const uint32_t acc_cols = MODE != kBucket && a.tile_queries <= 128 ? 128 : kMaxN;
-  const int stages_a = acc_cols == 128 ? kMaxStagesA : 2;
+  const uint32_t acc_cols = V == kSmall ? 64 : (MODE != kBucket && a.tile_queries <= 128 ? 128 : kMaxN);
+  const int stages_a = V == kSmall ? kRingB : (acc_cols == 128 ? 4 : 2);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStagesB; ++s) {
@@ -242,7 +260,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
       tc::mbar_init(tc::smem_u32(&sh.empty_b[s]), 1);
     }
     for (int s = 0; s < kMaxStagesA; ++s) {
-      tc::mbar_init(tc::smem_u32(&sh.full_a[s]), 16);  // eight producer warps of each CTA
+      // eight producer warps of each CTA (and, sharing the ring, the LUT bytes)
+      tc::mbar_init(tc::smem_u32(&sh.full_a[s]), V == kSmall ? 17 : 16);
       tc::mbar_init(tc::smem_u32(&sh.empty_a[s]), 1);
     }
     for (int s = 0; s < kStagesC; ++s) {
@@ -256,7 +275,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
     for (int b = 0; b < kParams; ++b) {
       tc::mbar_init(tc::smem_u32(&sh.full_p[b]), 1);
       // eight producer, eight epilogue and the gathering warps, and the issuing one
-      tc::mbar_init(tc::smem_u32(&sh.empty_p[b]), 16 + 2 * Config<ONE>::kGatherTeams + (rank == 0 ? 1 : 0));
+      tc::mbar_init(tc::smem_u32(&sh.empty_p[b]), 16 + 2 * Config<V>::kGatherTeams + (rank == 0 ? 1 : 0));
     }
     tc::mbar_init_fence();
     tc::prefetch_map(&lut_map);
@@ -272,6 +291,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
   tc::fence_after();
   const uint32_t tmem = sh.tmem;
   bool alive = true;  // false: a wait gave up; this role stops
+  uint64_t* const full_b = V == kSmall ? sh.full_a : sh.full_b;
+  uint64_t* const empty_b = V == kSmall ? sh.empty_a : sh.empty_b;
 
   // Every role walks the same items: number pair, pair + pairs, ... In bucket mode
   // their parameters come through shared memory (warp 19 fills them in).
@@ -312,7 +333,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
   if (warp < 8) {
     // ---- one-hot rows: set `set` builds its half of every stage; TMEM lane
     // 32 quad + lane holds vector 4 lane + quad of this CTA's 128.
-    tc::reg_dec<Config<ONE>::kRegsProducer>();
+    tc::reg_dec<Config<V>::kRegsProducer>();
     const int quad = warp & 3, set = warp >> 2;
     const uint32_t dst0 = tmem + 2 * acc_cols + set * kHalfColsA + (static_cast<uint32_t>(quad * 32) << 16);
     const uint32_t src0 = sC + set * kHalfGroups * 128 + lane * 4;
@@ -334,17 +355,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             // half's columns are stored while the second half is built.
             const uint32_t bar = tc::smem_u32(&sh.empty_a[slot]);
             const bool ready = tc::mbar_test(bar, ph ^ 1u);
-            uint32_t w[kHalfGroups], row[2][kHalfColsA / 2];
+            uint32_t w[kHalfGroups];
 #pragma unroll
             for (int g = 0; g < kHalfGroups; ++g) {
               asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[g]) : "r"(src + g * 128));
             }
-            // Half of the set's groups: high nibble (first half of the LUT row),
-            // then the low one.
-            auto build = [&](int h, uint32_t* out) {
+            // The set's rows in pieces of 16 columns: high nibble (first half of
+            // the LUT row), then the low one.
+            auto build = [&](int piece, uint32_t (&out)[kPieceCols]) {
 #pragma unroll
-              for (int g = 0; g < kHalfGroups / 2; ++g) {
-                const uint32_t word = w[h * (kHalfGroups / 2) + g];
+              for (int g = 0; g < G::kPiece; ++g) {
+                const uint32_t word = w[piece * G::kPiece + g];
                 const uint32_t v = __funnelshift_r(word, word, rot);
                 if constexpr (N8) {
                   onehot8(v >> 16, out + 4 * g);
@@ -355,15 +376,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
                 }
               }
             };
+            uint32_t row[2][kPieceCols];
             build(0, row[0]);
             if (!__all_sync(full_mask(), ready || tc::mbar_wait(bar, ph ^ 1u))) {
               alive = false;
               break;
             }
             tc::fence_after();
-            tc::tmem_st16(dst0 + slot * kStageColsA, row[0]);
-            build(1, row[1]);
-            tc::tmem_st16(dst0 + slot * kStageColsA + kHalfColsA / 2, row[1]);
+#pragma unroll
+            for (int piece = 0; piece < kHalfColsA / kPieceCols; ++piece) {
+              if (piece > 0) build(piece, row[piece & 1]);
+              tc::tmem_st16(dst0 + slot * kStageColsA + piece * kPieceCols, row[piece & 1]);
+            }
             tc::tmem_wait_st();
             tc::fence_before();
             __syncwarp();
@@ -385,7 +409,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
     }
     __syncwarp();
   } else if (warp >= 16) {
-    tc::reg_dec<Config<ONE>::kRegsIssue>();
+    tc::reg_dec<Config<V>::kRegsIssue>();
     if (MODE == kBucket && (warp == 16 || warp == 18 || (ONE && (warp == 20 || warp == 21)))) {
       // ---- LUT rows of the item's queries: warp 16 copies the first 128 bytes
       // of K of every stage, warp 18 the second, 16 bytes a lane, eight lanes a
@@ -399,7 +423,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
       const int team = warp >= 20;
       const uint32_t rl = lane >> 3, cl = lane & 7;
       const uint32_t dst_even = rl * 128 + ((cl ^ rl) << 4), dst_odd = rl * 128 + ((cl ^ (rl + 4)) << 4);
-      const uint32_t row_bytes = static_cast<uint32_t>(a.nbg) * Groups<N8>::kBytes;
+      const uint32_t row_bytes = static_cast<uint32_t>(a.nbg) * Groups<N8, V>::kBytes;
       int st = 0, sc = 0;
       uint32_t ph = 0, pc = 0;
       for (int it = pair; it < items && alive; it += pairs) {
@@ -423,13 +447,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
               }
             }
             if (!alive) break;
-            if (st % Config<ONE>::kGatherTeams == team) {
+            if (st % Config<V>::kGatherTeams == team) {
             if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) alive = false;
             if (!alive) break;
             const uint32_t at = static_cast<uint32_t>(s) * 256 + which * 128 + cl * 16;
             const uint32_t bytes = at < row_bytes ? 16u : 0u;  // zero past the row's end
             const uint8_t* src = a.luts + (bytes ? at : 0u);
-            uint32_t dst = sB + (st * 2 + which) * kTileB;
+            uint32_t dst = sB + (st * kTiles + which) * kTileBytes;
             // Eight rows' offsets first: read one by one between the copies, their
             // latency added up to 76 clocks a copy.
             for (int i = 0; i < groups4; i += 8, dst += 4096) {
@@ -463,20 +487,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
         const int half_rows = x.cols / 2;
         for (int t = 0; t < x.tiles && alive; ++t) {
           for (int s = 0; s < n_stages; ++s) {
-            if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) {
+            if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&empty_b[st]), ph ^ 1u))) {
               alive = false;
               break;
             }
-            const uint32_t bar = tc::smem_u32(&sh.full_b[st]);
-            const uint32_t dst = sB + st * 2 * kTileB, cbar = tc::mapa(bar, 0);
+            const uint32_t bar = tc::smem_u32(&full_b[st]);
+            const uint32_t dst = sB + st * kTiles * kTileBytes, cbar = tc::mapa(bar, 0);
             if (tc::elect_one()) {
               const int y = x.y + static_cast<int>(rank) * half_rows;
-              if (rank == 0) tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(x.cols) * 256u);
-              tc::tma_load_2d_pair(dst, &lut_map, s * 256, y, cbar);
-              tc::tma_load_2d_pair(dst + kTileB, &lut_map, s * 256 + 128, y, cbar);
+              if (rank == 0) tc::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(x.cols) * Config<V>::kStageBytes);
+#pragma unroll
+              for (int j = 0; j < kTiles; ++j) {  // tiles past the row are zero
+                tc::tma_load_2d_pair(dst + j * kTileBytes, &lut_map, (s * kTiles + j) * 128, y, cbar);
+              }
             }
             __syncwarp();
-            if (++st == kStagesB) {
+            if (++st == kRingB) {
               st = 0;
               ph ^= 1u;
             }
@@ -517,6 +543,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
       // ---- MMA ---------------------------------------------------------------
       int sa = 0, sb = 0;
       uint32_t pa = 0, pb = 0, batch = 0;
+      bool seen = false;
       for (int it = pair; it < items && alive; it += pairs) {
         const Item x = open_item(it);
         const uint32_t idesc = (2u << 4) | (static_cast<uint32_t>(x.cols >> 3) << 17) | (16u << 24);
@@ -530,40 +557,41 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             }
             const int s1 = min(s0 + kBatchStages, n_stages);
             for (int s = s0; s < s1; ++s) {
-              if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.full_b[sb]), pb) &&
-                                               tc::mbar_wait(tc::smem_u32(&sh.full_a[sa]), pa))) {
+              // `seen`: the stage was found ready while the one before was issued.
+              if (!seen && !__all_sync(full_mask(), (V == kSmall || tc::mbar_wait(tc::smem_u32(&full_b[sb]), pb)) &&
+                                                        tc::mbar_wait(tc::smem_u32(&sh.full_a[sa]), pa))) {
                 alive = false;
                 break;
               }
               tc::fence_after();
               const uint32_t ta = tmem + 2 * acc_cols + sa * kStageColsA;
-              const uint64_t db = tc::desc_k128(sB + sb * 2 * kTileB);
-              const uint64_t db2 = tc::desc_k128(sB + (sb * 2 + 1) * kTileB);
-              const bool second = s * kStageGroupsTc + kHalfGroups < a.nbg;
+              const uint64_t db = tc::desc_k128(sB + sb * kTiles * kTileBytes);
+              const int groups_left = a.nbg - s * kStageGroupsTc;  // tiles past the row are skipped
+              const int na = sa + 1 == stages_a ? 0 : sa + 1, nb = sb + 1 == kRingB ? 0 : sb + 1;
+              const uint32_t npa = pa ^ (na == 0 ? 1u : 0u), npb = pb ^ (nb == 0 ? 1u : 0u);
+              // kSmall: look at the next stage while this one is issued (with longer
+              // MMAs the look only costs: 1000 x 100k x 128 150 -> 160 us).
+              const bool peek = V == kSmall && tc::mbar_test(tc::smem_u32(&sh.full_a[na]), npa);
               if (tc::elect_one()) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  tc::mma_i8_pair_ta(d, ta + 8u * j, db + 2u * j, idesc, (s > s0 || j > 0) ? 1u : 0u);
-                }
-                if (second) {
+                for (int i = 0; i < kTiles; ++i) {
+                  if (i > 0 && groups_left <= i * G::kTile) break;
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
-                    tc::mma_i8_pair_ta(d, ta + kHalfColsA + 8u * j, db2 + 2u * j, idesc, 1u);
+                    tc::mma_i8_pair_ta(d, ta + 32u * i + 8u * j, db + (kTileBytes >> 4) * i + 2u * j, idesc,
+                                       (i > 0 || j > 0) ? 1u : (s > s0 ? 1u : 0u));
                   }
                 }
                 tc::commit2(tc::smem_u32(&sh.empty_a[sa]));
-                tc::commit2(tc::smem_u32(&sh.empty_b[sb]));
+                if (V != kSmall) tc::commit2(tc::smem_u32(&sh.empty_b[sb]));
                 if (s + 1 == s1) tc::commit2(tc::smem_u32(&sh.acc_full[buf]));
               }
               __syncwarp();
-              if (++sa == stages_a) {
-                sa = 0;
-                pa ^= 1u;
-              }
-              if (++sb == kStagesB) {
-                sb = 0;
-                pb ^= 1u;
-              }
+              if (V == kSmall) seen = __all_sync(full_mask(), peek);
+              sa = na;
+              sb = nb;
+              pa = npa;
+              pb = npb;
             }
           }
         }
@@ -592,7 +620,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             thr = fmaxf(-FLT_MAX, a.floor[q]);
           }
           p.q[at] = q;
-          p.row[at] = static_cast<uint32_t>(q) * static_cast<uint32_t>(a.nbg * Groups<N8>::kBytes);
+          p.row[at] = static_cast<uint32_t>(q) * static_cast<uint32_t>(a.nbg * Groups<N8, V>::kBytes);
           p.scale[at] = scale;
           p.init[at] = init;
           p.off[at] = off;
@@ -646,7 +674,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
     __syncwarp();
   } else {
     // ---- epilogue: warp quadrant = 32 vectors, half = N / 2 queries ------------
-    tc::reg_inc<Config<ONE>::kRegsEpilogue>();
+    tc::reg_inc<Config<V>::kRegsEpilogue>();
     const int quad = warp & 3, half = (warp - 8) >> 2;
     const long long list0 = (static_cast<long long>(blockIdx.x) * a.tile_queries + half * (a.tile_queries / 2)) * CAP;
     unsigned long long* lists = MODE == kTopK ? a.lists + list0 : nullptr;
@@ -820,27 +848,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
           // loaded meanwhile: 224 bytes of spills per thread and tile, slower.)
           const uint32_t acc_at = wait_acc();
 #pragma unroll
-          for (int c = 0; c < kHalfN / 32; ++c) {
+          for (int c = 0; c < kChunks; ++c) {
             if (c * 32 < cols) {
               uint32_t acc[32];
               tc::tmem_ld32(acc_at + c * 32, acc);
               tc::tmem_wait_ld32(acc);
-              if (c + 1 == kHalfN / 32 || (c + 1) * 32 >= cols) free_acc();
+              if (c + 1 == kChunks || (c + 1) * 32 >= cols) free_acc();
               tc::F2 f[16];
               flush_sums(c, acc, f);
               take_scores(c, f);
             }
           }
         } else {
-          tc::F2 fa[kHalfN / 32][16];
+          tc::F2 fa[kChunks][16];
 #pragma unroll
-          for (int c = 0; c < kHalfN / 32; ++c) {
+          for (int c = 0; c < kChunks; ++c) {
             if (c * 32 < cols) load_init(c, fa[c]);
           }
           for (int b = 0; b < n_batches; ++b) {
             const uint32_t acc_at = wait_acc();
 #pragma unroll
-            for (int c = 0; c < kHalfN / 32; ++c) {
+            for (int c = 0; c < kChunks; ++c) {
               if (c * 32 < cols) {
                 uint32_t acc[32];
                 tc::tmem_ld32(acc_at + c * 32, acc);
@@ -851,7 +879,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<ONE>::kThread
             free_acc();
           }
 #pragma unroll
-          for (int c = 0; c < kHalfN / 32; ++c) {
+          for (int c = 0; c < kChunks; ++c) {
             if (c * 32 < cols) take_scores(c, fa[c]);
           }
         }
@@ -962,14 +990,14 @@ __global__ void compact_luts_kernel(const uint2* __restrict__ luts, long long gr
   out[i] = make_uint4(hi.x, hi.y, lo.x, lo.y);
 }
 
-template <int MODE, int CAP, bool ONE, bool N8>
+template <int MODE, int CAP, int V, bool N8>
 cudaError_t launch_one(const OneHotArgs& a, int ctas, cudaStream_t stream) {
-  auto kern = onehot_scan_kernel<MODE, CAP, ONE, N8>;
+  auto kern = onehot_scan_kernel<MODE, CAP, V, N8>;
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
   if (e != cudaSuccess) return e;
   CUtensorMap luts, codes;
-  const uint64_t row_bytes = static_cast<uint64_t>(a.nbg) * Groups<N8>::kBytes;
+  const uint64_t row_bytes = static_cast<uint64_t>(a.nbg) * Groups<N8, V>::kBytes;
   e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, a.luts, row_bytes, static_cast<uint64_t>(a.nq), row_bytes, 128,
                static_cast<uint32_t>(a.tile_queries / 2),
                CU_TENSOR_MAP_SWIZZLE_128B, &luts);
@@ -978,19 +1006,25 @@ cudaError_t launch_one(const OneHotArgs& a, int ctas, cudaStream_t stream) {
   e = make_map(CU_TENSOR_MAP_DATA_TYPE_UINT32, a.codes, kTileWords, rows, kTileWords * 4, 32, kChunkGroups,
                CU_TENSOR_MAP_SWIZZLE_NONE, &codes);
   if (e != cudaSuccess) return e;
-  kern<<<static_cast<unsigned>(ctas), Config<ONE>::kThreads, kSmemBytes, stream>>>(luts, codes, a);
+  kern<<<static_cast<unsigned>(ctas), Config<V>::kThreads, kSmemBytes, stream>>>(luts, codes, a);
   return cudaGetLastError();
 }
 
 template <int MODE, int CAP>
 cudaError_t launch_t(const OneHotArgs& a, int ctas, cudaStream_t stream) {
   const bool one = a.nbg <= kFlushGroups;
-  if constexpr (MODE != kBucket) {
-    if (a.compact) {
-      return one ? launch_one<MODE, CAP, true, true>(a, ctas, stream) : launch_one<MODE, CAP, false, true>(a, ctas, stream);
+  if constexpr (MODE == kBucket) {
+    return one ? launch_one<MODE, CAP, kOne, false>(a, ctas, stream) : launch_one<MODE, CAP, kMulti, false>(a, ctas, stream);
+  } else {
+    if (a.tile_queries <= Config<kSmall>::kCols) {
+      return a.compact ? launch_one<MODE, CAP, kSmall, true>(a, ctas, stream)
+                       : launch_one<MODE, CAP, kSmall, false>(a, ctas, stream);
     }
+    if (a.compact) {
+      return one ? launch_one<MODE, CAP, kOne, true>(a, ctas, stream) : launch_one<MODE, CAP, kMulti, true>(a, ctas, stream);
+    }
+    return one ? launch_one<MODE, CAP, kOne, false>(a, ctas, stream) : launch_one<MODE, CAP, kMulti, false>(a, ctas, stream);
   }
-  return one ? launch_one<MODE, CAP, true, false>(a, ctas, stream) : launch_one<MODE, CAP, false, false>(a, ctas, stream);
 }
 
 // Ranges per query tile so that the items fill whole waves of CTA pairs: the
@@ -1040,7 +1074,7 @@ bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, O
   // at most 1/16 of it, 32768 vectors and 128 MiB of scores. (1000 queries x
   // 100k x 128, k = 10: scan + sample + selection 261 + 23 + 13 us with 1536
   // vectors, 188 + 35 + 25 us with the rule's 6144.)
-  const int stage = bits == 3 ? Groups<true>::kStage : Groups<false>::kStage;
+  const int stage = bits == 3 ? Groups<true, kOne>::kStage : Groups<false, kOne>::kStage;
   const long long n_stages = (nbg + stage - 1) / stage;
   plan->compact = bits == 3;
   long long sample = std::max<long long>(n / 64, 8192LL * k / n_stages);
