@@ -182,20 +182,9 @@ cudaError_t launch_scan(const ScanArgs& a, const ScanPlan& plan, cudaStream_t st
 cudaError_t launch_merge(const MergeArgs& a, cudaStream_t stream);
 
 // ---- batches of queries on the tensor cores (tq_onehot.cu) -------------------
-// The one-hot contraction costs the same up to about 64 queries, the lookup scan
-// grows with every four. Both measured (us per search, k = 10, lookup / one-hot):
-// 1M x 1536 4-bit 16 queries 1713 / 1642, 12 queries 1267 / 1641; 300k x 384
-// 2-bit 16 queries 141 / 134; 100k x 128 4-bit 32 queries 94 / 81, 24 queries
-// 69 / 80; 2M x 768 3-bit 32 queries 1987 / 1623, 24 queries 1430 / 1621 (3-bit
-// lookups take half the instructions). With k > 32 the lookup scan keeps its
-// lists in shared memory on one CTA per SM and loses from four queries on (1M x
-// 1536: 1716 / 1690; 100k x 128: 256 / 131).
-constexpr long long kOneHotMinQueries = 32;
-constexpr long long kOneHotMinQueriesWide = 16;        // 2- and 4-bit codes of at least ...
-constexpr long long kOneHotWideBytes = 20LL << 20;     // ... this many bytes
-constexpr long long kOneHotMinQueriesLists = 4;        // k > 32
-// Below this the launches (a sample, its thresholds) cost more than the scan.
-constexpr long long kOneHotMinVectors = 16384;
+// Which batches it takes over from the lookup scan is plan_onehot's estimate
+// (tq_onehot.cu); never an index below this size, where both are launches.
+constexpr long long kOneHotMinVectors = 8192;
 
 struct OneHotPlan {
   int tile_queries = 0;  // queries per tile (a multiple of 32, <= 256)

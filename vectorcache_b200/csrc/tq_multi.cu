@@ -335,8 +335,10 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
       set_direct(0);
       double best = h->time_ms(1);
       size_t best_d = 0;
-      for (size_t d : {size_t{1}, size_t{2}, size_t{4}, size_t{8}, size_t{16}, m}) {
-        if (d > m || d == 0) continue;
+      // The lightest of several batches always stays with the persistent launch.
+      const size_t most = m > 1 ? m - 1 : 1;
+      for (size_t d : {size_t{1}, size_t{2}, size_t{4}, size_t{8}, size_t{16}, most}) {
+        if (d > most) continue;
         set_direct(d);
         h->time_ms(1);
         const double ms = h->time_ms(1);
@@ -345,7 +347,7 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
           best = ms;
           best_d = d;
         }
-        if (d == m) break;
+        if (d == most) break;
       }
       set_direct(best_d);
     }

@@ -1049,12 +1049,45 @@ int choose_ranges(long long q_tiles, long long tiles, int pairs) {
   return 1;
 }
 
+// Whether a batch is faster here than on the lookup scan. Times in us beyond what
+// both spend (launches, query preparation, merge), fitted to searches of 8k to 2M
+// vectors of 128 to 1536 dimensions:
+//   * here, up to 64 queries: 25 for the sample, and 0.43 per 256-vector tile and
+//     16 byte groups (0.56 per 32 groups of 3-bit codes) on each CTA pair;
+//   * lookups, k <= 32, from three queries on: four queries a CTA over 2048-vector
+//     blocks, 0.31 per byte group (3-bit 0.17) and 14 per wave of two CTAs per SM,
+//     0.21 (0.11) per group while every CTA has an SM to itself. One and two
+//     queries stream the codes at HBM speed and stay there;
+//   * lookups, k > 32: lists in shared memory and a merge that sorts them; slower
+//     from three queries on everywhere, for one or two 15 + 0.035 (k - 8) per block
+//     over the stream of the codes.
+// Measured (lookup / here): 1M x 1536 4-bit 8 queries 937 / 1155, 12 queries
+// 1272 / 1155, 16 queries 1721 / 1155; 100k x 128 4-bit 24 queries 69 / 74, 32
+// queries 94 / 74; 2M x 768 3-bit 8 queries 647 / 774, 12 queries 826 / 774;
+// 20k x 768 4-bit 4 queries 125 / 85; one query of k = 64 over 100k x 128
+// 197 / 112, of k = 40 over 1M x 1536 706 / 1153, of k = 200 3431 / 1351.
+bool onehot_pays(long long n, long long nq, int nbg, int bits, int k, int sms) {
+  if (nq > Config<kSmall>::kCols) return true;
+  const long long pairs = sms / 2, tiles = (n + kPairVectors - 1) / kPairVectors;
+  const double blocks = static_cast<double>((n + kScanBlockVectors - 1) / kScanBlockVectors);
+  const double stages = static_cast<double>((nbg + (bits == 3 ? 31 : 15)) / (bits == 3 ? 32 : 16));
+  const double here = 25.0 + static_cast<double>((tiles + pairs - 1) / pairs) * stages * (bits == 3 ? 0.56 : 0.43);
+  if (nq <= 2) {
+    if (k <= 32) return false;
+    return static_cast<double>(n) * nbg / 4.8e6 + 15.0 + 0.035 * (k - 8) * blocks > here;
+  }
+  if (k > 32) return true;
+  const double ctas = static_cast<double>((nq + 3) / 4) * blocks;
+  double lookups = nbg * (bits == 3 ? 0.11 : 0.21);
+  if (ctas > sms) lookups = std::max(lookups, ctas / (2.0 * sms) * (nbg * (bits == 3 ? 0.17 : 0.31) + 14.0));
+  return lookups > here;
+}
+
 }  // namespace
 
 bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, OneHotPlan* plan) {
   if (n < kOneHotMinVectors || n > 0x7fffffffLL || nq < 1 || k < 1 || k > kMaxK || sms < 2) return false;
-  const bool wide = bits != 3 && n * nbg >= kOneHotWideBytes;
-  if (nq < (k > 32 ? kOneHotMinQueriesLists : (wide ? kOneHotMinQueriesWide : kOneHotMinQueries))) return false;
+  if (!onehot_pays(n, nq, nbg, bits, k, sms)) return false;
   const long long q_tiles = (nq + kMaxN - 1) / kMaxN;
   const long long per = (nq + q_tiles - 1) / q_tiles;
   plan->tile_queries = static_cast<int>((per + 31) / 32 * 32);
