@@ -594,45 +594,52 @@ __global__ void __launch_bounds__(1024) prefix_kernel(const uint32_t* __restrict
                                                       unsigned long long* __restrict__ out, int div,
                                                       unsigned long long* __restrict__ out_div,
                                                       unsigned long long* __restrict__ total_div) {
-  __shared__ unsigned long long part[1024];
-  __shared__ unsigned long long part_d[1024];
-  __shared__ unsigned long long carry, carry_d;
-  if (threadIdx.x == 0) {
-    carry = 0;
-    carry_d = 0;
-  }
+  __shared__ unsigned long long s_warp[2][32];
+  __shared__ unsigned long long s_carry[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 2) s_carry[threadIdx.x] = 0ull;
   __syncthreads();
   for (int base = 0; base < nb; base += 1024) {
     const int i = base + threadIdx.x;
     const unsigned long long c = i < nb ? counts[i] : 0ull;
     const unsigned long long cd = (i < nb && div > 0) ? (c + div - 1) / div : 0ull;
-    part[threadIdx.x] = c;
-    part_d[threadIdx.x] = cd;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      const unsigned long long v = threadIdx.x >= o ? part[threadIdx.x - o] : 0ull;
-      const unsigned long long vd = threadIdx.x >= o ? part_d[threadIdx.x - o] : 0ull;
-      __syncthreads();
-      part[threadIdx.x] += v;
-      part_d[threadIdx.x] += vd;
-      __syncthreads();
+    unsigned long long ic = c, id = cd;  // inclusive sums over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(full_mask(), ic, o), vd = __shfl_up_sync(full_mask(), id, o);
+      if (lane >= o) {
+        ic += v;
+        id += vd;
+      }
     }
+    if (lane == 31) {
+      s_warp[0][warp] = ic;
+      s_warp[1][warp] = id;
+    }
+    __syncthreads();
+    if (warp < 2) {  // warp 0 scans the counts' warp sums, warp 1 the quotients'
+      unsigned long long v = s_warp[warp][lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(full_mask(), v, o);
+        if (lane >= o) v += t;
+      }
+      s_warp[warp][lane] = v;
+    }
+    __syncthreads();
     if (i < nb) {
-      out[i] = carry + part[threadIdx.x] - c;
-      if (div > 0) out_div[i] = carry_d + part_d[threadIdx.x] - cd;
+      out[i] = s_carry[0] + (warp ? s_warp[0][warp - 1] : 0ull) + ic - c;
+      if (div > 0) out_div[i] = s_carry[1] + (warp ? s_warp[1][warp - 1] : 0ull) + id - cd;
     }
     __syncthreads();
-    if (threadIdx.x == 1023) {
-      carry += part[1023];
-      carry_d += part_d[1023];
-    }
+    if (threadIdx.x < 2) s_carry[threadIdx.x] += s_warp[threadIdx.x][31];
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    out[nb] = carry;
+    out[nb] = s_carry[0];
     if (div > 0) {
-      out_div[nb] = carry_d;
-      if (total_div) *total_div = carry_d;
+      out_div[nb] = s_carry[1];
+      if (total_div) *total_div = s_carry[1];
     }
   }
 }
@@ -972,56 +979,136 @@ __device__ __forceinline__ bool pair_in_range(const PairArgs& a, long long q, in
   return j >= lo && j < hi && j < np;
 }
 
-__global__ void pair_count_kernel(PairArgs a) {
+// The step's probe positions: thread t of `window` positions a query from
+// window_begin on -> its query and position.
+__device__ __forceinline__ bool pair_of(const PairArgs& a, long long t, int begin, int window, long long* q, int* j) {
+  *q = t / window;
+  *j = begin + static_cast<int>(t % window);
+  return pair_in_range(a, *q, *j);
+}
+
+__global__ void pair_count_kernel(PairArgs a, int begin, int window) {
   const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= a.nq * a.max_probe) return;
-  const long long q = t / a.max_probe;
-  const int j = static_cast<int>(t % a.max_probe);
-  if (!pair_in_range(a, q, j)) return;
+  long long q;
+  int j;
+  if (t >= a.nq * window || !pair_of(a, t, begin, window, &q, &j)) return;
   const uint32_t b = a.probes[q * (a.probe_stride ? a.probe_stride : a.max_probe) + j];
   if (b < static_cast<uint32_t>(a.nb)) atomicAdd(&a.counts[b], 1u);
 }
 
-__global__ void pair_scatter_kernel(PairArgs a) {
+// Groups the pairs and reads each one's offset <q_hat, enc[b]> from the
+// q_hat . enc^T product computed before.
+__global__ void pair_scatter_kernel(PairArgs a, int begin, int window) {
   const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= a.nq * a.max_probe) return;
-  const long long q = t / a.max_probe;
-  const int j = static_cast<int>(t % a.max_probe);
-  if (!pair_in_range(a, q, j)) return;
+  long long q;
+  int j;
+  if (t >= a.nq * window || !pair_of(a, t, begin, window, &q, &j)) return;
   const uint32_t b = a.probes[q * (a.probe_stride ? a.probe_stride : a.max_probe) + j];
   if (b >= static_cast<uint32_t>(a.nb)) return;
   const unsigned long long pos = a.pair_start[b] + atomicAdd(&a.fill[b], 1u);
-  a.pairs[pos] = static_cast<uint32_t>(t);
+  const long long pair = q * a.max_probe + j;
+  a.pairs[pos] = static_cast<uint32_t>(pair);
+  a.offsets[pair] = a.enc_scores[q * a.enc_ld + b];
 }
 
-// One thread per (query, probe): the offset <q_hat, enc[b]> read from the
-// q_hat . enc^T product computed before the pairs.
-__global__ void pair_offset_gather_kernel(PairArgs a) {
-  const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= a.nq * a.max_probe) return;
-  const long long q = t / a.max_probe;
-  const int j = static_cast<int>(t % a.max_probe);
-  if (!pair_in_range(a, q, j)) return;
-  const uint32_t b = a.probes[q * (a.probe_stride ? a.probe_stride : a.max_probe) + j];
-  if (b >= static_cast<uint32_t>(a.nb)) return;
-  a.offsets[t] = a.enc_scores[q * a.enc_ld + b];
-}
-
-__global__ void item_build_kernel(PairArgs a) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.nb) return;
-  const unsigned long long c = a.pair_start[b + 1] - a.pair_start[b];
-  const unsigned long long i0 = a.item_start[b];
+// Bucket b's work items: its c pairs from `first` on, numbered from item i0.
+__device__ __forceinline__ void write_items(const PairArgs& a, int b, unsigned long long c, unsigned long long first,
+                                            unsigned long long i0) {
   unsigned long long per = static_cast<unsigned long long>(a.item_queries);
   if (a.even_items && c > per) {
     const unsigned long long parts = (c + per - 1) / per;
     per = (c + parts - 1) / parts;
   }
   for (unsigned long long t = 0; t * per < c; ++t) {
-    const unsigned long long first = a.pair_start[b] + t * per;
-    const unsigned long long cnt = min(per, c - t * per);
-    a.items[i0 + t] = make_uint4(static_cast<unsigned>(b), static_cast<unsigned>(first),
-                                 static_cast<unsigned>(cnt), 0u);
+    a.items[i0 + t] = make_uint4(static_cast<unsigned>(b), static_cast<unsigned>(first + t * per),
+                                 static_cast<unsigned>(min(per, c - t * per)), 0u);
+  }
+}
+
+__global__ void item_build_kernel(PairArgs a) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= a.nb) return;
+  write_items(a, b, a.pair_start[b + 1] - a.pair_start[b], a.pair_start[b], a.item_start[b]);
+}
+
+// The whole grouping in one CTA for few pairs, counts and fills in shared memory:
+// the five kernels and two memsets it replaces cost about 38 us a step, and a
+// 16-query search takes three steps. Bucket counts are scanned 1024 at a time.
+constexpr int kSmallPairThreads = 1024;
+constexpr int kSmallPairBuckets = 11 * 1024;
+constexpr long long kSmallPairs = 16384;
+__global__ void __launch_bounds__(kSmallPairThreads) pair_small_kernel(PairArgs a, int begin, int window) {
+  extern __shared__ uint32_t s_count[];  // nb counts, then the next free place of each bucket
+  __shared__ uint32_t s_warp[2][32];
+  __shared__ uint32_t s_base[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b = threadIdx.x; b < a.nb; b += kSmallPairThreads) s_count[b] = 0u;
+  if (threadIdx.x < 2) s_base[threadIdx.x] = 0u;
+  __syncthreads();
+  const int stride = a.probe_stride ? a.probe_stride : a.max_probe;
+  const long long total = a.nq * window;
+  for (long long t = threadIdx.x; t < total; t += kSmallPairThreads) {
+    long long q;
+    int j;
+    if (!pair_of(a, t, begin, window, &q, &j)) continue;
+    const uint32_t b = a.probes[q * stride + j];
+    if (b < static_cast<uint32_t>(a.nb)) atomicAdd(&s_count[b], 1u);
+  }
+  __syncthreads();
+  for (int b0 = 0; b0 < a.nb; b0 += kSmallPairThreads) {
+    const int b = b0 + static_cast<int>(threadIdx.x);
+    const uint32_t c = b < a.nb ? s_count[b] : 0u;
+    const uint32_t n = (c + a.item_queries - 1) / a.item_queries;
+    uint32_t ic = c, in = n;  // inclusive sums over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t tc = __shfl_up_sync(full_mask(), ic, o), tn = __shfl_up_sync(full_mask(), in, o);
+      if (lane >= o) {
+        ic += tc;
+        in += tn;
+      }
+    }
+    if (lane == 31) {
+      s_warp[0][warp] = ic;
+      s_warp[1][warp] = in;
+    }
+    __syncthreads();
+    if (warp < 2) {
+      uint32_t v = s_warp[warp][lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(full_mask(), v, o);
+        if (lane >= o) v += t;
+      }
+      s_warp[warp][lane] = v;
+    }
+    __syncthreads();
+    const uint32_t first = s_base[0] + (warp ? s_warp[0][warp - 1] : 0u) + ic - c;
+    const uint32_t item = s_base[1] + (warp ? s_warp[1][warp - 1] : 0u) + in - n;
+    if (b < a.nb) {
+      a.pair_start[b] = first;
+      a.item_start[b] = item;
+      write_items(a, b, c, first, item);
+      s_count[b] = first;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) s_base[threadIdx.x] += s_warp[threadIdx.x][31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    a.pair_start[a.nb] = s_base[0];
+    a.item_start[a.nb] = s_base[1];
+    *a.n_items = s_base[1];
+  }
+  for (long long t = threadIdx.x; t < total; t += kSmallPairThreads) {
+    long long q;
+    int j;
+    if (!pair_of(a, t, begin, window, &q, &j)) continue;
+    const uint32_t b = a.probes[q * stride + j];
+    if (b >= static_cast<uint32_t>(a.nb)) continue;
+    const long long pair = q * a.max_probe + j;
+    a.pairs[atomicAdd(&s_count[b], 1u)] = static_cast<uint32_t>(pair);
+    a.offsets[pair] = a.enc_scores[q * a.enc_ld + b];
   }
 }
 
@@ -1743,21 +1830,28 @@ long long max_items(long long nq, int max_probe, int nb) {
 }
 
 cudaError_t launch_build_pairs(const PairArgs& a, cudaStream_t stream) {
+  // The positions the step can take: a last step starts after the first probes,
+  // at least kFloorProbes of every query that has more.
+  const int begin = a.first_split == 2 ? std::max(a.probe_begin, std::min(kFloorProbes, a.max_probe)) : a.probe_begin;
+  const int end = a.first_split == 1 ? std::min(a.probe_end, kFloorProbesWide) : a.probe_end;
+  const int window = std::max(1, std::min(end, a.max_probe) - begin);
+  const long long total = a.nq * window;
+  if (total <= kSmallPairs && a.nb <= kSmallPairBuckets) {
+    pair_small_kernel<<<1, kSmallPairThreads, static_cast<size_t>(a.nb) * 4, stream>>>(a, begin, window);
+    return cudaGetLastError();
+  }
   cudaError_t e = cudaMemsetAsync(a.counts, 0, static_cast<size_t>(a.nb) * 4, stream);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(a.fill, 0, static_cast<size_t>(a.nb) * 4, stream);
   if (e != cudaSuccess) return e;
-  const long long total = a.nq * a.max_probe;
   if (total > 0) {
-    pair_count_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a);
+    pair_count_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a, begin, window);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   prefix_kernel<<<1, 1024, 0, stream>>>(a.counts, a.nb, a.pair_start, a.item_queries, a.item_start, a.n_items);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (total > 0) {
-    pair_scatter_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    pair_offset_gather_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a);
+    pair_scatter_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a, begin, window);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   item_build_kernel<<<static_cast<unsigned>((a.nb + 255) / 256), 256, 0, stream>>>(a);
