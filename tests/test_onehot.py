@@ -1,13 +1,16 @@
 """Batches of queries on the tensor cores (tq_onehot.cu) against the CPU oracle,
 bit for bit: ids and scores of the top k at the edges of its tiles (256 vectors,
 32-query steps up to 192, 8 byte groups per stage, 256 per flush batch) and of
-its lists (k up to 64, up to 256), with equal scores across tiles."""
+its lists (k up to 64, up to 256), with equal scores across tiles. Batches above
+64 queries always run there; smaller ones by an estimate (k > 32 from three
+queries on). Bucketed passes of at least 16 pairs per bucket against passes
+small enough for the lookup scan."""
 import numpy as np
 import pytest
 
 import vectorcache_b200 as vcb
 from oracle.oracle import Oracle
-from vectorcache_b200.synthetic import power_law
+from vectorcache_b200.synthetic import power_law, vmf_mixture
 
 pytestmark = pytest.mark.gpu
 
@@ -47,6 +50,11 @@ def check(oracle, dim, bits, n, nq, k, tqplus=True, duplicates=False, order=None
     (520, 4, 16384, 64, 33),     # 260 groups: a flush batch of four
     (1024, 3, 16500, 5, 65),     # lists of 512 entries, five queries
     (136, 4, 40000, 385, 256),   # the largest k, three query tiles
+    (8, 4, 8192, 65, 10),        # the smallest index, one part-full stage
+    (24, 2, 16385, 66, 1),       # 6 byte groups, one vector in the last tile
+    (520, 3, 8449, 96, 10),      # 3-bit rows over two flush batches
+    (1032, 4, 9000, 64, 33),     # 516 groups: three flush batches, the small-batch form
+    (64, 3, 9000, 3, 40),        # three queries, 3-bit, the small-batch form
 ])
 def test_equals_the_oracle(oracle, dim, bits, n, nq, k):
     check(oracle, dim, bits, n, nq, k)
@@ -54,8 +62,45 @@ def test_equals_the_oracle(oracle, dim, bits, n, nq, k):
 
 def test_equal_scores_keep_the_lower_ids(oracle):
     check(oracle, 64, 4, 18000, 36, 12, tqplus=False, duplicates=True)
+    check(oracle, 64, 4, 18000, 70, 12, tqplus=False, duplicates=True)
 
 
 @pytest.mark.parametrize("k", [10, 100])
 def test_lists_that_overflow(oracle, k):
     check(oracle, 32, 4, 60000, 32, k, order="ascending")
+
+
+def test_many_queries_overflow_lists(oracle):
+    check(oracle, 32, 4, 60000, 70, 10, order="ascending")
+
+
+@pytest.mark.parametrize("dim,bits,n,k,n_probe,rerank_k", [
+    (100, 4, 12000, 10, 24, 40),
+    (51, 3, 12000, 7, 33, 0),      # dims padded to 56, 28 byte groups
+    (48, 2, 12000, 64, 40, 0),     # 12 byte groups: less than two stages
+    (520, 4, 6000, 10, 20, 0),     # two flush batches
+    # k = 1: a floor from one bucket, then random queries put more scores above
+    # it than a query's region holds: the redo kernel.
+    (64, 4, 12000, 1, 16, 0),
+])
+def test_bucketed_pass_equals_small_passes(dim, bits, n, k, n_probe, rerank_k):
+    db = vmf_mixture(n, dim, seed=21, clusters=60)
+    idx = vcb.BucketedTurboQuantIndex(dim, bits, vcb.BucketParams(
+        n_probe=8, max_bucket_size=300, energy_soft=150, kmeans_iters=3, seed=7, rerank_k=rerank_k))
+    idx.add(db)
+    idx.prepare()
+    nb = idx.info()["n_buckets"]
+    nq = 16 * nb + 5  # every step holds at least 16 pairs per bucket
+    q = np.random.default_rng(22).standard_normal((nq, dim)).astype(np.float32)
+    whole = idx.search(q, k, n_probe=n_probe)
+    step = nb // 4  # probes 1..7 and the far ones stay below 16 pairs per bucket
+    for s in range(0, min(nq, 8 * step), step):
+        part = idx.search(q[s:s + step], k, n_probe=n_probe)
+        assert np.array_equal(whole.ids[s:s + step], part.ids), s
+        assert np.array_equal(whole.scores[s:s + step].view(np.uint32), part.scores.view(np.uint32)), s
+    counts = (np.arange(nq) % n_probe + 1).astype(np.uint32)
+    mixed = idx.search(q, k, n_probe=n_probe, n_probe_per_query=counts)
+    rows = np.nonzero(counts == n_probe)[0]
+    assert np.array_equal(mixed.ids[rows], whole.ids[rows])
+    assert np.array_equal(mixed.scores[rows].view(np.uint32), whole.scores[rows].view(np.uint32))
+    idx.close()

@@ -191,6 +191,11 @@ cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStre
 // above the region's size, where the appends past its end are missing.
 constexpr int kOneHotItemQueries = 192;
 constexpr long long kOneHotPairsPerBucket = 16;
+// Its 32-bit offsets: slots, and bytes of the pass's LUTs (16,384 queries of 16,384
+// 4-bit dims are just too many); a pass that does not fit keeps launch_bucket_scan.
+constexpr bool onehot_buckets_fit(long long nq, long long n_slots, int nbg) {
+  return n_slots <= 0x7fffffffLL && nq * nbg * 32 <= 0xffffffffLL;
+}
 cudaError_t launch_onehot_buckets(const BucketScanArgs& a, long long nq, long long n_slots, int sms, unsigned* status,
                                   cudaStream_t stream);
 // Scans again, list by list, every query whose append_count passed its region:

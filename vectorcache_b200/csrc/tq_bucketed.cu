@@ -524,7 +524,8 @@ struct tq_bucketed {
       // Above a floor, steps with enough pairs per bucket go to the tensor cores.
       bool any_onehot = false, onehot = false;
       auto use_onehot = [&](long long step_pairs) {
-        onehot = ba.floor && step_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2;
+        onehot = ba.floor && step_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2 &&
+                 vcb::onehot_buckets_fit(static_cast<long long>(m), static_cast<long long>(n_slots), ba.nbg);
         pa.item_queries = onehot ? vcb::kOneHotItemQueries : vcb::kItemQueries;
         pa.even_items = onehot;
         any_onehot |= onehot;
@@ -535,7 +536,7 @@ struct tq_bucketed {
           return;
         }
         eng->check_status = true;
-        eng->status_foreign |= s != eng->stream;
+        if (s != eng->stream) eng->status_foreign = true;
         eng->launch(tq_index::kScan, s, what, [&] {
           return vcb::launch_onehot_buckets(ba, static_cast<long long>(m), static_cast<long long>(n_slots), eng->sms,
                                             eng->device_status(), s);

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <string>
@@ -186,7 +187,8 @@ struct tq_index {
   // Set once a search ran a kernel with bounded waits: sync() then looks at the
   // word such a kernel sets when a wait gave up (behind d_counter's count).
   // A search on another stream may still be running then: it keeps the flag set.
-  bool check_status = false, status_foreign = false;
+  // (Searches of one index may be queued from several threads.)
+  std::atomic<bool> check_status{false}, status_foreign{false};
 
   // Optional per-launch timing (tq_index_set_profiling).
   enum Kind { kPrep = 0, kScan = 1, kMerge = 2, kEncode = 3 };
@@ -253,7 +255,7 @@ struct tq_index {
       unsigned status = 0;
       vcb::check(cudaMemcpyAsync(&status, device_status(), 4, cudaMemcpyDeviceToHost, stream), "D2H");
       vcb::check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-      check_status = status_foreign;
+      check_status = status_foreign.load();
       if (status) {
         vcb::check(cudaMemsetAsync(device_status(), 0, 4, stream), "cudaMemsetAsync");
         vcb::fail(TQ_ERR_CUDA, "a scan kernel gave up waiting on its own pipeline; its results are not valid");
@@ -498,7 +500,7 @@ struct tq_index {
     }
     a.status = device_status();
     check_status = true;
-    status_foreign |= s != stream;
+    if (s != stream) status_foreign = true;
     launch(kPrep, s, "threshold sample kernel", [&] { return vcb::launch_onehot_sample(a, p, sms, s); });
     launch(kPrep, s, "threshold kernel", [&] {
       return vcb::launch_kth_floor(a.dense, static_cast<long long>(p.sample_tiles) * 256, nullptr,

@@ -187,7 +187,7 @@ cudaError_t launch_merge(const MergeArgs& a, cudaStream_t stream);
 constexpr long long kOneHotMinVectors = 8192;
 
 struct OneHotPlan {
-  int tile_queries = 0;  // queries per tile (a multiple of 32, <= 256)
+  int tile_queries = 0;  // queries per tile (a multiple of 32, <= 192)
   int q_tiles = 0;
   int tiles = 0;         // 256-vector tiles of the index
   int range_tiles = 0, n_ranges = 0;

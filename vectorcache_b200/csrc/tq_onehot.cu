@@ -11,18 +11,19 @@
 // for bit to tq_scan.cu's.
 //
 // A pair of CTAs (cta_group::2) owns a tile of 256 vectors (128 per CTA) x N
-// queries (N <= 192). Per stage of 4 byte groups (128 bytes of K):
-//   * a TMA load per CTA brings its half of the N queries' LUT bytes to shared
+// queries (N <= 192). Per stage of 8 byte groups (256 bytes of K; 512 for at most
+// 64 queries, and 3-bit codes take half the K per group):
+//   * TMA loads bring each CTA's half of the N queries' LUT bytes to shared
 //     memory (K-major, 128-byte swizzle);
-//   * four of eight producer warps read the codes, build each vector's one-hot
-//     row in registers (its own TMEM lane) and store it to TMEM;
-//   * one thread of the pair issues four K = 32 MMAs (A in TMEM, B in shared
-//     memory).
+//   * eight producer warps, two sets of four, read the codes, build each vector's
+//     one-hot row in registers (its own TMEM lane) and store it to TMEM;
+//   * one thread of the pair issues a K = 32 MMA per byte group (A in TMEM, B in
+//     shared memory).
 // The one-hot operand lives in TMEM because shared memory could not carry it as
 // well: writing and reading it there next to the LUT tiles takes all of the 128
 // bytes per clock at N = 256 (measured: 631 clocks per stage instead of 512).
 // Accumulators are double-buffered in TMEM per 256-group batch (2 x 192 columns,
-// the other 128 hold four one-hot stages); eight warps per CTA read them back,
+// the other 128 hold two one-hot stages); eight warps per CTA read them back,
 // keep the f32 sums in registers across batches (96 queries each), and append
 // scores at or above the query's threshold to a list, cut back to the top k when
 // it fills up.
@@ -416,8 +417,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<V>::kThreads,
       // row, in the 128-byte swizzle (16-byte chunk c of row r at c ^ (r % 8)); the
       // copies arrive at landed_b themselves and warp 19 passes them on.
       // A one-row-box TMA gather (tile::gather4) took about 77 clocks per four
-      // rows and bound the kernel (10k queries x 464 probes of 1.2M x 100: 8.8 ms
-      // against GATHER_MS). Warp 16 also loads the code chunks.
+      // rows and bound the kernel (far scan of 10k queries x 464 probes of 1.2M x
+      // 100: 8.8 ms, 4.9 ms with the copies). Warp 16 also loads the code chunks.
       // Two pairs of warps (ONE) take the stages in turn.
       const int which = warp == 18 || warp == 21;
       const int team = warp >= 20;
@@ -448,27 +449,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<V>::kThreads,
             }
             if (!alive) break;
             if (st % Config<V>::kGatherTeams == team) {
-            if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) alive = false;
-            if (!alive) break;
-            const uint32_t at = static_cast<uint32_t>(s) * 256 + which * 128 + cl * 16;
-            const uint32_t bytes = at < row_bytes ? 16u : 0u;  // zero past the row's end
-            const uint8_t* src = a.luts + (bytes ? at : 0u);
-            uint32_t dst = sB + (st * kTiles + which) * kTileBytes;
-            // Eight rows' offsets first: read one by one between the copies, their
-            // latency added up to 76 clocks a copy.
-            for (int i = 0; i < groups4; i += 8, dst += 4096) {
-              uint32_t off[8];
+              if (!__all_sync(full_mask(), tc::mbar_wait(tc::smem_u32(&sh.empty_b[st]), ph ^ 1u))) alive = false;
+              if (!alive) break;
+              const uint32_t at = static_cast<uint32_t>(s) * 256 + which * 128 + cl * 16;
+              const uint32_t bytes = at < row_bytes ? 16u : 0u;  // zero past the row's end
+              const uint8_t* src = a.luts + (bytes ? at : 0u);
+              uint32_t dst = sB + (st * kTiles + which) * kTileBytes;
+              // Eight rows' offsets first: read one by one between the copies, their
+              // latency added up to 76 clocks a copy.
+              for (int i = 0; i < groups4; i += 8, dst += 4096) {
+                uint32_t off[8];
 #pragma unroll
-              for (int u = 0; u < 8; ++u) off[u] = row[4 * (i + u)];
+                for (int u = 0; u < 8; ++u) off[u] = row[4 * (i + u)];
 #pragma unroll
-              for (int u = 0; u < 8; u += 2) {
-                if (i + u < groups4) {
-                  tc::cp_async16_zfill(dst + u * 512 + dst_even, src + off[u], bytes);
-                  tc::cp_async16_zfill(dst + u * 512 + 512 + dst_odd, src + off[u + 1], bytes);
+                for (int u = 0; u < 8; u += 2) {
+                  if (i + u < groups4) {
+                    tc::cp_async16_zfill(dst + u * 512 + dst_even, src + off[u], bytes);
+                    tc::cp_async16_zfill(dst + u * 512 + 512 + dst_odd, src + off[u + 1], bytes);
+                  }
                 }
-              }
             }
-            tc::cp_async_arrive(tc::smem_u32(&sh.landed_b[st]));
+              tc::cp_async_arrive(tc::smem_u32(&sh.landed_b[st]));
             }
             if (++st == kStagesB) {
               st = 0;
@@ -1163,8 +1164,7 @@ cudaError_t launch_onehot_scan(const OneHotArgs& in, const OneHotPlan& p, cudaSt
 
 cudaError_t launch_onehot_buckets(const BucketScanArgs& b, long long nq, long long n_slots, int sms, unsigned* status,
                                   cudaStream_t stream) {
-  if (!b.append_count || !b.floor || b.n_items == nullptr || n_slots > 0x7fffffffLL ||
-      nq * b.nbg * 32 > 0xffffffffLL) {
+  if (!b.append_count || !b.floor || b.n_items == nullptr || !onehot_buckets_fit(nq, n_slots, b.nbg)) {
     return cudaErrorInvalidValue;
   }
   OneHotArgs a{};
