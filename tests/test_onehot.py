@@ -79,9 +79,10 @@ def test_many_queries_overflow_lists(oracle):
     (51, 3, 12000, 7, 33, 0),      # dims padded to 56, 28 byte groups
     (48, 2, 12000, 64, 40, 0),     # 12 byte groups: less than two stages
     (520, 4, 6000, 10, 20, 0),     # two flush batches
-    # k = 1: a floor from one bucket, then random queries put more scores above
-    # it than a query's region holds: the redo kernel.
-    (64, 4, 12000, 1, 16, 0),
+    (64, 4, 12000, 1, 16, 0),      # a floor of one score
+    # zero queries: every score equals the floor, more of them than a query's
+    # region holds (4096 entries): the redo kernel.
+    (64, 4, 12000, 1, 64, 0),
 ])
 def test_bucketed_pass_equals_small_passes(dim, bits, n, k, n_probe, rerank_k):
     db = vmf_mixture(n, dim, seed=21, clusters=60)
@@ -92,6 +93,8 @@ def test_bucketed_pass_equals_small_passes(dim, bits, n, k, n_probe, rerank_k):
     nb = idx.info()["n_buckets"]
     nq = 16 * nb + 5  # every step holds at least 16 pairs per bucket
     q = np.random.default_rng(22).standard_normal((nq, dim)).astype(np.float32)
+    if n_probe == 64:
+        q[::5] = 0.0
     whole = idx.search(q, k, n_probe=n_probe)
     step = nb // 4  # probes 1..7 and the far ones stay below 16 pairs per bucket
     for s in range(0, min(nq, 8 * step), step):

@@ -1515,8 +1515,7 @@ __device__ __forceinline__ void bucket_scan_item(const BucketScanArgs& a, const 
       const int q = static_cast<int>(pr / static_cast<uint32_t>(a.max_probe));
       iq.q[t] = q;
       // (query, probe) lists, or the query's region when appending
-      iq.list[t] = (a.append_count ? static_cast<long long>(q) * a.max_probe : static_cast<long long>(pr)) *
-                   kBsListsPerProbe;
+      iq.list[t] = a.append_count ? static_cast<long long>(q) * a.lists : static_cast<long long>(pr) * kBsListsPerProbe;
       iq.scale[t] = a.lut_scale[q];
       iq.init[t] = a.fa_init[q];
       iq.off[t] = a.offsets[pr];
@@ -1568,8 +1567,7 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ ItemQueries iq;
   const int q = static_cast<int>(blockIdx.x);
-  const long long region = static_cast<long long>(a.max_probe) * kBsListsPerProbe * a.k;
-  if (a.append_count[q] <= region) return;  // the whole CTA
+  if (a.append_count[q] <= a.lists * a.k) return;  // the whole CTA
   __syncthreads();
   if (threadIdx.x == 0) a.append_count[q] = 0u;
   const int np = n_probe ? min(static_cast<int>(n_probe[q]), a.max_probe) : fixed_probe;
@@ -1580,7 +1578,7 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5)
     if (threadIdx.x < kItemQueries) {
       const int t = threadIdx.x;
       iq.q[t] = t == 0 ? q : -1;
-      iq.list[t] = t == 0 ? static_cast<long long>(q) * a.max_probe * kBsListsPerProbe : 0;
+      iq.list[t] = t == 0 ? static_cast<long long>(q) * a.lists : 0;
       iq.scale[t] = t == 0 ? a.lut_scale[q] : 0.f;
       iq.init[t] = t == 0 ? a.fa_init[q] : 0.f;
       iq.off[t] = t == 0 ? a.offsets[static_cast<long long>(q) * a.max_probe + j] : 0.f;

@@ -172,16 +172,18 @@ struct BucketScanArgs {
   const unsigned long long* n_items;
   unsigned long long* next_item;  // work counter (zeroed by launch_bucket_scan)
   int nbg, bits, k, max_probe;
-  float* cand_score;         // (nq * max_probe * kBsListsPerProbe) lists of k
+  float* cand_score;         // (nq * max_probe * kBsListsPerProbe) lists of k, appending: nq * lists
   uint32_t* cand_id;
   // Optional per query: scores below floor[q] cannot reach the query's top k
   // and are not kept (nullptr: no floor).
   const float* floor = nullptr;
   // Optional per query (zeroed by the caller): the kept candidates of query q
-  // are appended, unpadded, to its region of L = max_probe * kBsListsPerProbe
-  // lists of k entries at cand_score/cand_id + q * L * k, and append_count[q]
-  // counts them. nullptr: one -inf padded list of k per (query, probe, tile set).
+  // are appended, unpadded, to its region of `lists` lists of k entries (at least
+  // max_probe * kBsListsPerProbe) at cand_score/cand_id + q * lists * k, and
+  // append_count[q] counts them. nullptr: one -inf padded list of k per (query,
+  // probe, tile set).
   uint32_t* append_count = nullptr;
+  long long lists = 0;
 };
 // `grid`: a bound of the item count; the launch runs min(grid, resident CTAs).
 cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStream_t stream);
@@ -191,6 +193,11 @@ cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStre
 // above the region's size, where the appends past its end are missing.
 constexpr int kOneHotItemQueries = 192;
 constexpr long long kOneHotPairsPerBucket = 16;
+// Entries a region holds at least: what passes a floor of one bucket is no list of
+// k, and one query past its region costs a scan of all its probes by one CTA (1,893
+// queries x 27 probes of 84,838 x 119, k = 24, regions of 648: that kernel took 388
+// of 876 us).
+constexpr long long kOneHotMinRegion = 4096;
 // Its 32-bit offsets: slots, and bytes of the pass's LUTs (16,384 queries of 16,384
 // 4-bit dims are just too many); a pass that does not fit keeps launch_bucket_scan.
 constexpr bool onehot_buckets_fit(long long nq, long long n_slots, int nbg) {

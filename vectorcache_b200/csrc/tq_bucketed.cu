@@ -391,6 +391,15 @@ struct tq_bucketed {
     });
   }
 
+  // Lists of kscan entries in a query's candidate region: one per probe, and at
+  // least kOneHotMinRegion entries (or all its probes' vectors) where a search
+  // has steps above a floor.
+  size_t region_lists(size_t max_probe, size_t kscan) const {
+    const size_t lists = max_probe * vcb::kBsListsPerProbe;
+    if (max_probe <= static_cast<size_t>(vcb::kFloorProbes)) return lists;
+    const size_t entries = std::min<size_t>(vcb::kOneHotMinRegion, max_probe * p.max_bucket_size);
+    return std::max(lists, (entries + kscan - 1) / kscan);
+  }
   // Queries per pass: routing scores (nb floats per query) within 256 MiB and
   // candidate lists (max_probe lists of kscan (score, id) per query) within
   // 8 GiB — 13,981 queries at 768 probes and a re-rank of 100. Every pass
@@ -400,7 +409,7 @@ struct tq_bucketed {
   size_t pass_queries(size_t max_probe = 1, size_t kscan = 1) const {
     const size_t by_route = std::max<size_t>(1, (size_t{256} << 20) / (static_cast<size_t>(nb) * 4));
     const size_t by_cand =
-        std::max<size_t>(1, (size_t{8} << 30) / (max_probe * vcb::kBsListsPerProbe * kscan * 8));
+        std::max<size_t>(1, (size_t{8} << 30) / (region_lists(max_probe, kscan) * kscan * 8));
     return std::min<size_t>({16384, by_route, by_cand});
   }
 
@@ -479,9 +488,9 @@ struct tq_bucketed {
       });
       pa.enc_scores = sc.encs.as<float>();
       pa.enc_ld = nb;
-      const size_t lists = m * max_probe * vcb::kBsListsPerProbe;
-      sc.cand_s.reserve(lists * kscan * 4);
-      sc.cand_i.reserve(lists * kscan * 4);
+      const size_t lists = region_lists(static_cast<size_t>(max_probe), kscan);
+      sc.cand_s.reserve(m * lists * kscan * 4);
+      sc.cand_i.reserve(m * lists * kscan * 4);
       sc.floor.reserve(m * 4);
       const float* qf = sc.flat.qf.as<float>();
       vcb::BucketScanArgs ba{};
@@ -509,6 +518,7 @@ struct tq_bucketed {
       sc.acount.reserve(m * 4);
       if (!vcb::dry_run_flag()) vcb::check(cudaMemsetAsync(sc.acount.get(), 0, m * 4, s), "cudaMemsetAsync");
       ba.append_count = sc.acount.as<uint32_t>();
+      ba.lists = static_cast<long long>(lists);
       // The best-routed buckets first: the k-th best score over a query's
       // first 8 (32 from 128 probes) probes is a lower bound of its k-th best over all
       // probes, so the scan of the remaining probes keeps only scores at or
@@ -543,8 +553,7 @@ struct tq_bucketed {
         });
       };
       if (two_phase) {
-        // a query's candidate region: max_probe lists of kscan entries
-        const long long region = static_cast<long long>(max_probe) * vcb::kBsListsPerProbe * kscan;
+        const long long region = ba.lists * static_cast<long long>(kscan);
         // Probe 0 alone, then probes 1..first-1 above probe 0's floor (the
         // first probes cost most without a floor), then the floor of all
         // first probes for the rest. Each floor is the k-th best of the
@@ -602,7 +611,7 @@ struct tq_bucketed {
       mg.cand_score = ba.cand_score;
       mg.cand_id = ba.cand_id;
       mg.nq = static_cast<long long>(m);
-      mg.n_lists = max_probe * vcb::kBsListsPerProbe;
+      mg.n_lists = static_cast<int>(lists);
       mg.k = static_cast<int>(kscan);
       mg.k_out = static_cast<int>(kscan);
       mg.out_score = d_scores + q0 * ke;
