@@ -1170,6 +1170,9 @@ struct ItemView {
   // (in lists of k) of the query's candidate region and the kept candidates
   // are appended there at append_count[query] (atomically), unpadded.
   uint32_t* append_count = nullptr;
+  // Appending, QW = 2: the warps that an item of at most four queries leaves idle
+  // take tile sets of its own (up to kBsWarps lists of k per query).
+  bool split = false;
 };
 
 // The item's queries, in shared memory (filled by the calling kernel).
@@ -1184,15 +1187,20 @@ struct ItemQueries {
 // (query, tile set). QW = 4: 2 groups of 4 queries x 2 tile sets (a warp scans
 // every other 256-slot tile set); QW = 2: 4 groups of 2 queries x 1 tile set
 // (a warp scans every tile set: half the registers for accumulators, so more
-// CTAs fit on an SM; the bucket scan takes this form).
+// CTAs fit on an SM; the bucket scan takes this form). With ItemView::split an
+// item of one or two queries puts its four warps side by side on the tile sets,
+// one of three or four queries two: such an item is one warp's serial chain
+// otherwise (16 queries x 128 probes of 1.2M x 100, 100 kept: the three scans
+// 80 + 91 + 62 -> 36 + 30 + 37 us; one query, 10 kept: 26 + 25 + 26 -> 14 + 10 + 15 us).
 // WHOLE: every 256-group batch of the item's index is a whole number of
 // kBsPrefetch-group rings (nbg a multiple of kBsPrefetch); the ring loop then
 // runs without bounds checks.
 template <bool NIBBLE8, int QW = 4, bool WHOLE = false>
 __device__ __forceinline__ void scan_item(const ItemView& v, const ItemQueries& iq, unsigned char* smem) {
-  constexpr int kGroups = kItemQueries / QW;  // query groups per item
-  constexpr int kTsets = kBsWarps / kGroups;  // tile sets scanned side by side
   const int nbg = v.nbg, k = v.k, pc = v.pc;
+  // Query groups per item, tile sets scanned side by side.
+  const int groups = (QW == 2 && v.split && pc <= 4) ? (pc <= 2 ? 1 : 2) : kItemQueries / QW;
+  const int tsets = kBsWarps / groups;
   const int chunk = nbg < kFlushGroups ? nbg : kFlushGroups;
   const bool resident = chunk >= nbg;
 
@@ -1224,7 +1232,7 @@ __device__ __forceinline__ void scan_item(const ItemView& v, const ItemQueries& 
     __syncthreads();
   }
 
-  const int quad = warp % kGroups, tset = warp / kGroups;
+  const int quad = warp & (groups - 1), tset = warp / groups;
   const bool quad_ok = quad * QW < pc;
   const unsigned long long slot0 = static_cast<unsigned long long>(v.slot0);
   const int size = v.size;
@@ -1243,9 +1251,9 @@ __device__ __forceinline__ void scan_item(const ItemView& v, const ItemQueries& 
   const int k_rank = (k + j_rank - 1) / j_rank;  // rank among the 32 lane values
   constexpr long long kGroupStride = kTileWords / 2;  // uint2 per group row
 
-  const int rounds = (n_sub + kTsets - 1) / kTsets;
+  const int rounds = (n_sub + tsets - 1) / tsets;
   for (int r = 0; r < rounds; ++r) {
-    const int st = tset + kTsets * r;
+    const int st = tset + tsets * r;
     const bool active = quad_ok && st < n_sub;
     const long long sub = static_cast<long long>(slot0 / kBucketSlotAlign) + st;
     const long long tile = sub >> 1;
@@ -1532,7 +1540,7 @@ __device__ __forceinline__ void bucket_scan_item(const BucketScanArgs& a, const 
   __syncthreads();
   const ItemView v{a.codes, a.alpha, a.slot_ids, static_cast<long long>(a.slot_start[b]),
                    static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, pc, a.cand_score, a.cand_id,
-                   a.append_count};
+                   a.append_count, a.append_count && a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
   scan_item<NIBBLE8, kBsQueriesPerWarp, WHOLE>(v, iq, smem);
 }
 
@@ -1560,7 +1568,7 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5) bucket_scan_kernel(BucketSca
 }
 
 // launch_bucket_redo: probe by probe with the same item code, so at most k
-// entries per probe are appended and the region holds them all.
+// entries per probe and tile set are appended and the region holds them all.
 template <bool NIBBLE8, bool WHOLE>
 __global__ void __launch_bounds__(kBsWarps * 32, 5)
     bucket_redo_kernel(BucketScanArgs a, const uint32_t* probes, int probe_stride, const uint32_t* n_probe, int fixed_probe) {
@@ -1586,7 +1594,8 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5)
     }
     __syncthreads();
     const ItemView v{a.codes, a.alpha, a.slot_ids, static_cast<long long>(a.slot_start[b]),
-                     static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, 1, a.cand_score, a.cand_id, a.append_count};
+                     static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, 1, a.cand_score, a.cand_id, a.append_count,
+                     a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
     scan_item<NIBBLE8, kBsQueriesPerWarp, WHOLE>(v, iq, smem);
   }
 }

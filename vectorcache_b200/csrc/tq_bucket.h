@@ -193,6 +193,10 @@ cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStre
 // above the region's size, where the appends past its end are missing.
 constexpr int kOneHotItemQueries = 192;
 constexpr long long kOneHotPairsPerBucket = 16;
+// Up to this many (query, probe) pairs a pass has regions of four lists per probe,
+// which lets an item's warps split its tile sets (ItemView::split).
+constexpr long long kSplitPairs = 16384;
+constexpr int kSplitLists = 4;
 // Entries a region holds at least: what passes a floor of one bucket is no list of
 // k, and one query past its region costs a scan of all its probes by one CTA (1,893
 // queries x 27 probes of 84,838 x 119, k = 24, regions of 648: that kernel took 388

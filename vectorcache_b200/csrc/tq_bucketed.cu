@@ -488,9 +488,13 @@ struct tq_bucketed {
       });
       pa.enc_scores = sc.encs.as<float>();
       pa.enc_ld = nb;
-      const size_t lists = region_lists(static_cast<size_t>(max_probe), kscan);
-      sc.cand_s.reserve(m * lists * kscan * 4);
-      sc.cand_i.reserve(m * lists * kscan * 4);
+      const size_t probes = static_cast<size_t>(max_probe), split = vcb::kSplitPairs;
+      size_t lists = region_lists(probes, kscan);
+      if (m * probes <= split) lists = std::max(lists, vcb::kSplitLists * probes);
+      // The smaller passes of a scratch reserved for this one fit it too.
+      const size_t entries = std::max(m * lists, vcb::kSplitLists * std::min(m * probes, split)) * kscan;
+      sc.cand_s.reserve(entries * 4);
+      sc.cand_i.reserve(entries * 4);
       sc.floor.reserve(m * 4);
       const float* qf = sc.flat.qf.as<float>();
       vcb::BucketScanArgs ba{};
