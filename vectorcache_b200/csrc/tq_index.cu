@@ -33,6 +33,80 @@ bool& dry_run_flag() {
   return flag;
 }
 
+BlockCache& BlockCache::get() {
+  static BlockCache* cache = new BlockCache;  // outlives every index, static ones too
+  return *cache;
+}
+
+void* BlockCache::take(size_t bytes, size_t* capacity, int* device) {
+  check(cudaGetDevice(device), "cudaGetDevice");
+  // Whole 2 MiB pages, what cudaMalloc takes for a block of this size.
+  *capacity = bytes < kMinBlock ? bytes : round_up(bytes, size_t{2} << 20);
+  if (bytes >= kMinBlock) {
+    std::lock_guard<std::mutex> lock(mu_);
+    size_t best = blocks_.size();
+    for (size_t i = 0; i < blocks_.size(); ++i) {  // the smallest that fits, at most a quarter larger
+      const Block& b = blocks_[i];
+      if (b.device != *device || b.capacity < *capacity || b.capacity > *capacity + *capacity / 4) continue;
+      if (best == blocks_.size() || b.capacity < blocks_[best].capacity) best = i;
+    }
+    if (best < blocks_.size()) {
+      const Block b = blocks_[best];
+      blocks_.erase(blocks_.begin() + static_cast<std::ptrdiff_t>(best));
+      total_ -= b.capacity;
+      *capacity = b.capacity;
+      return b.ptr;
+    }
+  }
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, *capacity);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim();
+    *capacity = bytes;
+    e = cudaMalloc(&p, bytes);
+  }
+  check(e, "cudaMalloc");
+  return p;
+}
+
+void BlockCache::give(void* ptr, size_t capacity, int device) noexcept {
+  int prev = device;
+  const bool keep = capacity >= kMinBlock && capacity <= kLimit && cudaGetDevice(&prev) == cudaSuccess &&
+                    (prev == device || cudaSetDevice(device) == cudaSuccess);
+  bool kept = false;
+  if (keep && cudaDeviceSynchronize() == cudaSuccess) {
+    std::vector<void*> out;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      try {
+        blocks_.push_back({ptr, capacity, device});
+        total_ += capacity;
+        kept = true;
+        while (total_ > kLimit) {
+          out.push_back(blocks_.front().ptr);
+          total_ -= blocks_.front().capacity;
+          blocks_.erase(blocks_.begin());
+        }
+      } catch (...) {  // no host memory for the list: ptr is freed below
+      }
+    }
+    for (void* p : out) cudaFree(p);
+  }
+  if (!kept) cudaFree(ptr);
+  if (keep && prev != device) cudaSetDevice(prev);
+}
+
+void BlockCache::trim() noexcept {
+  std::vector<Block> blocks;
+  {
+    std::lock_guard<std::mutex> lock(mu_);
+    blocks.swap(blocks_);
+    total_ = 0;
+  }
+  for (const Block& b : blocks) cudaFree(b.ptr);
+}
+
 void calibrate_index(tq_index* h, const float* d_sample, size_t n, cudaStream_t s) {
   require(n >= 2, TQ_ERR_INVALID_ARGUMENT, "calibration needs at least 2 rows");
   require(!h->prepared && h->n == 0, TQ_ERR_STATE, "calibrate must precede prepare()");

@@ -486,6 +486,7 @@ struct tq_server {
     }
     slot_bytes = max_batch * (max_dim * 4 + max_k * 12);
     size_t free_b = 0, total_b = 0;
+    vcb::BlockCache::get().trim();  // what it holds counts as free
     vcb::check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
     resident_bytes = total_b - free_b;  // indexes, kernels, context and the slots' buffers
     // The largest scratch any admissible batch needs: full batches at the
