@@ -107,3 +107,49 @@ def test_bucketed_pass_equals_small_passes(dim, bits, n, k, n_probe, rerank_k):
     assert np.array_equal(mixed.ids[rows], whole.ids[rows])
     assert np.array_equal(mixed.scores[rows].view(np.uint32), whole.scores[rows].view(np.uint32))
     idx.close()
+
+
+@pytest.mark.parametrize("n,nq,k", [
+    (40_000, 1, 64),    # thousands of equal candidates: the merge's chunks
+    (200_000, 1, 10),   # 980 of them: its sort
+    (9_000, 1, 10),     # 50: no bound
+    (60_000, 2, 256),
+    (20_000, 70, 100),  # one-hot lists that every score enters
+])
+def test_zero_queries_return_the_lowest_ids(oracle, n, nq, k):
+    db = power_law(n, 8, seed=31)
+    q = np.zeros((nq, 8), np.float32)
+    idx = vcb.TurboQuantIndex(8, 4)
+    idx.add(db)
+    idx.prepare()
+    res = idx.search(q, k)
+    packed, alpha = oracle.encode(db, 4, None, None)
+    want_s, want_i = oracle.search_flat(q, 4, packed, alpha, k, None, None)
+    assert np.array_equal(res.ids, want_i)
+    assert np.array_equal(res.scores.view(np.uint32), want_s.view(np.uint32))
+    idx.close()
+
+
+def test_indexes_built_and_closed_by_several_threads():
+    # Closed indexes' device blocks serve the next ones, across threads and streams.
+    from concurrent.futures import ThreadPoolExecutor
+
+    shapes = [(30_000, 64, 4, 5, 10), (50_000, 128, 3, 70, 10), (20_000, 256, 2, 3, 40)]
+
+    def one(i):
+        n, dim, bits, nq, k = shapes[i % 3]
+        db, q = power_law(n, dim, seed=50 + i % 3), power_law(nq, dim, seed=60 + i % 3)
+        idx = vcb.TurboQuantIndex(dim, bits)
+        idx.calibrate(db[:2000])
+        idx.add(db)
+        idx.prepare()
+        res = idx.search(q, k)
+        idx.close()
+        return res.ids, res.scores
+
+    want = [one(i) for i in range(3)]
+    with ThreadPoolExecutor(4) as pool:
+        got = list(pool.map(one, range(12)))
+    for i, (ids, scores) in enumerate(got):
+        assert np.array_equal(ids, want[i % 3][0]), i
+        assert np.array_equal(scores.view(np.uint32), want[i % 3][1].view(np.uint32)), i
