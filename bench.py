@@ -668,7 +668,13 @@ def run_ours(args, world, rank, local):
                                     "peak": peak, "frac": encode_bytes / (encode_kernels_ms / 1e3) / 1e9 / peak},
                 "latency_ms": latency,
             },
-            "roofline": {"kernel": "scan_kernel", "bound": "hbm", "achieved": achieved, "peak": peak,
+            # bound: batches above 64 queries run on the tensor pipe (u8 one-hot contraction,
+            # 32 columns per byte group, 16 for 3-bit codes); achieved/frac are the code stream's.
+            "roofline": {"kernel": "onehot_scan_kernel" if args.nq > 64 else "scan_kernel",
+                         "bound": "tensor" if args.nq > 64 else "hbm",
+                         "tensor_ops_per_s": 2.0 * args.n * args.nq * nbg * (16 if args.bits == 3 else 32)
+                         * args.steps / (prof["scan_ms"] / 1e3) if args.nq > 64 and prof["scan_ms"] else None,
+                         "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": tr,
                          "bytes_per_launch": bytes_per_launch, "ms_per_launch": scan_ms_avg,
                          "share_of_kernel_time": prof["scan_ms"] / total_kernel_ms if total_kernel_ms else None,
