@@ -75,7 +75,9 @@ void BlockCache::give(void* ptr, size_t capacity, int device) noexcept {
   const bool keep = capacity >= kMinBlock && capacity <= kLimit && cudaGetDevice(&prev) == cudaSuccess &&
                     (prev == device || cudaSetDevice(device) == cudaSuccess);
   bool kept = false;
-  if (keep && cudaDeviceSynchronize() == cudaSuccess) {
+  const bool idle = keep && cudaDeviceSynchronize() == cudaSuccess;
+  if (keep && !idle) cudaGetLastError();  // not the next launch's error
+  if (idle) {
     std::vector<void*> out;
     {
       std::lock_guard<std::mutex> lock(mu_);

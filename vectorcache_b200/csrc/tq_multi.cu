@@ -334,7 +334,7 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
         h->ctas = h->sms * std::min(best_c, ps);
       };
       set_direct(0, best_rv);
-      double best = h->time_ms(1);
+      double best = h->time_ms(3);
       size_t best_d = 0;
       long long best_d_rv = best_rv;
       // The range length above suits all batches; what is left of them may be a few
@@ -350,7 +350,7 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
         for (long long rv : {best_rv, kShortRange}) {
           set_direct(d, rv);
           h->time_ms(1);
-          const double ms = h->time_ms(1);
+          const double ms = h->time_ms(3);  // candidates differ by less than single runs do
           h->tuned_ms.push_back(ms);
           if (ms < best) {
             best = ms;
