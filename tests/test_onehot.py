@@ -153,3 +153,32 @@ def test_indexes_built_and_closed_by_several_threads():
     for i, (ids, scores) in enumerate(got):
         assert np.array_equal(ids, want[i % 3][0]), i
         assert np.array_equal(scores.view(np.uint32), want[i % 3][1].view(np.uint32)), i
+
+
+@pytest.mark.parametrize("n_probe,k", [(9, 10), (10, 10), (10, 1), (14, 64)])
+def test_lookup_step_after_a_onehot_step(n_probe, k):
+    # Probes 1..7 have at least 16 pairs per bucket and the last step has not: it
+    # appends to regions that the one-hot step may have filled. A zero query scores
+    # every vector of seven buckets at its floor, more than the 4096 entries of its
+    # region; its neighbours' regions, and the memory behind the last query's, have
+    # to stay as they are.
+    n, dim = 60000, 32
+    db = vmf_mixture(n, dim, seed=23, clusters=60)
+    idx = vcb.BucketedTurboQuantIndex(dim, 4, vcb.BucketParams(
+        n_probe=8, max_bucket_size=4000, energy_soft=2000, kmeans_iters=3, seed=7))
+    idx.add(db)
+    idx.prepare()
+    nb = idx.info()["n_buckets"]
+    sizes = idx.layout()["bucket_size"]
+    assert sizes[1:8].sum() > 4096  # a zero query's first probes: equal scores, lowest ids
+    nq = 5 * nb // 2
+    assert 7 * nq >= 16 * nb > (n_probe - 8) * nq
+    q = np.random.default_rng(24).standard_normal((nq, dim)).astype(np.float32)
+    q[::3] = 0.0
+    q[-1] = 0.0
+    whole = idx.search(q, k, n_probe=n_probe)
+    for s in range(0, nq, nb):  # 7 nb pairs: every step on the lookup scan
+        part = idx.search(q[s:s + nb], k, n_probe=n_probe)
+        assert np.array_equal(whole.ids[s:s + nb], part.ids), s
+        assert np.array_equal(whole.scores[s:s + nb].view(np.uint32), part.scores.view(np.uint32)), s
+    idx.close()

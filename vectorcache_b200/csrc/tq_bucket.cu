@@ -1168,8 +1168,10 @@ struct ItemView {
   // nullptr: each (query, tile set) writes its own list of k entries at
   // ItemQueries::list, -inf padded. Otherwise ItemQueries::list is the start
   // (in lists of k) of the query's candidate region and the kept candidates
-  // are appended there at append_count[query] (atomically), unpadded.
+  // are appended there at append_count[query] (atomically), unpadded; the region
+  // holds `region` entries, and what comes past its end is counted but not written.
   uint32_t* append_count = nullptr;
+  long long region = 0;
   // Appending, QW = 2: the warps that an item of at most four queries leaves idle
   // take tile sets of its own (up to kBsWarps lists of k per query).
   bool split = false;
@@ -1489,7 +1491,11 @@ __device__ __forceinline__ void scan_item(const ItemView& v, const ItemQueries& 
       if (lane == 0) at = atomicAdd(v.append_count + iq.q[quad * QW + q], static_cast<unsigned>(c));
       at = __shfl_sync(full_mask(), at, 0);
       const long long base = iq.list[quad * QW + q] * k + at;
-      for (int t = lane; t < c; t += kWarp) {
+      // A one-hot step before this one may have filled the region (it appends every
+      // score above the floor, not k a probe): nothing is written past its end, the
+      // count says so and the query is scanned again (launch_bucket_redo).
+      const int room = static_cast<int>(min(static_cast<long long>(c), max(0ll, v.region - at)));
+      for (int t = lane; t < room; t += kWarp) {
         v.cand_s[base + t] = list_s[q * kmax + t];
         v.cand_i[base + t] = list_i[q * kmax + t];
       }
@@ -1540,7 +1546,7 @@ __device__ __forceinline__ void bucket_scan_item(const BucketScanArgs& a, const 
   __syncthreads();
   const ItemView v{a.codes, a.alpha, a.slot_ids, static_cast<long long>(a.slot_start[b]),
                    static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, pc, a.cand_score, a.cand_id,
-                   a.append_count, a.append_count && a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
+                   a.append_count, a.lists * a.k, a.append_count && a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
   scan_item<NIBBLE8, kBsQueriesPerWarp, WHOLE>(v, iq, smem);
 }
 
@@ -1567,8 +1573,8 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5) bucket_scan_kernel(BucketSca
   }
 }
 
-// launch_bucket_redo: probe by probe with the same item code, so at most k
-// entries per probe and tile set are appended and the region holds them all.
+// launch_bucket_redo: probe by probe with the same item code, from an empty region,
+// so at most k entries per probe and tile set are appended and the region holds them all.
 template <bool NIBBLE8, bool WHOLE>
 __global__ void __launch_bounds__(kBsWarps * 32, 5)
     bucket_redo_kernel(BucketScanArgs a, const uint32_t* probes, int probe_stride, const uint32_t* n_probe, int fixed_probe) {
@@ -1595,7 +1601,7 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5)
     __syncthreads();
     const ItemView v{a.codes, a.alpha, a.slot_ids, static_cast<long long>(a.slot_start[b]),
                      static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, 1, a.cand_score, a.cand_id, a.append_count,
-                     a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
+                     a.lists * a.k, a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
     scan_item<NIBBLE8, kBsQueriesPerWarp, WHOLE>(v, iq, smem);
   }
 }

@@ -180,8 +180,12 @@ struct BucketScanArgs {
   // Optional per query (zeroed by the caller): the kept candidates of query q
   // are appended, unpadded, to its region of `lists` lists of k entries (at least
   // max_probe * kBsListsPerProbe) at cand_score/cand_id + q * lists * k, and
-  // append_count[q] counts them. nullptr: one -inf padded list of k per (query,
-  // probe, tile set).
+  // append_count[q] counts them. No scan writes past a region's end; a count above
+  // the region's size says that appends are missing there. Steps of this scan alone
+  // append at most k entries per probe and tile set, which fit; after a one-hot step
+  // (launch_onehot_buckets, every score at or above the floor) either kind of step may
+  // pass the end, and launch_bucket_redo has to follow. nullptr: one -inf padded list
+  // of k per (query, probe, tile set).
   uint32_t* append_count = nullptr;
   long long lists = 0;
 };
@@ -190,7 +194,7 @@ cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStre
 // The same items (PairArgs::item_queries = kOneHotItemQueries, even_items) on the
 // tensor cores (tq_onehot.cu): every score at or above its query's floor is
 // appended to the query's region, without the lists of k; append_count may end
-// above the region's size, where the appends past its end are missing.
+// above the region's size, here or in a later step of launch_bucket_scan.
 constexpr int kOneHotItemQueries = 192;
 constexpr long long kOneHotPairsPerBucket = 16;
 // Up to this many (query, probe) pairs a pass has regions of four lists per probe,
