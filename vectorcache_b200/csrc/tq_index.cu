@@ -70,12 +70,22 @@ void* BlockCache::take(size_t bytes, size_t* capacity, int* device) {
   return p;
 }
 
+// Waits for the current device's queued work the way freeing a block does. Not
+// cudaDeviceSynchronize: CUDA refuses that while any stream is being captured, and
+// ends the capture with an error, whichever thread it runs on; cudaFree is refused by a
+// global-mode capture only. That a free waits was measured with 256 bytes, 512 KiB and
+// 8 MiB behind 1.7 s of queued products.
+static bool wait_for_device() {
+  void* p = nullptr;
+  return cudaMalloc(&p, 256) == cudaSuccess && cudaFree(p) == cudaSuccess;
+}
+
 void BlockCache::give(void* ptr, size_t capacity, int device) noexcept {
   int prev = device;
   const bool keep = capacity >= kMinBlock && capacity <= kLimit && cudaGetDevice(&prev) == cudaSuccess &&
                     (prev == device || cudaSetDevice(device) == cudaSuccess);
   bool kept = false;
-  const bool idle = keep && cudaDeviceSynchronize() == cudaSuccess;
+  const bool idle = keep && wait_for_device();
   if (keep && !idle) cudaGetLastError();  // not the next launch's error
   if (idle) {
     std::vector<void*> out;

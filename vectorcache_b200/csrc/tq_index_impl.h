@@ -69,7 +69,7 @@ struct ScratchArena {
 // allocations on the same device: cudaMalloc and cudaFree of 1 MiB or more take
 // about 0.33 ms each, whatever the size, and a new index with its first search makes
 // ten (262,144 x 1536, create to close around a first search: 8.9 -> 3.05 ms). A block is
-// given back idle (the device is synchronized first, as cudaFree does), so that any
+// given back idle (the device's work is waited for first, as cudaFree does), so that any
 // stream and thread may take it. At most kLimit bytes per process stay, the oldest
 // go first; all go when cudaMalloc fails or trim() asks.
 class BlockCache {
