@@ -1573,22 +1573,35 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5) bucket_scan_kernel(BucketSca
   }
 }
 
-// launch_bucket_redo: probe by probe with the same item code, from an empty region,
-// so at most k entries per probe and tile set are appended and the region holds them all.
+// launch_bucket_redo, first: the queries whose count passed their region, their
+// counts back to zero. redo: how many, then which.
+__global__ void overflow_list_kernel(uint32_t* __restrict__ append_count, long long nq, long long region,
+                                     uint32_t* __restrict__ redo) {
+  const long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (q >= nq || append_count[q] <= region) return;
+  append_count[q] = 0u;
+  redo[1 + atomicAdd(redo, 1u)] = static_cast<uint32_t>(q);
+}
+
+// Then their probes, one item each over the whole grid, with the lookup scan's item
+// code: from an empty region, so at most k entries per probe and tile set are appended
+// and the region holds them all. (One CTA per query took its probes one by one, and a
+// single such query cost 1 ms of 256 probes, 2 ms of 464: 512 queries x 256 probes of
+// 300k x 64 3-bit 1625 us.)
 template <bool NIBBLE8, bool WHOLE>
 __global__ void __launch_bounds__(kBsWarps * 32, 5)
-    bucket_redo_kernel(BucketScanArgs a, const uint32_t* probes, int probe_stride, const uint32_t* n_probe, int fixed_probe) {
+    bucket_redo_kernel(BucketScanArgs a, const uint32_t* redo, const uint32_t* probes, int probe_stride,
+                       const uint32_t* n_probe, int fixed_probe) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ ItemQueries iq;
-  const int q = static_cast<int>(blockIdx.x);
-  if (a.append_count[q] <= a.lists * a.k) return;  // the whole CTA
-  __syncthreads();
-  if (threadIdx.x == 0) a.append_count[q] = 0u;
-  const int np = n_probe ? min(static_cast<int>(n_probe[q]), a.max_probe) : fixed_probe;
-  for (int j = 0; j < np; ++j) {
+  const long long items = static_cast<long long>(redo[0]) * a.max_probe;
+  for (long long it = blockIdx.x; it < items; it += gridDim.x) {
+    const int q = static_cast<int>(redo[1 + it / a.max_probe]), j = static_cast<int>(it % a.max_probe);
+    const int np = n_probe ? min(static_cast<int>(n_probe[q]), a.max_probe) : fixed_probe;
+    if (j >= np) continue;  // the whole CTA
     const uint32_t b = probes[static_cast<long long>(q) * probe_stride + j];
     if (b == 0xffffffffu) continue;
-    __syncthreads();  // the previous probe is done with iq and the LUT area
+    __syncthreads();  // the previous item is done with iq and the LUT area
     if (threadIdx.x < kItemQueries) {
       const int t = threadIdx.x;
       iq.q[t] = t == 0 ? q : -1;
@@ -1991,17 +2004,23 @@ static size_t bucket_scan_smem(int nbg, int k) {
          static_cast<size_t>(kBsWarps) * (static_cast<size_t>(kBsQueriesPerWarp) * kmax_of(k) * 8 + kBsBuf * 8);
 }
 
-cudaError_t launch_bucket_redo(const BucketScanArgs& a, long long nq, const uint32_t* probes, int probe_stride,
-                               const uint32_t* n_probe, int fixed_probe, cudaStream_t stream) {
+cudaError_t launch_bucket_redo(const BucketScanArgs& a, long long nq, uint32_t* redo, const uint32_t* probes,
+                               int probe_stride, const uint32_t* n_probe, int fixed_probe, int sms,
+                               cudaStream_t stream) {
   if (nq <= 0) return cudaSuccess;
-  if (a.k < 1 || a.k > kMaxK || !a.append_count) return cudaErrorInvalidValue;
+  if (a.k < 1 || a.k > kMaxK || !a.append_count || !redo) return cudaErrorInvalidValue;
+  overflow_list_kernel<<<static_cast<unsigned>((nq + 255) / 256), 256, 0, stream>>>(a.append_count, nq, a.lists * a.k,
+                                                                                    redo);
   const size_t smem = bucket_scan_smem(a.nbg, a.k);
   const bool whole = a.nbg % kBsPrefetch == 0;
   auto kern = a.bits == 3 ? (whole ? bucket_redo_kernel<true, true> : bucket_redo_kernel<true, false>)
                           : (whole ? bucket_redo_kernel<false, true> : bucket_redo_kernel<false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  kern<<<static_cast<unsigned>(nq), kBsWarps * 32, smem, stream>>>(a, probes, probe_stride, n_probe, fixed_probe);
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (e != cudaSuccess) return e;
+  const long long grid = std::min<long long>(nq * a.max_probe, 5ll * sms);  // as many as its registers let reside
+  kern<<<static_cast<unsigned>(grid), kBsWarps * 32, smem, stream>>>(a, redo, probes, probe_stride, n_probe, fixed_probe);
   return cudaGetLastError();
 }
 

@@ -202,9 +202,8 @@ constexpr long long kOneHotPairsPerBucket = 16;
 constexpr long long kSplitPairs = 16384;
 constexpr int kSplitLists = 4;
 // Entries a region holds at least: what passes a floor of one bucket is no list of
-// k, and one query past its region costs a scan of all its probes by one CTA (1,893
-// queries x 27 probes of 84,838 x 119, k = 24, regions of 648: that kernel took 388
-// of 876 us).
+// k, and a query past its region is scanned twice (1,893 queries x 27 probes of
+// 84,838 x 119, k = 24: 876 us with regions of 648, 503 with these).
 constexpr long long kOneHotMinRegion = 4096;
 // Its 32-bit offsets: slots, and bytes of the pass's LUTs (16,384 queries of 16,384
 // 4-bit dims are just too many); a pass that does not fit keeps launch_bucket_scan.
@@ -214,10 +213,11 @@ constexpr bool onehot_buckets_fit(long long nq, long long n_slots, int nbg) {
 cudaError_t launch_onehot_buckets(const BucketScanArgs& a, long long nq, long long n_slots, int sms, unsigned* status,
                                   cudaStream_t stream);
 // Scans again, list by list, every query whose append_count passed its region:
-// all its probes (n_probe[q], or fixed_probe), from an empty region. One CTA per
-// query; the others return at once.
-cudaError_t launch_bucket_redo(const BucketScanArgs& a, long long nq, const uint32_t* probes, int probe_stride,
-                               const uint32_t* n_probe, int fixed_probe, cudaStream_t stream);
+// all its probes (n_probe[q], or fixed_probe), from an empty region. redo: nq + 1
+// words, the first one zeroed by the caller.
+cudaError_t launch_bucket_redo(const BucketScanArgs& a, long long nq, uint32_t* redo, const uint32_t* probes,
+                               int probe_stride, const uint32_t* n_probe, int fixed_probe, int sms,
+                               cudaStream_t stream);
 // floor[q] = the k-th largest score (above -inf) among the first count[q]
 // (count null: all `stride`) candidates of query q's region (cand + q * stride), -inf when there are
 // fewer than k: the k-th score of their merged top k, a lower bound of the

@@ -519,8 +519,9 @@ struct tq_bucketed {
       ba.cand_id = sc.cand_i.as<uint32_t>();
       // Every (query, probe, tile set) appends its kept candidates to the
       // query's region; the merges read exactly those.
-      sc.acount.reserve(m * 4);
-      if (!vcb::dry_run_flag()) vcb::check(cudaMemsetAsync(sc.acount.get(), 0, m * 4, s), "cudaMemsetAsync");
+      // Behind the counts: the queries to scan again (launch_bucket_redo).
+      sc.acount.reserve((2 * m + 1) * 4);
+      if (!vcb::dry_run_flag()) vcb::check(cudaMemsetAsync(sc.acount.get(), 0, (m + 1) * 4, s), "cudaMemsetAsync");
       ba.append_count = sc.acount.as<uint32_t>();
       ba.lists = static_cast<long long>(lists);
       // The best-routed buckets first: the k-th best score over a query's
@@ -608,7 +609,8 @@ struct tq_bucketed {
       scan("bucket scan kernel", last_items);
       if (any_onehot) {
         eng->launch(tq_index::kScan, s, "bucket redo kernel", [&] {
-          return vcb::launch_bucket_redo(ba, static_cast<long long>(m), pa.probes, ptop, np_pass, max_probe, s);
+          return vcb::launch_bucket_redo(ba, static_cast<long long>(m), ba.append_count + m, pa.probes, ptop, np_pass,
+                                         max_probe, eng->sms, s);
         });
       }
       vcb::MergeArgs mg{};
