@@ -182,3 +182,24 @@ def test_lookup_step_after_a_onehot_step(n_probe, k):
         assert np.array_equal(whole.ids[s:s + nb], part.ids), s
         assert np.array_equal(whole.scores[s:s + nb].view(np.uint32), part.scores.view(np.uint32)), s
     idx.close()
+
+
+@pytest.mark.parametrize("nb_queries,many", [(4, 4), (4, 1), (16, 1)])
+def test_probe_counts_per_query_decide_by_their_pairs(nb_queries, many):
+    # One query in `many` has 40 probes, the others 9: the steps' bounds allow the
+    # one-hot scan, their pairs do for some steps only (few pairs: the lookup scan).
+    idx = vcb.BucketedTurboQuantIndex(64, 4, vcb.BucketParams(
+        n_probe=8, max_bucket_size=300, energy_soft=150, kmeans_iters=3, seed=7))
+    idx.add(vmf_mixture(12000, 64, seed=25, clusters=60))
+    idx.prepare()
+    nb = idx.info()["n_buckets"]
+    nq = nb_queries * nb
+    q = np.random.default_rng(26).standard_normal((nq, 64)).astype(np.float32)
+    counts = np.where(np.arange(nq) % many == 0, 40, 9).astype(np.uint32)
+    whole = idx.search(q, 10, n_probe=40, n_probe_per_query=counts)
+    step = nb // 4
+    for s in range(0, nq, step):
+        part = idx.search(q[s:s + step], 10, n_probe=40, n_probe_per_query=counts[s:s + step])
+        assert np.array_equal(whole.ids[s:s + step], part.ids), s
+        assert np.array_equal(whole.scores[s:s + step].view(np.uint32), part.scores.view(np.uint32)), s
+    idx.close()

@@ -588,17 +588,41 @@ __global__ void label_hist_kernel(const uint32_t* __restrict__ label, long long 
   if (i < n) atomicAdd(&counts[label[i]], 1u);
 }
 
+// Sum of a value over the CTA's 1024 threads, in every thread; s_sum: 32 words.
+__device__ __forceinline__ unsigned long long cta_sum_1024(unsigned long long v, unsigned long long* s_sum) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(full_mask(), v, o);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = s_sum[threadIdx.x & 31];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(full_mask(), v, o);
+  __syncthreads();
+  return v;
+}
+
 // Exclusive prefix sums of counts (and of ceil(counts / div) when div > 0) in
-// one CTA; out[nb] = total.
+// one CTA; out[nb] = total. With n_onehot, a total of at least onehot_from takes
+// kOneHotItemQueries for div, and its quotients' total goes to *n_onehot instead of
+// *total_div; the other of the two is 0.
 __global__ void __launch_bounds__(1024) prefix_kernel(const uint32_t* __restrict__ counts, int nb,
                                                       unsigned long long* __restrict__ out, int div,
                                                       unsigned long long* __restrict__ out_div,
-                                                      unsigned long long* __restrict__ total_div) {
+                                                      unsigned long long* __restrict__ total_div,
+                                                      unsigned long long* __restrict__ n_onehot = nullptr,
+                                                      long long onehot_from = 0) {
   __shared__ unsigned long long s_warp[2][32];
   __shared__ unsigned long long s_carry[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < 2) s_carry[threadIdx.x] = 0ull;
   __syncthreads();
+  bool onehot = false;
+  if (n_onehot) {
+    unsigned long long sum = 0ull;
+    for (int i = threadIdx.x; i < nb; i += 1024) sum += counts[i];
+    onehot = cta_sum_1024(sum, s_warp[0]) >= static_cast<unsigned long long>(onehot_from);
+    if (onehot) div = kOneHotItemQueries;
+  }
   for (int base = 0; base < nb; base += 1024) {
     const int i = base + threadIdx.x;
     const unsigned long long c = i < nb ? counts[i] : 0ull;
@@ -639,7 +663,8 @@ __global__ void __launch_bounds__(1024) prefix_kernel(const uint32_t* __restrict
     out[nb] = s_carry[0];
     if (div > 0) {
       out_div[nb] = s_carry[1];
-      if (total_div) *total_div = s_carry[1];
+      if (total_div) *total_div = onehot ? 0ull : s_carry[1];
+      if (n_onehot) *n_onehot = onehot ? s_carry[1] : 0ull;
     }
   }
 }
@@ -1012,10 +1037,10 @@ __global__ void pair_scatter_kernel(PairArgs a, int begin, int window) {
 }
 
 // Bucket b's work items: its c pairs from `first` on, numbered from item i0.
-__device__ __forceinline__ void write_items(const PairArgs& a, int b, unsigned long long c, unsigned long long first,
-                                            unsigned long long i0) {
-  unsigned long long per = static_cast<unsigned long long>(a.item_queries);
-  if (a.even_items && c > per) {
+__device__ __forceinline__ void write_items(const PairArgs& a, bool onehot, int b, unsigned long long c,
+                                            unsigned long long first, unsigned long long i0) {
+  unsigned long long per = static_cast<unsigned long long>(onehot ? kOneHotItemQueries : kItemQueries);
+  if (onehot && c > per) {  // evenly
     const unsigned long long parts = (c + per - 1) / per;
     per = (c + parts - 1) / parts;
   }
@@ -1028,7 +1053,9 @@ __device__ __forceinline__ void write_items(const PairArgs& a, int b, unsigned l
 __global__ void item_build_kernel(PairArgs a) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= a.nb) return;
-  write_items(a, b, a.pair_start[b + 1] - a.pair_start[b], a.pair_start[b], a.item_start[b]);
+  const bool onehot = a.n_onehot ? *a.n_onehot > 0ull : a.onehot;
+  if (b == 0) *a.next_item = 0ull;
+  write_items(a, onehot, b, a.pair_start[b + 1] - a.pair_start[b], a.pair_start[b], a.item_start[b]);
 }
 
 // The whole grouping in one CTA for few pairs, counts and fills in shared memory:
@@ -1041,6 +1068,7 @@ __global__ void __launch_bounds__(kSmallPairThreads) pair_small_kernel(PairArgs 
   extern __shared__ uint32_t s_count[];  // nb counts, then the next free place of each bucket
   __shared__ uint32_t s_warp[2][32];
   __shared__ uint32_t s_base[2];
+  __shared__ unsigned long long s_sum[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int b = threadIdx.x; b < a.nb; b += kSmallPairThreads) s_count[b] = 0u;
   if (threadIdx.x < 2) s_base[threadIdx.x] = 0u;
@@ -1055,10 +1083,17 @@ __global__ void __launch_bounds__(kSmallPairThreads) pair_small_kernel(PairArgs 
     if (b < static_cast<uint32_t>(a.nb)) atomicAdd(&s_count[b], 1u);
   }
   __syncthreads();
+  bool onehot = a.onehot;
+  if (a.n_onehot) {
+    unsigned long long sum = 0ull;
+    for (int b = threadIdx.x; b < a.nb; b += kSmallPairThreads) sum += s_count[b];
+    onehot = cta_sum_1024(sum, s_sum) >= static_cast<unsigned long long>(a.onehot_from);
+  }
+  const uint32_t item_queries = onehot ? kOneHotItemQueries : kItemQueries;
   for (int b0 = 0; b0 < a.nb; b0 += kSmallPairThreads) {
     const int b = b0 + static_cast<int>(threadIdx.x);
     const uint32_t c = b < a.nb ? s_count[b] : 0u;
-    const uint32_t n = (c + a.item_queries - 1) / a.item_queries;
+    const uint32_t n = (c + item_queries - 1) / item_queries;
     uint32_t ic = c, in = n;  // inclusive sums over the warp
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1088,7 +1123,7 @@ __global__ void __launch_bounds__(kSmallPairThreads) pair_small_kernel(PairArgs 
     if (b < a.nb) {
       a.pair_start[b] = first;
       a.item_start[b] = item;
-      write_items(a, b, c, first, item);
+      write_items(a, onehot, b, c, first, item);
       s_count[b] = first;
     }
     __syncthreads();
@@ -1098,7 +1133,9 @@ __global__ void __launch_bounds__(kSmallPairThreads) pair_small_kernel(PairArgs 
   if (threadIdx.x == 0) {
     a.pair_start[a.nb] = s_base[0];
     a.item_start[a.nb] = s_base[1];
-    *a.n_items = s_base[1];
+    *a.n_items = a.n_onehot && onehot ? 0ull : s_base[1];
+    if (a.n_onehot) *a.n_onehot = onehot ? s_base[1] : 0ull;
+    *a.next_item = 0ull;
   }
   for (long long t = threadIdx.x; t < total; t += kSmallPairThreads) {
     long long q;
@@ -1874,7 +1911,8 @@ cudaError_t launch_build_pairs(const PairArgs& a, cudaStream_t stream) {
     pair_count_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a, begin, window);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  prefix_kernel<<<1, 1024, 0, stream>>>(a.counts, a.nb, a.pair_start, a.item_queries, a.item_start, a.n_items);
+  prefix_kernel<<<1, 1024, 0, stream>>>(a.counts, a.nb, a.pair_start, a.onehot ? kOneHotItemQueries : kItemQueries,
+                                        a.item_start, a.n_items, a.n_onehot, a.onehot_from);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (total > 0) {
     pair_scatter_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(a, begin, window);
@@ -2058,7 +2096,6 @@ cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStre
     cache[0] = Resident{device, smem, reinterpret_cast<const void*>(kern), std::max(1, per_sm) * sms};
     hit = &cache[0];
   }
-  if ((e = cudaMemsetAsync(a.next_item, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
   const long long ctas = std::min<long long>(grid, hit->ctas);
   kern<<<static_cast<unsigned>(ctas), kBsWarps * 32, smem, stream>>>(a);
   return cudaGetLastError();

@@ -140,6 +140,7 @@ struct PairArgs {
   float* offsets;            // nq * max_probe: <q_hat, enc[probe]>
   uint4* items;              // (bucket, first pair, pair count, 0)
   unsigned long long* n_items;
+  unsigned long long* next_item;  // the scan's work counter, zeroed here
   // Probe positions [probe_begin, probe_end) of each query get pairs (the
   // search scans its first probes before the rest).
   int probe_begin = 0;
@@ -149,9 +150,14 @@ struct PairArgs {
   // probes, else kFloorProbes (at most its n_probe).
   int first_split = 0;
   int wide_from = kFloorWideFrom;
-  // Queries per work item; even_items: a bucket's pairs split evenly.
-  int item_queries = kItemQueries;
-  bool even_items = false;
+  // The items are for the one-hot scan: up to kOneHotItemQueries queries, a bucket's
+  // pairs split evenly (otherwise kItemQueries each, for launch_bucket_scan).
+  bool onehot = false;
+  // Set: the device decides by the pairs it counts, from onehot_from on the one-hot
+  // scan. The item count goes to n_items or to n_onehot, the other is 0, and both
+  // scans are launched; the one without items returns at once.
+  unsigned long long* n_onehot = nullptr;
+  long long onehot_from = 0;
 };
 // Groups the (query, probe) pairs by bucket and builds the scan work items.
 cudaError_t launch_build_pairs(const PairArgs& a, cudaStream_t stream);
@@ -170,7 +176,7 @@ struct BucketScanArgs {
   const float* offsets;
   const uint4* items;
   const unsigned long long* n_items;
-  unsigned long long* next_item;  // work counter (zeroed by launch_bucket_scan)
+  unsigned long long* next_item;  // work counter (zeroed by launch_build_pairs)
   int nbg, bits, k, max_probe;
   float* cand_score;         // (nq * max_probe * kBsListsPerProbe) lists of k, appending: nq * lists
   uint32_t* cand_id;
@@ -196,7 +202,18 @@ cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStre
 // appended to the query's region, without the lists of k; append_count may end
 // above the region's size, here or in a later step of launch_bucket_scan.
 constexpr int kOneHotItemQueries = 192;
+// Pairs per bucket from which a step runs there (fewer fill few of a tile's 32 or more
+// columns). Whole searches, lookups / here, at 12, 16 and 24 pairs per bucket in the far
+// step: 128 probes of 1.2M x 100 4-bit 894 / 829, 1040 / 881, 1317 / 971 us; 464 probes
+// of it 680 / 735, 773 / 765, 942 / 827; 256 probes of 400k x 192 2-bit 280 / 304,
+// 333 / 336, 393 / 362; 256 probes of 300k x 64 3-bit 180 / 216, 202 / 224, 228 / 238.
 constexpr long long kOneHotPairsPerBucket = 16;
+// The same where the device counts the pairs, in steps whose bound passed the line above:
+// they are uneven there, many in the buckets that most queries reach. 1.2M x 100, one
+// query in five with 464 probes, the others with 8, counted line at 16, 10 and 6:
+// 10,000 queries 3980, 3881, 3872 us, 256 queries 690, 690, 815; learned counts
+// (coverage 0.3, 2,048 queries) 1973, 1828, 1828.
+constexpr long long kOneHotPairsCounted = 10;
 // Up to this many (query, probe) pairs a pass has regions of four lists per probe,
 // which lets an item's warps split its tile sets (ItemView::split).
 constexpr long long kSplitPairs = 16384;

@@ -462,7 +462,7 @@ struct tq_bucketed {
       sc.pairs.reserve(m * max_probe * 4);
       sc.off.reserve(m * max_probe * 4);
       sc.items.reserve(static_cast<size_t>(items) * 16);
-      sc.nitems.reserve(16);  // item count, then the scan's work counter
+      sc.nitems.reserve(24);  // item count, the scan's work counter, items for the one-hot scan
       vcb::PairArgs pa{};
       pa.probes = sc.top_i.as<uint32_t>();
       pa.probe_stride = ptop;
@@ -479,6 +479,7 @@ struct tq_bucketed {
       pa.offsets = sc.off.as<float>();
       pa.items = sc.items.as<uint4>();
       pa.n_items = sc.nitems.as<unsigned long long>();
+      pa.next_item = pa.n_items + 1;
       // Offsets <q_hat, encode_c> of every probed bucket: one q_hat . enc^T
       // product per pass, gathered per pair.
       sc.encs.reserve(m * nb * 4);
@@ -510,7 +511,7 @@ struct tq_bucketed {
       ba.offsets = pa.offsets;
       ba.items = pa.items;
       ba.n_items = pa.n_items;
-      ba.next_item = pa.n_items + 1;
+      ba.next_item = pa.next_item;
       ba.nbg = static_cast<int>(nbg);
       ba.bits = static_cast<int>(bits);
       ba.k = static_cast<int>(kscan);
@@ -536,24 +537,31 @@ struct tq_bucketed {
       const int first =
           std::min(max_probe >= pa.wide_from ? vcb::kFloorProbesWide : vcb::kFloorProbes, max_probe);
       const bool two_phase = max_probe > vcb::kFloorProbes;
-      // Above a floor, steps with enough pairs per bucket go to the tensor cores.
-      bool any_onehot = false, onehot = false;
+      // Above a floor, steps with enough pairs per bucket go to the tensor cores. With
+      // one probe count for all queries step_pairs is what they have; with counts per
+      // query (given or learned) it is a bound, and the device decides by the pairs that
+      // it counts, both scans being launched.
+      bool any_onehot = false, ask = false;
       auto use_onehot = [&](long long step_pairs) {
-        onehot = ba.floor && step_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2 &&
-                 vcb::onehot_buckets_fit(static_cast<long long>(m), static_cast<long long>(n_slots), ba.nbg);
-        pa.item_queries = onehot ? vcb::kOneHotItemQueries : vcb::kItemQueries;
-        pa.even_items = onehot;
-        any_onehot |= onehot;
+        pa.onehot_from = vcb::kOneHotPairsCounted * nb;
+        const bool may = ba.floor && step_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2 &&
+                         vcb::onehot_buckets_fit(static_cast<long long>(m), static_cast<long long>(n_slots), ba.nbg);
+        ask = may && np_pass != nullptr;
+        pa.onehot = may && !ask;
+        pa.n_onehot = ask ? pa.n_items + 2 : nullptr;
+        any_onehot |= may;
       };
       auto scan = [&](const char* what, long long grid) {
-        if (!onehot) {
+        if (!pa.onehot) {
           eng->launch(tq_index::kScan, s, what, [&] { return vcb::launch_bucket_scan(ba, grid, s); });
-          return;
         }
+        if (!pa.onehot && !ask) return;
         eng->check_status = true;
         if (s != eng->stream) eng->status_foreign = true;
+        vcb::BucketScanArgs oa = ba;
+        if (ask) oa.n_items = pa.n_onehot;
         eng->launch(tq_index::kScan, s, what, [&] {
-          return vcb::launch_onehot_buckets(ba, static_cast<long long>(m), static_cast<long long>(n_slots), eng->sms,
+          return vcb::launch_onehot_buckets(oa, static_cast<long long>(m), static_cast<long long>(n_slots), eng->sms,
                                             eng->device_status(), s);
         });
       };
