@@ -203,3 +203,24 @@ def test_probe_counts_per_query_decide_by_their_pairs(nb_queries, many):
         assert np.array_equal(whole.ids[s:s + step], part.ids), s
         assert np.array_equal(whole.scores[s:s + step].view(np.uint32), part.scores.view(np.uint32)), s
     idx.close()
+
+
+@pytest.mark.parametrize("n,nq,k", [
+    (2048, 3, 1), (2048, 2, 32),   # one list: fewer candidates than lanes, as many
+    (16384, 1, 32),                # 256 candidates: the most that one warp merges
+    (16385, 2, 32), (18433, 1, 29),  # one list more
+    (524288, 1, 1), (524289, 1, 1),
+])
+@pytest.mark.parametrize("zeros", [False, True])
+def test_merge_of_few_candidates(oracle, n, nq, k, zeros):
+    db = power_law(n, 8, seed=33)
+    q = np.zeros((nq, 8), np.float32) if zeros else power_law(nq, 8, seed=34)
+    idx = vcb.TurboQuantIndex(8, 4)
+    idx.add(db)
+    idx.prepare()
+    res = idx.search(q, k)
+    packed, alpha = oracle.encode(db, 4, None, None)
+    want_s, want_i = oracle.search_flat(q, 4, packed, alpha, k, None, None)
+    assert np.array_equal(res.ids, want_i)
+    assert np.array_equal(res.scores.view(np.uint32), want_s.view(np.uint32))
+    idx.close()

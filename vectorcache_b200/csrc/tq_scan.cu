@@ -560,6 +560,75 @@ __device__ __forceinline__ uint32_t score_key(float s) {
 // ranges): 150 -> 20 us against sorting 1024 candidates at a time.
 constexpr int kMergeRank = 512;
 constexpr int kMergeDirect = 64;  // candidates that need no bound
+constexpr int kMergeOneWarp = 256;  // candidates that one warp merges by itself (k <= 32)
+
+// The best kout of at most kMergeOneWarp candidates, kout <= 32, by one warp: as in
+// merge_kernel, the lanes' best scores giving the bound, but without barriers, which cost
+// more than the other warps bring here: one query over 50k x 128, k = 2 to 5 (50 to 125
+// candidates) 29.0 us by the whole CTA, 27.0 by one warp; 200k x 128 3-bit, k = 1 29.4 and
+// 26.3. (A kernel of one-warp CTAs of its own: no faster.)
+// buf_s, s_rank: kMergeOneWarp entries.
+__device__ __forceinline__ void merge_one_warp(const MergeArgs& a, long long qi, int total, const float* cs,
+                                               const uint32_t* ci, float* buf_s, unsigned long long* s_rank, int lane) {
+  constexpr int kEach = kMergeOneWarp / kWarp;
+  const int kout = a.k_out;
+  float sc[kEach];
+  uint32_t id[kEach];
+#pragma unroll
+  for (int u = 0; u < kEach; ++u) {
+    const int at = u * kWarp + lane;
+    sc[u] = at < total ? cs[at] : -INFINITY;
+    id[u] = at < total ? ci[at] : 0u;
+  }
+  uint32_t bound = 0u;
+#pragma unroll
+  for (int u = 0; u < kEach; ++u) {
+    if (sc[u] > -INFINITY) bound = max(bound, score_key(sc[u]));
+  }
+#pragma unroll
+  for (int size = 2; size <= kWarp; size <<= 1) {
+#pragma unroll
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      const uint32_t o = __shfl_xor_sync(full_mask(), bound, step);
+      const bool lower = (lane & step) == 0, desc = (lane & size) == 0;
+      bound = lower == desc ? max(bound, o) : min(bound, o);
+    }
+  }
+  bound = max(1u, __shfl_sync(full_mask(), bound, kout - 1));
+  int n = 0;
+#pragma unroll
+  for (int u = 0; u < kEach; ++u) {
+    const uint32_t key = score_key(sc[u]);
+    const bool take = sc[u] > -INFINITY && key >= bound;
+    const unsigned votes = __ballot_sync(full_mask(), take);
+    if (take) {
+      const int at = n + __popc(votes & ((1u << lane) - 1u));
+      buf_s[at] = sc[u];
+      s_rank[at] = (static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(~id[u]);
+    }
+    n += __popc(votes);
+  }
+  const int padded = (n + 7) / 8 * 8;  // the padding ranks behind everything
+  if (lane < padded - n) s_rank[n + lane] = 0ull;
+  __syncwarp();
+  for (int t = lane; t < n; t += kWarp) {
+    const unsigned long long key = s_rank[t];
+    int rank = 0;
+    for (int j = 0; j < padded; j += 8) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) rank += s_rank[j + u] >= key + (j + u < t ? 0ull : 1ull) ? 1 : 0;
+    }
+    if (rank < kout) {
+      a.out_score[qi * kout + rank] = buf_s[t];
+      a.out_id[qi * kout + rank] = static_cast<uint64_t>(static_cast<uint32_t>(~static_cast<uint32_t>(key)));
+    }
+  }
+  if (lane >= n && lane < kout) {
+    a.out_score[qi * kout + lane] = 0.f;
+    a.out_id[qi * kout + lane] = a.pad_id;
+  }
+}
+
 __global__ void __launch_bounds__(kMergeThreads) merge_kernel(MergeArgs a) {
   __shared__ float buf_s[kMergeCap];
   __shared__ uint32_t buf_i[kMergeCap];
@@ -577,6 +646,10 @@ __global__ void __launch_bounds__(kMergeThreads) merge_kernel(MergeArgs a) {
   const float* cs = a.cand_score + qi * stride;
   const uint32_t* ci = a.cand_id + qi * stride;
   const int kout = a.k_out;
+  if (total <= kMergeOneWarp && kout <= kWarp) {
+    if (tid < kWarp) merge_one_warp(a, qi, static_cast<int>(total), cs, ci, buf_s, s_rank, lane);
+    return;
+  }
   if (tid == 0) n_new = 0;
   uint32_t bound = 1u;  // every score above -inf
   float v[kAhead];
