@@ -1061,13 +1061,18 @@ int choose_ranges(long long q_tiles, long long tiles, int pairs) {
 //     queries stream the codes at HBM speed and stay there;
 //   * lookups, k > 32: lists in shared memory and a merge that sorts them; slower
 //     from three queries on everywhere, for one or two 15 + 0.035 (k - 8) per block
-//     over the stream of the codes.
+//     over the stream of the codes, which they keep up to 5 % above the estimate here
+//     (one query of k = 64 over 1M x 1536 1096 / 1126).
 // Measured (lookup / here): 1M x 1536 4-bit 8 queries 937 / 1155, 12 queries
 // 1272 / 1155, 16 queries 1721 / 1155; 100k x 128 4-bit 24 queries 69 / 74, 32
 // queries 94 / 74; 2M x 768 3-bit 8 queries 647 / 774, 12 queries 826 / 774;
 // 20k x 768 4-bit 4 queries 125 / 85; one query of k = 64 over 100k x 128
 // 197 / 112, of k = 40 over 1M x 1536 706 / 1153, of k = 200 3431 / 1351.
 bool onehot_pays(long long n, long long nq, int nbg, int bits, int k, int sms) {
+  // Above 64 queries here everywhere: the smallest indexes are launches on both sides
+  // (lookups / here, 65 queries of k = 10: 8,192 x 64 4-bit 47.6 / 43.5 us, 3-bit
+  // 45.6 / 43.2, 8,192 x 128 3-bit 48.1 / 48.6, 32,768 x 64 3-bit 48.6 / 49.0; 96 to 512
+  // queries over 8k to 100k vectors of 64 to 1536 dims 0.98 to 19.8 times).
   if (nq > Config<kSmall>::kCols) return true;
   const long long pairs = sms / 2, tiles = (n + kPairVectors - 1) / kPairVectors;
   const double blocks = static_cast<double>((n + kScanBlockVectors - 1) / kScanBlockVectors);
@@ -1075,7 +1080,7 @@ bool onehot_pays(long long n, long long nq, int nbg, int bits, int k, int sms) {
   const double here = 25.0 + static_cast<double>((tiles + pairs - 1) / pairs) * stages * (bits == 3 ? 0.56 : 0.43);
   if (nq <= 2) {
     if (k <= 32) return false;
-    return static_cast<double>(n) * nbg / 4.8e6 + 15.0 + 0.035 * (k - 8) * blocks > here;
+    return static_cast<double>(n) * nbg / 4.8e6 + 15.0 + 0.035 * (k - 8) * blocks > 1.05 * here;
   }
   if (k > 32) return true;
   const double ctas = static_cast<double>((nq + 3) / 4) * blocks;
