@@ -40,6 +40,9 @@ inline void throw_on_error(int rc) {
   }
 }
 
+// Frees the device memory kept for later allocations (tq_trim).
+inline void trim() { throw_on_error(tq_trim()); }
+
 // Row-major top-k like vectorcache::SearchResults (search.hpp:77-84).
 struct SearchResults {
   std::vector<float> scores;      // nq * k

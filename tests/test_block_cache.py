@@ -1,5 +1,6 @@
 """Device blocks that closed indexes leave for later allocations: giving one back
-does not disturb a graph that another thread captures."""
+does not disturb a graph that another thread captures, and trim() hands them to
+the rest of the process."""
 import threading
 
 import pytest
@@ -40,3 +41,17 @@ def test_an_index_closes_while_another_thread_captures():
     again, db = _index(40_000, 128)
     assert (again.search(db[:4], 1).ids[:, 0] == range(4)).all()
     again.close()
+
+
+def test_trim_gives_kept_blocks_back():
+    torch = pytest.importorskip("torch")
+    vcb.trim()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    idx, _ = _index(400_000, 128)  # 205 MB of rows until prepare(), 25.6 MB of codes
+    idx.close()
+    kept = before - torch.cuda.mem_get_info()[0]
+    vcb.trim()
+    assert kept >= 200 << 20
+    assert before - torch.cuda.mem_get_info()[0] <= 8 << 20
+    assert vcb.trim() is None  # nothing left: no error

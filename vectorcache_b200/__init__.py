@@ -30,6 +30,7 @@ __all__ = [
     "rotation_tables",
     "scan_plan_shape",
     "load_library",
+    "trim",
     "LIB_PATH",
 ]
 
@@ -76,6 +77,7 @@ def _declare(lib):
     sig = {
         "tq_last_error": (C.c_char_p, []),
         "tq_version": (C.c_char_p, []),
+        "tq_trim": (C.c_int, []),
         "tq_codebook": (C.c_int, [_SZ, _SZ, _P, _P]),
         "tq_rotation_tables": (C.c_int, [_SZ, _P, _P]),
         "tq_index_create": (C.c_int, [_SZ, _SZ, C.c_uint32, C.c_int, C.POINTER(_P)]),
@@ -167,6 +169,12 @@ def _rows(x, dim: int) -> np.ndarray:
     if a.ndim != 2 or a.shape[1] != dim:
         raise InvalidArgument(TQ_ERR_INVALID_ARGUMENT, f"expected [n, {dim}] float32 rows")
     return a
+
+
+def trim() -> None:
+    """Free the device memory kept for later allocations: blocks of closed indexes
+    and outgrown buffers, at most 2 GiB a process."""
+    _check(load_library().tq_trim())
 
 
 def codebook(bits: int, dim: int) -> tuple[np.ndarray, np.ndarray]:

@@ -228,6 +228,10 @@ extern "C" {
 
 const char* tq_last_error(void) { return vcb::g_last_error.c_str(); }
 
+int tq_trim(void) {
+  return vcb::guarded([&] { vcb::BlockCache::get().trim(); });
+}
+
 const char* tq_version(void) { return "vectorcache_b200 0.1.0 (sm_100a)"; }
 
 int tq_codebook(size_t bits, size_t dim, float* boundaries, float* centroids) {
