@@ -103,7 +103,12 @@ int tq_index_search(tq_index* h, const float* queries, size_t nq, size_t k, floa
 int tq_index_search_device(tq_index* h, const float* d_queries, size_t nq, size_t k,
                            float* d_scores, uint64_t* d_ids, size_t* k_eff, void* stream);
 
-/* Block until the index's queued work is done. */
+/* Block until the index's queued work is done. TQ_ERR_CUDA also when a search that
+ * tq_index_search_device (or a bucketed *_device search of this engine) queued since
+ * the last call gave up waiting on its own pipeline, which bounds every wait to about
+ * two seconds: its results are not valid. Wait for a caller's stream first; its
+ * searches are reported once they are complete. The host-buffer searches, the server
+ * and the multi-index launch report theirs themselves. */
 int tq_index_synchronize(tq_index* h);
 
 /* ---- persistence and file formats -------------------------------------------
@@ -479,6 +484,8 @@ int tq_multi_buffers(tq_multi* h, size_t i, float** d_queries, float** d_scores,
 int tq_multi_launch(tq_multi* h, void* stream);
 /* The same sequence issued kernel by kernel (no graph), for comparison. */
 int tq_multi_run_uncaptured(tq_multi* h, void* stream);
+/* Block until the last launch is done, on whichever stream it was queued.
+ * TQ_ERR_CUDA also when a kernel of a launch gave up waiting (tq_index_synchronize). */
 int tq_multi_synchronize(tq_multi* h);
 /* Chosen configuration; tuned_ms receives up to *n_tuned candidate timings
  * (on return *n_tuned = candidates timed). */

@@ -556,13 +556,11 @@ struct tq_bucketed {
           eng->launch(tq_index::kScan, s, what, [&] { return vcb::launch_bucket_scan(ba, grid, s); });
         }
         if (!pa.onehot && !ask) return;
-        eng->check_status = true;
-        if (s != eng->stream) eng->status_foreign = true;
         vcb::BucketScanArgs oa = ba;
         if (ask) oa.n_items = pa.n_onehot;
         eng->launch(tq_index::kScan, s, what, [&] {
           return vcb::launch_onehot_buckets(oa, static_cast<long long>(m), static_cast<long long>(n_slots), eng->sms,
-                                            eng->device_status(), s);
+                                            sc.flat.status, s);
         });
       };
       if (two_phase) {
@@ -810,6 +808,7 @@ int tq_bucketed_search_device(tq_bucketed* h, const float* d_queries, size_t nq,
     require(np >= 1 && np <= static_cast<size_t>(vcb::kMaxProbe), TQ_ERR_INVALID_ARGUMENT, "n_probe must be in [1, 2048]");
     vcb::DeviceGuard g(h->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : h->stream();
+    h->own.flat.status = h->eng->queued_status.word();
     h->search_device(d_queries, nq, ke, static_cast<int>(std::min<size_t>(np, h->nb)), d_n_probe, d_scores, d_ids,
                      s);
   });
@@ -838,11 +837,13 @@ int tq_bucketed_search(tq_bucketed* h, const float* queries, size_t nq, size_t k
       h->eng->upload(h->s_np.get(), n_probe_per_query, nq * 4);
       d_np = h->s_np.as<uint32_t>();
     }
+    h->own.flat.status = h->eng->call_status.word();
     h->search_device(h->s_q.as<float>(), nq, ke, static_cast<int>(std::min<size_t>(np, h->nb)), d_np,
                      h->s_out_s.as<float>(), h->s_out_i.as<uint64_t>(), h->stream());
     vcb::check(cudaMemcpyAsync(scores, h->s_out_s.get(), nq * ke * 4, cudaMemcpyDeviceToHost, h->stream()), "D2H");
     vcb::check(cudaMemcpyAsync(ids, h->s_out_i.get(), nq * ke * 8, cudaMemcpyDeviceToHost, h->stream()), "D2H");
     h->sync();
+    h->eng->call_status.check();
   });
 }
 
@@ -869,11 +870,13 @@ int tq_bucketed_search_trace(tq_bucketed* h, const float* queries, size_t nq, si
       h->eng->upload(h->s_np.get(), n_probe_per_query, nq * 4);
       d_np = h->s_np.as<uint32_t>();
     }
+    h->own.flat.status = h->eng->call_status.word();
     h->search_device(h->s_q.as<float>(), nq, ke, static_cast<int>(np), d_np, h->s_out_s.as<float>(),
                      h->s_out_i.as<uint64_t>(), h->stream(), offsets, probes, q_hat);
     vcb::check(cudaMemcpyAsync(scores, h->s_out_s.get(), nq * ke * 4, cudaMemcpyDeviceToHost, h->stream()), "D2H");
     vcb::check(cudaMemcpyAsync(ids, h->s_out_i.get(), nq * ke * 8, cudaMemcpyDeviceToHost, h->stream()), "D2H");
     h->sync();
+    h->eng->call_status.check();
   });
 }
 
@@ -896,6 +899,7 @@ int tq_bucketed_search_learned_device(tq_bucketed* h, const float* d_queries, si
     vcb::DeviceGuard g(h->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : h->stream();
     const vcb::LearnedProbe lp{mlp, coverage, min_confidence};
+    h->own.flat.status = h->eng->queued_status.word();
     h->search_device(d_queries, nq, ke, static_cast<int>(std::min<size_t>(np, h->nb)), nullptr, d_scores, d_ids, s,
                      h->own, nullptr, nullptr, nullptr, &lp);
   });
@@ -1049,6 +1053,7 @@ namespace vcb {
 
 BucketScratch* bucket_scratch_new() { return new BucketScratch(); }
 void bucket_scratch_delete(BucketScratch* sc) { delete sc; }
+void bucket_scratch_status(BucketScratch* sc, unsigned* word) { sc->flat.status = word; }
 void bucket_scratch_bind(BucketScratch* sc, ScratchArena* a) { sc->bind(a); }
 
 size_t bucketed_dim_in(const tq_bucketed* h) { return h->dim_in; }

@@ -33,6 +33,53 @@ bool& dry_run_flag() {
   return flag;
 }
 
+// The words come from pages of pinned memory that the process keeps; as many pages as
+// the most words in use at a time need.
+namespace {
+struct WordPool {
+  std::mutex mu;
+  std::vector<unsigned*> free;
+  static WordPool& get() {
+    static WordPool* pool = new WordPool;  // outlives every owner, static ones too
+    return *pool;
+  }
+};
+}  // namespace
+
+WaitStatus::~WaitStatus() {
+  if (!word_) return;
+  *static_cast<volatile unsigned*>(word_) = 0u;
+  WordPool& pool = WordPool::get();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  pool.free.push_back(word_);  // within the capacity that word() reserved
+}
+
+unsigned* WaitStatus::word() {
+  if (word_) return word_;
+  constexpr size_t kWords = 1024;
+  WordPool& pool = WordPool::get();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  if (pool.free.empty()) {
+    static size_t words = 0;  // under the lock
+    pool.free.reserve(words + kWords);  // every word fits: giving one back never allocates
+    void* page = nullptr;
+    vcb::check(cudaHostAlloc(&page, kWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped), "cudaHostAlloc");
+    std::memset(page, 0, kWords * sizeof(unsigned));
+    words += kWords;
+    for (size_t i = 0; i < kWords; ++i) pool.free.push_back(static_cast<unsigned*>(page) + i);
+  }
+  word_ = pool.free.back();
+  pool.free.pop_back();
+  return word_;
+}
+
+bool WaitStatus::take() {
+  volatile unsigned* w = word_;
+  if (!w || *w == 0u) return false;
+  *w = 0u;
+  return true;
+}
+
 BlockCache& BlockCache::get() {
   static BlockCache* cache = new BlockCache;  // outlives every index, static ones too
   return *cache;
@@ -287,7 +334,9 @@ int tq_index_create(size_t dim, size_t bits, uint32_t flags, int device, tq_inde
     h->d_perm_sign.reserve(dim * 4);
     h->d_bnd.reserve(64);
     h->d_cen.reserve(64);
-    h->d_counter.reserve(16);  // replay count, wait status
+    h->d_counter.reserve(8);
+    h->call_status.word();
+    h->queued_status.word();
     h->upload(h->d_perm_sign.get(), ps.data(), dim * 4);
     h->upload(h->d_bnd.get(), bnd.data(), 64);
     h->upload(h->d_cen.get(), cen.data(), 64);
@@ -301,7 +350,7 @@ int tq_index_create(size_t dim, size_t bits, uint32_t flags, int device, tq_inde
       h->upload(h->d_grid.get(), cells.data(), cells.size() * 4);
       h->has_grid = true;
     }
-    vcb::check(cudaMemsetAsync(h->d_counter.get(), 0, 16, h->stream), "cudaMemsetAsync");
+    vcb::check(cudaMemsetAsync(h->d_counter.get(), 0, 8, h->stream), "cudaMemsetAsync");
     h->sync();
     *out = h.release();
   });
@@ -390,7 +439,8 @@ int tq_index_search_device(tq_index* h, const float* d_queries, size_t nq, size_
     require(d_queries && d_scores && d_ids, TQ_ERR_INVALID_ARGUMENT, "null buffer");
     check_aligned(d_queries, "queries");
     vcb::DeviceGuard g(h->device);
-    h->search_device(d_queries, nq, k, d_scores, d_ids, ke, h->pick(stream));
+    h->search_device(d_queries, nq, k, d_scores, d_ids, ke, h->pick(stream),
+                     h->own_scratch(h->queued_status.word()));
   });
 }
 
@@ -410,11 +460,12 @@ int tq_index_search(tq_index* h, const float* queries, size_t nq, size_t k, floa
     h->d_out_i.reserve(nq * ke * 8);
     h->upload(h->d_queries.get(), queries, nq * h->dim * 4);
     h->search_device(h->d_queries.as<float>(), nq, k, h->d_out_s.as<float>(), h->d_out_i.as<uint64_t>(),
-                     ke, h->stream);
+                     ke, h->stream, h->own_scratch(h->call_status.word()));
     vcb::check(cudaMemcpyAsync(scores, h->d_out_s.get(), nq * ke * 4, cudaMemcpyDeviceToHost, h->stream),
                "D2H");
     vcb::check(cudaMemcpyAsync(ids, h->d_out_i.get(), nq * ke * 8, cudaMemcpyDeviceToHost, h->stream), "D2H");
     h->sync();
+    h->call_status.check();
   });
 }
 
@@ -423,7 +474,13 @@ int tq_index_synchronize(tq_index* h) {
     require(h != nullptr, TQ_ERR_INVALID_ARGUMENT, "null index");
     vcb::DeviceGuard g(h->device);
     h->sync();
+    h->queued_status.check();
   });
+}
+
+// For tests, which set the word as a kernel would (not in the header).
+unsigned* tq_test_index_status(tq_index* h, size_t queued) {
+  return queued ? h->queued_status.word() : h->call_status.word();
 }
 
 int tq_index_info(const tq_index* h, size_t* dim, size_t* bits, size_t* n, int* prepared, int* calibrated) {

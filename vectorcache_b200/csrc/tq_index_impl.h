@@ -6,7 +6,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -93,6 +92,29 @@ class BlockCache {
   size_t total_ = 0;
 };
 
+// A word that a kernel with bounded waits (tq_onehot.cu) sets when one of them gave up:
+// its results are not valid then. Each owner of searches has its own, so that the call
+// that waits for the work reports it and no other does. Pinned host memory, written by
+// the device: once the work was waited for, reading it costs no copy.
+class WaitStatus {
+ public:
+  WaitStatus() = default;
+  WaitStatus(const WaitStatus&) = delete;
+  WaitStatus& operator=(const WaitStatus&) = delete;
+  ~WaitStatus();
+  unsigned* word();
+  // Whether it was set since the last look.
+  bool take();
+  void check() {
+    if (take()) fail(TQ_ERR_CUDA, kGaveUp);
+  }
+  static constexpr const char* kGaveUp =
+      "a scan kernel gave up waiting on its own pipeline; its results are not valid";
+
+ private:
+  unsigned* word_ = nullptr;
+};
+
 // Grow-only device allocation: a block of the cache, or a piece of a bound ScratchArena.
 class DeviceBuffer {
  public:
@@ -173,15 +195,17 @@ struct FlatScratch {
   DeviceBuffer* partial = nullptr;  // nullptr: the scan does not split
   long long range_cap = 0;          // > 0: at most this many vectors per scan CTA
   DeviceBuffer* onehot = nullptr;   // nullptr: batches stay on the lookup scan
+  unsigned* status = nullptr;       // WaitStatus::word of the search's owner
 };
 
 // Owning variant for callers that run searches concurrently (one per stream).
 struct FlatScratchStore {
   DeviceBuffer luts, qf, cand_s, cand_i, partial, onehot;
   long long range_cap = 0;  // see FlatScratch::range_cap
+  unsigned* status = nullptr;
   // Searches that bound a CTA's vectors (the server's) keep the lookup scan:
   // the one-hot kernel holds its SMs for the whole search.
-  FlatScratch ref() { return {&luts, &qf, &cand_s, &cand_i, &partial, range_cap, range_cap > 0 ? nullptr : &onehot}; }
+  FlatScratch ref() { return {&luts, &qf, &cand_s, &cand_i, &partial, range_cap, range_cap > 0 ? nullptr : &onehot, status}; }
   void bind(ScratchArena* a) {
     for (DeviceBuffer* b : {&luts, &qf, &cand_s, &cand_i, &partial, &onehot}) b->bind(a);
   }
@@ -197,6 +221,8 @@ void calibrate_index(tq_index* h, const float* d_sample, size_t n, cudaStream_t 
 }  // namespace vcb
 
 struct tq_index {
+  // Of searches that the host call waits for, and of those that search_device queues.
+  vcb::WaitStatus call_status, queued_status;
   int device = 0;
   int sms = 148;
   cudaStream_t stream = nullptr;
@@ -216,11 +242,6 @@ struct tq_index {
   vcb::DeviceBuffer d_codes, d_alpha, d_staged, d_flat, d_counter;
   // search scratch
   vcb::DeviceBuffer d_queries, d_luts, d_qf, d_cand_s, d_cand_i, d_out_s, d_out_i, d_qrot, d_partial, d_onehot;
-  // Set once a search ran a kernel with bounded waits: sync() then looks at the
-  // word such a kernel sets when a wait gave up (behind d_counter's count).
-  // A search on another stream may still be running then: it keeps the flag set.
-  // (Searches of one index may be queued from several threads.)
-  std::atomic<bool> check_status{false}, status_foreign{false};
 
   // Optional per-launch timing (tq_index_set_profiling).
   enum Kind { kPrep = 0, kScan = 1, kMerge = 2, kEncode = 3 };
@@ -281,20 +302,7 @@ struct tq_index {
     timed_launches.push_back(t);
   }
 
-  void sync() {
-    vcb::check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-    if (check_status) {
-      unsigned status = 0;
-      vcb::check(cudaMemcpyAsync(&status, device_status(), 4, cudaMemcpyDeviceToHost, stream), "D2H");
-      vcb::check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-      check_status = status_foreign.load();
-      if (status) {
-        vcb::check(cudaMemsetAsync(device_status(), 0, 4, stream), "cudaMemsetAsync");
-        vcb::fail(TQ_ERR_CUDA, "a scan kernel gave up waiting on its own pipeline; its results are not valid");
-      }
-    }
-  }
-  unsigned* device_status() const { return d_counter.as<unsigned>() + 2; }
+  void sync() { vcb::check(cudaStreamSynchronize(stream), "cudaStreamSynchronize"); }
 
   cudaStream_t pick(void* s) const { return s ? static_cast<cudaStream_t>(s) : stream; }
 
@@ -380,7 +388,9 @@ struct tq_index {
   }
 
   // The index's own search scratch (one search at a time on one stream).
-  vcb::FlatScratch own_scratch() { return {&d_luts, &d_qf, &d_cand_s, &d_cand_i, &d_partial, 0, &d_onehot}; }
+  vcb::FlatScratch own_scratch(unsigned* status = nullptr) {
+    return {&d_luts, &d_qf, &d_cand_s, &d_cand_i, &d_partial, 0, &d_onehot, status};
+  }
 
   // LUTs and per-query constants for nq device rows.
   void prep_queries(const float* d_q, size_t nq, cudaStream_t s, float* q_rot_out) {
@@ -414,12 +424,8 @@ struct tq_index {
   }
 
   // Full device search of nq rows at d_q into d_scores/d_ids (stride k_eff).
-  void search_device(const float* d_q, size_t nq, size_t k, float* d_scores, uint64_t* d_ids,
-                     size_t k_eff, cudaStream_t s) {
-    search_device(d_q, nq, k, d_scores, d_ids, k_eff, s, own_scratch());
-  }
-  // Same with caller-owned scratch: searches with distinct scratch may run
-  // concurrently on distinct streams (the index data is only read).
+  // Searches with distinct scratch may run concurrently on distinct streams (the
+  // index data is only read).
   void search_device(const float* d_q, size_t nq, size_t k, float* d_scores, uint64_t* d_ids,
                      size_t k_eff, cudaStream_t s, vcb::FlatScratch sc) {
     if (nq == 0 || k_eff == 0) return;
@@ -530,9 +536,7 @@ struct tq_index {
       });
       a.luts = compact_luts;
     }
-    a.status = device_status();
-    check_status = true;
-    if (s != stream) status_foreign = true;
+    a.status = sc.status;
     launch(kPrep, s, "threshold sample kernel", [&] { return vcb::launch_onehot_sample(a, p, sms, s); });
     launch(kPrep, s, "threshold kernel", [&] {
       return vcb::launch_kth_floor(a.dense, static_cast<long long>(p.sample_tiles) * 256, nullptr,

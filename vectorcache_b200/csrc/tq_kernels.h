@@ -215,7 +215,7 @@ struct OneHotArgs {
   const float* floor;   // per query: no score below it reaches the top k
   float* dense;         // sample: nq x dense_stride scores
   long long dense_stride;
-  unsigned* status;     // device word, set to 1 when a wait gave up
+  unsigned* status;     // set to 1 when a wait gave up (WaitStatus::word, or null)
   // Bucket items (launch_onehot_buckets): see BucketScanArgs in tq_bucket.h.
   const uint4* items;
   const unsigned long long* n_items;

@@ -34,8 +34,10 @@
 #include "tq_kernels.h"
 
 struct tq_multi {
+  vcb::WaitStatus status;  // of the direct batches
   int device = 0, sms = 148;
   cudaStream_t stream = nullptr;
+  cudaEvent_t done = nullptr;  // behind the last launch, on whichever stream
   std::vector<tq_index*> idx;
   // plan
   std::vector<size_t> nq, k, ke;
@@ -59,7 +61,15 @@ struct tq_multi {
     if (stream) cudaStreamSynchronize(stream);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
+    if (done) cudaEventDestroy(done);
     if (stream) cudaStreamDestroy(stream);
+  }
+
+  // A launch that a caller's capture records is waited for with that graph.
+  void mark_done(cudaStream_t s) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    vcb::check(cudaStreamIsCapturing(s, &capturing), "cudaStreamIsCapturing");
+    if (capturing == cudaStreamCaptureStatusNone) vcb::check(cudaEventRecord(done, s), "cudaEventRecord");
   }
 
   // Items and descriptors for a range length; sizes the scratch.
@@ -238,6 +248,7 @@ int tq_multi_create(tq_index* const* indexes, size_t n_indexes, tq_multi** out) 
     vcb::DeviceGuard g(h->device);
     h->sms = indexes[0]->sms;
     vcb::check(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    vcb::check(cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming), "cudaEventCreate");
     h->d_counter.reserve(8);
     *out = h.release();
   });
@@ -270,6 +281,7 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
       require(k[i] >= 1 && k[i] <= static_cast<size_t>(vcb::kMaxK), TQ_ERR_INVALID_ARGUMENT, "k must be in [1, 256]");
       h->ke[i] = std::min(k[i], h->idx[i]->n);
       h->scratch.push_back(std::make_unique<vcb::FlatScratchStore>());
+      h->scratch[i]->status = h->status.word();
       h->d_q.push_back(std::make_unique<vcb::DeviceBuffer>());
       h->d_s.push_back(std::make_unique<vcb::DeviceBuffer>());
       h->d_i.push_back(std::make_unique<vcb::DeviceBuffer>());
@@ -363,6 +375,7 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
       set_direct(best_d, best_d_rv);
     }
     h->capture();
+    h->status.check();  // the runs so far are complete
     h->planned = true;
   });
 }
@@ -386,6 +399,7 @@ int tq_multi_launch(tq_multi* h, void* stream) {
     vcb::DeviceGuard g(h->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : h->stream;
     vcb::check(cudaGraphLaunch(h->exec, s), "cudaGraphLaunch");
+    h->mark_done(s);
   });
 }
 
@@ -394,7 +408,9 @@ int tq_multi_run_uncaptured(tq_multi* h, void* stream) {
     checked(h);
     require(h->planned, TQ_ERR_STATE, "plan() first");
     vcb::DeviceGuard g(h->device);
-    h->run(stream ? static_cast<cudaStream_t>(stream) : h->stream);
+    cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : h->stream;
+    h->run(s);
+    h->mark_done(s);
   });
 }
 
@@ -403,8 +419,13 @@ int tq_multi_synchronize(tq_multi* h) {
     checked(h);
     vcb::DeviceGuard g(h->device);
     vcb::check(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    vcb::check(cudaEventSynchronize(h->done), "cudaEventSynchronize");
+    h->status.check();
   });
 }
+
+// For tests, which set the word as a kernel would (not in the header).
+unsigned* tq_test_multi_status(tq_multi* h) { return h->status.word(); }
 
 int tq_multi_config(tq_multi* h, long long* range_vectors, int* ctas, size_t* n_items, size_t* smem_bytes,
                     double* tuned_ms, size_t* n_tuned) {

@@ -943,7 +943,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Config<V>::kThreads,
       close_item();
     }
   }
-  if (!alive && a.status) atomicExch(a.status, 1u);
+  if (!alive && a.status) {  // pinned host memory
+    *static_cast<volatile unsigned*>(a.status) = 1u;
+    __threadfence_system();
+  }
   // A role that gave up waited about two seconds first, so no copy of this
   // CTA is still in flight here; otherwise every load was consumed.
   __syncwarp();

@@ -77,6 +77,7 @@ struct Request {
 };
 
 struct Slot {
+  vcb::WaitStatus status;
   cudaStream_t stream = nullptr;     // flat batches (normal priority)
   cudaStream_t stream_hi = nullptr;  // bucketed batches (highest priority)
   cudaEvent_t done = nullptr;
@@ -260,6 +261,12 @@ struct tq_server {
 
   void retire(Slot& sl) {
     free_region(sl);
+    if (sl.status.take()) {
+      fail_batch(sl.batch, TQ_ERR_CUDA, vcb::WaitStatus::kGaveUp);
+      sl.batch.clear();
+      sl.busy = false;
+      return;
+    }
     size_t row = 0;
     const int64_t t = sl.done_ns.load();
     for (Request* r : sl.batch) {
@@ -442,9 +449,12 @@ struct tq_server {
       // kernels are loaded on their first launch, and that device memory is
       // resident, not part of the scratch arena.
       vcb::DeviceBuffer q, sc_s, sc_i;
+      vcb::WaitStatus status;
       vcb::FlatScratchStore fs;
       fs.range_cap = kServingRangeVectors;
+      fs.status = status.word();
       vcb::BucketScratch* bs = vcb::bucket_scratch_new();
+      vcb::bucket_scratch_status(bs, status.word());
       const size_t m = max_batch;
       q.reserve(m * max_dim * 4);
       sc_s.reserve(m * max_k * 4);
@@ -465,6 +475,7 @@ struct tq_server {
       }
       vcb::check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
       vcb::bucket_scratch_delete(bs);
+      status.check();
     }
     for (size_t s = 0; s < max_slots; ++s) {
       auto sl = std::make_unique<Slot>();
@@ -481,7 +492,9 @@ struct tq_server {
       sl->d_q.reserve(max_batch * max_dim * 4);
       sl->d_s.reserve(max_batch * max_k * 4);
       sl->d_i.reserve(max_batch * max_k * 8);
+      sl->flat.status = sl->status.word();
       sl->bkt = vcb::bucket_scratch_new();
+      vcb::bucket_scratch_status(sl->bkt, sl->status.word());
       slots.push_back(std::move(sl));
     }
     slot_bytes = max_batch * (max_dim * 4 + max_k * 12);
@@ -598,6 +611,9 @@ int tq_server_start(tq_server* h) {
     h->start();
   });
 }
+
+// For tests, which set the word as a kernel would (not in the header).
+unsigned* tq_test_server_status(tq_server* h, size_t slot) { return h->slots.at(slot)->status.word(); }
 
 int tq_server_info(tq_server* h, size_t* n_slots, size_t* slot_bytes, size_t* resident_bytes) {
   return vcb::guarded([&] {
