@@ -1062,15 +1062,16 @@ int choose_ranges(long long q_tiles, long long tiles, int pairs) {
 //     blocks, 0.31 per byte group (3-bit 0.17) and 14 per wave of two CTAs per SM,
 //     0.21 (0.11) per group while every CTA has an SM to itself. One and two
 //     queries stream the codes at HBM speed and stay there;
-//   * lookups, k > 32: lists in shared memory and a merge that sorts them; slower
-//     from three queries on everywhere, for one or two 15 + 0.035 (k - 8) per block
-//     over the stream of the codes, which they keep up to 5 % above the estimate here
-//     (one query of k = 64 over 1M x 1536 1096 / 1126).
+//   * lookups, k > 32: lists in shared memory and a longer merge; slower from three
+//     queries on nearly everywhere (20k x 128 3-bit, 24 queries of k = 256 82 / 139 us
+//     is the worst of the others), for one or two by a fit of its own to 616 searches of
+//     8k to 3M vectors, k 33 to 256, that picks the faster side or one at most 10 %
+//     slower in all but 33 of them (a third slower at worst).
 // Measured (lookup / here): 1M x 1536 4-bit 8 queries 937 / 1155, 12 queries
 // 1272 / 1155, 16 queries 1721 / 1155; 100k x 128 4-bit 24 queries 69 / 74, 32
 // queries 94 / 74; 2M x 768 3-bit 8 queries 647 / 774, 12 queries 826 / 774;
-// 20k x 768 4-bit 4 queries 125 / 85; one query of k = 64 over 100k x 128
-// 197 / 112, of k = 40 over 1M x 1536 706 / 1153, of k = 200 3431 / 1351.
+// 20k x 768 4-bit 4 queries 125 / 85; one query of k = 100 over 1M x 1536 551 / 1137,
+// of k = 33 over 3M x 384 398 / 896, two of k = 48 over 8,192 x 128 58 / 39.
 bool onehot_pays(long long n, long long nq, int nbg, int bits, int k, int sms) {
   // Above 64 queries here everywhere: the smallest indexes are launches on both sides
   // (lookups / here, 65 queries of k = 10: 8,192 x 64 4-bit 47.6 / 43.5 us, 3-bit
@@ -1080,10 +1081,13 @@ bool onehot_pays(long long n, long long nq, int nbg, int bits, int k, int sms) {
   const long long pairs = sms / 2, tiles = (n + kPairVectors - 1) / kPairVectors;
   const double blocks = static_cast<double>((n + kScanBlockVectors - 1) / kScanBlockVectors);
   const double stages = static_cast<double>((nbg + (bits == 3 ? 31 : 15)) / (bits == 3 ? 32 : 16));
-  const double here = 25.0 + static_cast<double>((tiles + pairs - 1) / pairs) * stages * (bits == 3 ? 0.56 : 0.43);
+  const double scan = static_cast<double>((tiles + pairs - 1) / pairs) * stages * (bits == 3 ? 0.56 : 0.43);
+  const double here = 25.0 + scan;
   if (nq <= 2) {
     if (k <= 32) return false;
-    return static_cast<double>(n) * nbg / 4.8e6 + 15.0 + 0.035 * (k - 8) * blocks > 1.05 * here;
+    const double q = static_cast<double>(nq), nd = static_cast<double>(n);
+    return 10.0 + 18.0 * q + nd * nbg / 3.1e6 + 0.03 * nbg * q + blocks * (0.0015 * k * (1.0 + q) + 0.057 * q) + 0.1 * k >
+           28.0 + scan + 0.19 * k + 0.04 * nbg + 44e-6 * nd;
   }
   if (k > 32) return true;
   const double ctas = static_cast<double>((nq + 3) / 4) * blocks;
