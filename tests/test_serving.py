@@ -177,3 +177,45 @@ def test_batch_sizing_matches_what_runs(indexes):
         want = _alone(flat, bkt, target, fid, q, k, npb)
         assert np.array_equal(i, want.ids)
     srv.close()
+
+
+def test_the_arena_holds_a_full_batch_of_every_k(indexes):
+    # One slot: the arena is one largest batch. (Regions of at least 4096 entries in
+    # whole lists of k, and re-rank buffers below max_k, need more at some smaller k.)
+    _, bkt, _, _ = indexes
+    for max_k in (40, 64):
+        srv = vcb.Server(max_slots=1, max_batch=1024)
+        target = srv.add_bucketed(bkt, max_k, 32)
+        srv.start()
+        top = srv.memory()["max_batch_bytes"]
+        assert srv.memory()["arena_bytes"] + 256 > top
+        for n_probe in (4, 9, 17, 32):
+            assert max(srv.batch_bytes(target, 1024, k, n_probe) for k in range(1, max_k + 1)) <= top, n_probe
+        srv.close()
+
+
+def test_a_tight_budget_serves_with_less_scratch(indexes):
+    # A budget that holds the lists of a full batch but not the one-hot scan's larger
+    # regions is served on the lookup scan, with the same results.
+    _, bkt, _, xb = indexes
+
+    def start(budget):
+        srv = vcb.Server(hbm_budget_bytes=budget, max_slots=1, max_batch=1024)
+        target = srv.add_bucketed(bkt, 4, 12)
+        srv.start()
+        return srv, target
+
+    srv, target = start(100 << 30)
+    roomy = srv.batch_bytes(target, 1024, 4, 12)
+    srv.close()
+    with pytest.raises(vcb.TurboQuantError, match="bytes needed") as e:
+        start(1)
+    least = int(str(e.value).split("(")[1].split()[0])
+    srv, target = start(least + (4 << 20))
+    assert srv.batch_bytes(target, 1024, 4, 12) + (16 << 20) < roomy
+    q = xb[:900]
+    got = srv.submit(target, q, 4, 12).wait()
+    want = bkt.search(q, 4, n_probe=12)
+    assert np.array_equal(got[1], want.ids)
+    assert np.array_equal(got[0].view(np.uint32), want.scores.view(np.uint32))
+    srv.close()

@@ -1204,7 +1204,7 @@ struct ItemView {
   uint32_t* cand_i;
   // nullptr: each (query, tile set) writes its own list of k entries at
   // ItemQueries::list, -inf padded. Otherwise ItemQueries::list is the start
-  // (in lists of k) of the query's candidate region and the kept candidates
+  // (in entries) of the query's candidate region and the kept candidates
   // are appended there at append_count[query] (atomically), unpadded; the region
   // holds `region` entries, and what comes past its end is counted but not written.
   uint32_t* append_count = nullptr;
@@ -1217,7 +1217,7 @@ struct ItemView {
 // The item's queries, in shared memory (filled by the calling kernel).
 struct ItemQueries {
   int q[kItemQueries];           // LUT row (-1: no query)
-  long long list[kItemQueries];  // candidate list written by tile set 0 (tile set 1: list + 1)
+  long long list[kItemQueries];  // candidate list written by tile set 0 (tile set 1: list + 1), or the region
   float scale[kItemQueries], init[kItemQueries], off[kItemQueries];
   float floor[kItemQueries];     // scores below it are not kept (-inf: keep all)
 };
@@ -1527,7 +1527,7 @@ __device__ __forceinline__ void scan_item(const ItemView& v, const ItemQueries& 
       unsigned at = 0;
       if (lane == 0) at = atomicAdd(v.append_count + iq.q[quad * QW + q], static_cast<unsigned>(c));
       at = __shfl_sync(full_mask(), at, 0);
-      const long long base = iq.list[quad * QW + q] * k + at;
+      const long long base = iq.list[quad * QW + q] + at;
       // A one-hot step before this one may have filled the region (it appends every
       // score above the floor, not k a probe): nothing is written past its end, the
       // count says so and the query is scanned again (launch_bucket_redo).
@@ -1566,7 +1566,7 @@ __device__ __forceinline__ void bucket_scan_item(const BucketScanArgs& a, const 
       const int q = static_cast<int>(pr / static_cast<uint32_t>(a.max_probe));
       iq.q[t] = q;
       // (query, probe) lists, or the query's region when appending
-      iq.list[t] = a.append_count ? static_cast<long long>(q) * a.lists : static_cast<long long>(pr) * kBsListsPerProbe;
+      iq.list[t] = a.append_count ? static_cast<long long>(q) * a.region : static_cast<long long>(pr) * kBsListsPerProbe;
       iq.scale[t] = a.lut_scale[q];
       iq.init[t] = a.fa_init[q];
       iq.off[t] = a.offsets[pr];
@@ -1583,7 +1583,7 @@ __device__ __forceinline__ void bucket_scan_item(const BucketScanArgs& a, const 
   __syncthreads();
   const ItemView v{a.codes, a.alpha, a.slot_ids, static_cast<long long>(a.slot_start[b]),
                    static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, pc, a.cand_score, a.cand_id,
-                   a.append_count, a.lists * a.k, a.append_count && a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
+                   a.append_count, a.region, a.append_count && a.region >= static_cast<long long>(kBsWarps) * a.max_probe * a.k};
   scan_item<NIBBLE8, kBsQueriesPerWarp, WHOLE>(v, iq, smem);
 }
 
@@ -1642,7 +1642,7 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5)
     if (threadIdx.x < kItemQueries) {
       const int t = threadIdx.x;
       iq.q[t] = t == 0 ? q : -1;
-      iq.list[t] = t == 0 ? static_cast<long long>(q) * a.lists : 0;
+      iq.list[t] = t == 0 ? static_cast<long long>(q) * a.region : 0;
       iq.scale[t] = t == 0 ? a.lut_scale[q] : 0.f;
       iq.init[t] = t == 0 ? a.fa_init[q] : 0.f;
       iq.off[t] = t == 0 ? a.offsets[static_cast<long long>(q) * a.max_probe + j] : 0.f;
@@ -1651,7 +1651,7 @@ __global__ void __launch_bounds__(kBsWarps * 32, 5)
     __syncthreads();
     const ItemView v{a.codes, a.alpha, a.slot_ids, static_cast<long long>(a.slot_start[b]),
                      static_cast<int>(a.bucket_size[b]), a.nbg, a.luts, a.k, 1, a.cand_score, a.cand_id, a.append_count,
-                     a.lists * a.k, a.lists >= static_cast<long long>(kBsWarps) * a.max_probe};
+                     a.region, a.region >= static_cast<long long>(kBsWarps) * a.max_probe * a.k};
     scan_item<NIBBLE8, kBsQueriesPerWarp, WHOLE>(v, iq, smem);
   }
 }
@@ -2047,8 +2047,7 @@ cudaError_t launch_bucket_redo(const BucketScanArgs& a, long long nq, uint32_t* 
                                cudaStream_t stream) {
   if (nq <= 0) return cudaSuccess;
   if (a.k < 1 || a.k > kMaxK || !a.append_count || !redo) return cudaErrorInvalidValue;
-  overflow_list_kernel<<<static_cast<unsigned>((nq + 255) / 256), 256, 0, stream>>>(a.append_count, nq, a.lists * a.k,
-                                                                                    redo);
+  overflow_list_kernel<<<static_cast<unsigned>((nq + 255) / 256), 256, 0, stream>>>(a.append_count, nq, a.region, redo);
   const size_t smem = bucket_scan_smem(a.nbg, a.k);
   const bool whole = a.nbg % kBsPrefetch == 0;
   auto kern = a.bits == 3 ? (whole ? bucket_redo_kernel<true, true> : bucket_redo_kernel<true, false>)

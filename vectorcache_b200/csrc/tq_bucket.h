@@ -178,14 +178,14 @@ struct BucketScanArgs {
   const unsigned long long* n_items;
   unsigned long long* next_item;  // work counter (zeroed by launch_build_pairs)
   int nbg, bits, k, max_probe;
-  float* cand_score;         // (nq * max_probe * kBsListsPerProbe) lists of k, appending: nq * lists
+  float* cand_score;         // (nq * max_probe * kBsListsPerProbe) lists of k, appending: nq regions
   uint32_t* cand_id;
   // Optional per query: scores below floor[q] cannot reach the query's top k
   // and are not kept (nullptr: no floor).
   const float* floor = nullptr;
   // Optional per query (zeroed by the caller): the kept candidates of query q
-  // are appended, unpadded, to its region of `lists` lists of k entries (at least
-  // max_probe * kBsListsPerProbe) at cand_score/cand_id + q * lists * k, and
+  // are appended, unpadded, to its region of `region` entries (at least max_probe *
+  // kBsListsPerProbe lists of k) at cand_score/cand_id + q * region, and
   // append_count[q] counts them. No scan writes past a region's end; a count above
   // the region's size says that appends are missing there. Steps of this scan alone
   // append at most k entries per probe and tile set, which fit; after a one-hot step
@@ -193,7 +193,7 @@ struct BucketScanArgs {
   // pass the end, and launch_bucket_redo has to follow. nullptr: one -inf padded list
   // of k per (query, probe, tile set).
   uint32_t* append_count = nullptr;
-  long long lists = 0;
+  long long region = 0;
 };
 // `grid`: a bound of the item count; the launch runs min(grid, resident CTAs).
 cudaError_t launch_bucket_scan(const BucketScanArgs& a, long long grid, cudaStream_t stream);

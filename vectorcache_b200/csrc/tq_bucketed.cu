@@ -48,6 +48,7 @@ struct BucketScratch {
       cand_i, rr_s, rr_i, np, floor, acount, encs;
   FlatScratchStore flat;
   ProbeScratch probe;
+  bool lean = false;  // the lookup scan alone, in regions of one list per probe
   void bind(ScratchArena* a) {
     for (DeviceBuffer* b : {&qh, &route, &top_s, &top_i, &counts, &fill, &pstart, &istart, &pairs, &off, &items,
                             &nitems, &cand_s, &cand_i, &rr_s, &rr_i, &np, &floor, &acount, &encs}) {
@@ -391,14 +392,13 @@ struct tq_bucketed {
     });
   }
 
-  // Lists of kscan entries in a query's candidate region: one per probe, and at
-  // least kOneHotMinRegion entries (or all its probes' vectors) where a search
-  // has steps above a floor.
-  size_t region_lists(size_t max_probe, size_t kscan) const {
-    const size_t lists = max_probe * vcb::kBsListsPerProbe;
-    if (max_probe <= static_cast<size_t>(vcb::kFloorProbes)) return lists;
-    const size_t entries = std::min<size_t>(vcb::kOneHotMinRegion, max_probe * p.max_bucket_size);
-    return std::max(lists, (entries + kscan - 1) / kscan);
+  // Entries of a query's candidate region: a list of kscan per probe, and at least
+  // kOneHotMinRegion (or all its probes' vectors) where a search has steps above a floor.
+  // In entries, not rounded to lists, so that a smaller k never needs more.
+  size_t region_entries(size_t max_probe, size_t kscan, bool lean) const {
+    const size_t entries = max_probe * vcb::kBsListsPerProbe * kscan;
+    if (lean || max_probe <= static_cast<size_t>(vcb::kFloorProbes)) return entries;
+    return std::max(entries, std::min<size_t>(vcb::kOneHotMinRegion, max_probe * p.max_bucket_size));
   }
   // Queries per pass: routing scores (nb floats per query) within 256 MiB and
   // candidate lists (max_probe lists of kscan (score, id) per query) within
@@ -406,10 +406,10 @@ struct tq_bucketed {
   // repeats the routing, pair and floor launches on a smaller grid: at 1 GiB
   // with two lists per probe the same search ran in 8 passes and took 1.7x
   // as long for 64 probes per query under a 512-probe cap.
-  size_t pass_queries(size_t max_probe = 1, size_t kscan = 1) const {
+  size_t pass_queries(size_t max_probe = 1, size_t kscan = 1, bool lean = true) const {
     const size_t by_route = std::max<size_t>(1, (size_t{256} << 20) / (static_cast<size_t>(nb) * 4));
     const size_t by_cand =
-        std::max<size_t>(1, (size_t{8} << 30) / (region_lists(max_probe, kscan) * kscan * 8));
+        std::max<size_t>(1, (size_t{8} << 30) / (region_entries(max_probe, kscan, lean) * 8));
     return std::min<size_t>({16384, by_route, by_cand});
   }
 
@@ -431,7 +431,7 @@ struct tq_bucketed {
     const bool rerank = p.rerank_k > ke;
     // With re-ranking the scan keeps kscan candidates per query.
     const size_t kscan = rerank ? std::min<size_t>({static_cast<size_t>(p.rerank_k), n, 256}) : ke;
-    const size_t pass = pass_queries(static_cast<size_t>(max_probe), kscan);
+    const size_t pass = pass_queries(static_cast<size_t>(max_probe), kscan, sc.lean);
     for (size_t q0 = 0; q0 < nq; q0 += pass) {
       const size_t m = std::min(pass, nq - q0);
       sc.qh.reserve(m * dim * 4);
@@ -489,11 +489,11 @@ struct tq_bucketed {
       });
       pa.enc_scores = sc.encs.as<float>();
       pa.enc_ld = nb;
-      const size_t probes = static_cast<size_t>(max_probe), split = vcb::kSplitPairs;
-      size_t lists = region_lists(probes, kscan);
-      if (m * probes <= split) lists = std::max(lists, vcb::kSplitLists * probes);
+      const size_t probes = static_cast<size_t>(max_probe), split = sc.lean ? 0 : vcb::kSplitPairs;
+      size_t region = region_entries(probes, kscan, sc.lean);
+      if (m * probes <= split) region = std::max(region, vcb::kSplitLists * probes * kscan);
       // The smaller passes of a scratch reserved for this one fit it too.
-      const size_t entries = std::max(m * lists, vcb::kSplitLists * std::min(m * probes, split)) * kscan;
+      const size_t entries = std::max(m * region, vcb::kSplitLists * std::min(m * probes, split) * kscan);
       sc.cand_s.reserve(entries * 4);
       sc.cand_i.reserve(entries * 4);
       sc.floor.reserve(m * 4);
@@ -524,7 +524,7 @@ struct tq_bucketed {
       sc.acount.reserve((2 * m + 1) * 4);
       if (!vcb::dry_run_flag()) vcb::check(cudaMemsetAsync(sc.acount.get(), 0, (m + 1) * 4, s), "cudaMemsetAsync");
       ba.append_count = sc.acount.as<uint32_t>();
-      ba.lists = static_cast<long long>(lists);
+      ba.region = static_cast<long long>(region);
       // The best-routed buckets first: the k-th best score over a query's
       // first 8 (32 from 128 probes) probes is a lower bound of its k-th best over all
       // probes, so the scan of the remaining probes keeps only scores at or
@@ -544,7 +544,7 @@ struct tq_bucketed {
       bool any_onehot = false, ask = false;
       auto use_onehot = [&](long long step_pairs) {
         pa.onehot_from = vcb::kOneHotPairsCounted * nb;
-        const bool may = ba.floor && step_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2 &&
+        const bool may = !sc.lean && ba.floor && step_pairs >= vcb::kOneHotPairsPerBucket * nb && eng->sms >= 2 &&
                          vcb::onehot_buckets_fit(static_cast<long long>(m), static_cast<long long>(n_slots), ba.nbg);
         ask = may && np_pass != nullptr;
         pa.onehot = may && !ask;
@@ -564,7 +564,6 @@ struct tq_bucketed {
         });
       };
       if (two_phase) {
-        const long long region = ba.lists * static_cast<long long>(kscan);
         // Probe 0 alone, then probes 1..first-1 above probe 0's floor (the
         // first probes cost most without a floor), then the floor of all
         // first probes for the rest. Each floor is the k-th best of the
@@ -599,7 +598,7 @@ struct tq_bucketed {
           scan(st == 0 ? "bucket scan kernel (probe 0)" : "bucket scan kernel (first probes)",
                std::min(items, step_items));
           eng->launch(tq_index::kPrep, s, "floor kernel", [&] {
-            return vcb::launch_kth_floor(ba.cand_score, region, ba.append_count, static_cast<long long>(m),
+            return vcb::launch_kth_floor(ba.cand_score, ba.region, ba.append_count, static_cast<long long>(m),
                                          static_cast<int>(kscan), sc.floor.as<float>(), s);
           });
           ba.floor = sc.floor.as<float>();
@@ -623,8 +622,8 @@ struct tq_bucketed {
       mg.cand_score = ba.cand_score;
       mg.cand_id = ba.cand_id;
       mg.nq = static_cast<long long>(m);
-      mg.n_lists = static_cast<int>(lists);
-      mg.k = static_cast<int>(kscan);
+      mg.n_lists = static_cast<int>(region);  // rows of `region` entries, entry_count of them filled
+      mg.k = 1;
       mg.k_out = static_cast<int>(kscan);
       mg.out_score = d_scores + q0 * ke;
       mg.out_id = d_ids + q0 * ke;
@@ -1054,6 +1053,7 @@ namespace vcb {
 BucketScratch* bucket_scratch_new() { return new BucketScratch(); }
 void bucket_scratch_delete(BucketScratch* sc) { delete sc; }
 void bucket_scratch_status(BucketScratch* sc, unsigned* word) { sc->flat.status = word; }
+void bucket_scratch_lean(BucketScratch* sc, bool lean) { sc->lean = lean; }
 void bucket_scratch_bind(BucketScratch* sc, ScratchArena* a) { sc->bind(a); }
 
 size_t bucketed_dim_in(const tq_bucketed* h) { return h->dim_in; }

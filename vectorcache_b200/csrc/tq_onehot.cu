@@ -1202,7 +1202,7 @@ cudaError_t launch_onehot_buckets(const BucketScanArgs& b, long long nq, long lo
   a.slot_start = b.slot_start;
   a.bucket_size = b.bucket_size;
   a.append_count = b.append_count;
-  a.region = static_cast<uint32_t>(b.lists * b.k);
+  a.region = static_cast<uint32_t>(b.region);
   a.max_probe = b.max_probe;
   return launch_t<kBucket, 256>(a, sms / 2 * 2, stream);
 }

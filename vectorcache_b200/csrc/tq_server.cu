@@ -502,20 +502,33 @@ struct tq_server {
     vcb::BlockCache::get().trim();  // what it holds counts as free
     vcb::check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
     resident_bytes = total_b - free_b;  // indexes, kernels, context and the slots' buffers
-    // The largest scratch any admissible batch needs: full batches at the
-    // largest k and n_probe (and one- and two-query batches, which may take
-    // the batch-split scan).
+    // The scratch a full batch needs at the largest k and n_probe (and one- and
+    // two-query batches, which may take the batch-split scan) has to fit the budget;
+    // bucketed batches leave the one-hot scan and its larger regions where only that
+    // fits.
     sizer_flat.range_cap = kServingRangeVectors;
     sizer_bkt = vcb::bucket_scratch_new();
-    for (const Target& t : targets) {
-      for (size_t m : {max_batch, std::min<size_t>(max_batch, 2), size_t{1}}) {
-        max_need = std::max(max_need, batch_need(t, m, t.max_k, t.max_probe));
+    auto largest = [&](bool every_k) {
+      size_t need = 0;
+      for (const Target& t : targets) {
+        for (size_t m : {max_batch, std::min<size_t>(max_batch, 2), size_t{1}}) {
+          for (size_t k = every_k ? 1 : t.max_k; k <= t.max_k; ++k) need = std::max(need, batch_need(t, m, k, t.max_probe));
+        }
       }
-    }
-    if (budget <= resident_bytes || budget - resident_bytes < max_need) {
+      return need;
+    };
+    const size_t room = budget > resident_bytes ? budget - resident_bytes : 0;
+    const bool lean = largest(false) > room;
+    vcb::bucket_scratch_lean(sizer_bkt, lean);
+    for (auto& sl : slots) vcb::bucket_scratch_lean(sl->bkt, lean);
+    const size_t least = largest(false);
+    if (least > room || room == 0) {
       vcb::fail(TQ_ERR_OUT_OF_MEMORY, "the HBM budget does not hold the resident indexes plus the scratch of one "
-                                      "full batch (" + std::to_string(resident_bytes + max_need) + " bytes needed)");
+                                      "full batch (" + std::to_string(resident_bytes + least) + " bytes needed)");
     }
+    // The arena holds a batch of any admissible k (a k below an index's re-rank depth
+    // needs buffers that max_k may not).
+    max_need = largest(true);
     arena_bytes = std::min(budget - resident_bytes, max_slots * max_need);
     arena_bytes = arena_bytes / vcb::ScratchArena::kAlign * vcb::ScratchArena::kAlign;
     arena.reserve(arena_bytes);

@@ -21,6 +21,8 @@ BucketScratch* bucket_scratch_new();
 void bucket_scratch_delete(BucketScratch* sc);
 // The word (WaitStatus::word) that searches with sc set when a kernel gave up.
 void bucket_scratch_status(BucketScratch* sc, unsigned* word);
+// Lean searches keep the lookup scan and need the least scratch.
+void bucket_scratch_lean(BucketScratch* sc, bool lean);
 // Later reserves of every buffer of sc draw from a (nullptr: cudaMalloc).
 struct ScratchArena;
 void bucket_scratch_bind(BucketScratch* sc, ScratchArena* a);
