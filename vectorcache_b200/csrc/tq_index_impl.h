@@ -430,13 +430,20 @@ struct tq_index {
                      size_t k_eff, cudaStream_t s, vcb::FlatScratch sc) {
     if (nq == 0 || k_eff == 0) return;
     // Bound the scratch per pass: LUTs + candidate lists.
-    const size_t max_pass = 1 << 16;
-    for (size_t q0 = 0; q0 < nq; q0 += max_pass) {
-      const size_t m = std::min(max_pass, nq - q0);
-      prep_queries(d_q + q0 * dim, m, s, nullptr, sc);
+    constexpr size_t max_pass = 1 << 16;
+    for (size_t q0 = 0, m = 0; q0 < nq; q0 += m) {
+      m = std::min(max_pass, nq - q0);
+      // A pass that shrinks to bound the one-hot lists is planned again.
       vcb::OneHotPlan oh;
-      if (sc.onehot && vcb::plan_onehot(static_cast<long long>(n), static_cast<long long>(m), static_cast<int>(nbg),
-                                        static_cast<int>(bits), static_cast<int>(k_eff), sms, &oh)) {
+      bool onehot = sc.onehot != nullptr;
+      for (long long fit = 0; onehot && fit != static_cast<long long>(m);) {
+        if (fit) m = static_cast<size_t>(fit);
+        onehot = vcb::plan_onehot(static_cast<long long>(n), static_cast<long long>(m), static_cast<int>(nbg),
+                                  static_cast<int>(bits), static_cast<int>(k_eff), sms, &oh);
+        if (onehot) fit = vcb::onehot_pass(oh, static_cast<long long>(m));
+      }
+      prep_queries(d_q + q0 * dim, m, s, nullptr, sc);
+      if (onehot) {
         search_onehot(oh, m, k_eff, d_scores + q0 * k_eff, d_ids + q0 * k_eff, s, sc);
         continue;
       }
@@ -504,16 +511,13 @@ struct tq_index {
   // sample of the index, the scan above them, the merge of its lists.
   void search_onehot(const vcb::OneHotPlan& p, size_t m, size_t k_eff, float* d_scores, uint64_t* d_ids, cudaStream_t s,
                      vcb::FlatScratch sc) {
-    const size_t lists = 2 * static_cast<size_t>(p.n_ranges);
-    sc.cand_s->reserve(m * lists * p.list_len * 4);
-    sc.cand_i->reserve(m * lists * p.list_len * 4);
-    // The sample's scores and the scan's running lists share one region.
-    const size_t region = vcb::round_up(
-        std::max(vcb::onehot_list_bytes(p), vcb::onehot_sample_bytes(p, static_cast<long long>(m))), 256);
-    const size_t compact = p.compact ? m * nbg * 16 : 0;
-    sc.onehot->reserve(region + compact + m * 4);
-    uint8_t* compact_luts = sc.onehot->as<uint8_t>() + region;
-    float* floor = reinterpret_cast<float*>(compact_luts + compact);
+    // One block, so that a first search allocates once (cudaMalloc of 1 MiB and more
+    // takes 0.33 ms and up).
+    const vcb::OneHotScratch at = vcb::onehot_scratch(p, static_cast<long long>(m), static_cast<int>(nbg));
+    sc.onehot->reserve(at.bytes);
+    uint8_t* block = sc.onehot->as<uint8_t>();
+    uint8_t* compact_luts = block + at.compact;
+    float* floor = reinterpret_cast<float*>(block + at.floor);
     const float* qf = sc.qf->as<float>();
     vcb::OneHotArgs a{};
     a.codes = d_codes.as<uint32_t>();
@@ -525,11 +529,11 @@ struct tq_index {
     a.nbg = static_cast<int>(nbg);
     a.nq = static_cast<long long>(m);
     a.k = static_cast<int>(k_eff);
-    a.lists = sc.onehot->as<unsigned long long>();
-    a.cand_score = sc.cand_s->as<float>();
-    a.cand_id = sc.cand_i->as<uint32_t>();
+    a.lists = reinterpret_cast<unsigned long long*>(block);  // after the sample, in its place
+    a.cand_score = reinterpret_cast<float*>(block + at.cand_score);
+    a.cand_id = reinterpret_cast<uint32_t*>(block + at.cand_id);
     a.floor = floor;
-    a.dense = sc.onehot->as<float>();
+    a.dense = reinterpret_cast<float*>(block);
     if (p.compact) {
       launch(kPrep, s, "compact LUT kernel", [&] {
         return vcb::launch_compact_luts(a.luts, static_cast<long long>(m), static_cast<int>(nbg), compact_luts, s);
@@ -551,7 +555,7 @@ struct tq_index {
     mg.cand_score = a.cand_score;
     mg.cand_id = a.cand_id;
     mg.nq = static_cast<long long>(m);
-    mg.n_lists = static_cast<int>(lists);
+    mg.n_lists = 2 * p.n_ranges;
     mg.k = p.list_len;
     mg.k_out = static_cast<int>(k_eff);
     mg.out_score = d_scores;

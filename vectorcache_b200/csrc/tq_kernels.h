@@ -233,8 +233,17 @@ struct OneHotArgs {
 };
 // False when the batch belongs to the lookup scan.
 bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, OneHotPlan* plan);
-size_t onehot_list_bytes(const OneHotPlan& p);
-size_t onehot_sample_bytes(const OneHotPlan& p, long long nq);
+// Queries of one pass: what keeps its published lists within kOneHotListBytes and
+// its sample within 128 MiB (at least one full tile).
+constexpr size_t kOneHotListBytes = size_t{1} << 30;
+constexpr long long kOneHotMaxPass = 32768;
+long long onehot_pass(const OneHotPlan& p, long long nq);
+// Device scratch of a pass, one block: running lists and sample scores (one region),
+// published scores and ids, compact LUTs, floors.
+struct OneHotScratch {
+  size_t cand_score, cand_id, compact, floor, bytes;  // offsets; the region is first
+};
+OneHotScratch onehot_scratch(const OneHotPlan& p, long long nq, int nbg);
 // luts (nq x nbg x 32) -> out (nq x nbg x 16), the form a compact plan scans.
 cudaError_t launch_compact_luts(const uint8_t* luts, long long nq, int nbg, uint8_t* out, cudaStream_t stream);
 cudaError_t launch_onehot_sample(const OneHotArgs& a, const OneHotPlan& p, int sms, cudaStream_t stream);

@@ -1117,7 +1117,8 @@ bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, O
   // About n k / sample scores per query then pass them and cost the epilogue
   // some hundred clocks each per warp, which rows of few stages (768 clocks of
   // MMA each) do not hide: at least 8192 k / stages vectors, 1/64 of the index,
-  // at most 1/16 of it, 32768 vectors and 128 MiB of scores. (1000 queries x
+  // at most 1/16 of it, 32768 vectors and 128 MiB of scores, at least 1024 vectors
+  // (128 MiB at kOneHotMaxPass queries). (1000 queries x
   // 100k x 128, k = 10: scan + sample + selection 261 + 23 + 13 us with 1536
   // vectors, 188 + 35 + 25 us with the rule's 6144.)
   const int stage = bits == 3 ? Groups<true, kOne>::kStage : Groups<false, kOne>::kStage;
@@ -1134,9 +1135,25 @@ bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, O
   return true;
 }
 
-size_t onehot_list_bytes(const OneHotPlan& p) { return static_cast<size_t>(p.ctas) * p.tile_queries * p.cap * 8; }
-size_t onehot_sample_bytes(const OneHotPlan& p, long long nq) {
-  return static_cast<size_t>(nq) * p.sample_tiles * kPairVectors * 4;
+long long onehot_pass(const OneHotPlan& p, long long nq) {
+  const long long per_query = 2LL * p.n_ranges * p.list_len * 8;
+  const long long fit = static_cast<long long>(kOneHotListBytes) / per_query / kMaxN * kMaxN;
+  return std::min<long long>({nq, kOneHotMaxPass, std::max<long long>(fit, kMaxN)});
+}
+
+OneHotScratch onehot_scratch(const OneHotPlan& p, long long nq, int nbg) {
+  auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+  const size_t m = static_cast<size_t>(nq);
+  const size_t running = static_cast<size_t>(p.ctas) * p.tile_queries * p.cap * 8;
+  const size_t sample = m * p.sample_tiles * kPairVectors * 4;
+  const size_t lists = up(m * 2 * p.n_ranges * p.list_len * 4);
+  OneHotScratch s;
+  s.cand_score = up(std::max(running, sample));
+  s.cand_id = s.cand_score + lists;
+  s.compact = s.cand_id + lists;
+  s.floor = s.compact + (p.compact ? up(m * nbg * 16) : 0);
+  s.bytes = s.floor + m * 4;
+  return s;
 }
 
 cudaError_t launch_compact_luts(const uint8_t* luts, long long nq, int nbg, uint8_t* out, cudaStream_t stream) {
