@@ -487,7 +487,8 @@ int tq_multi_run_uncaptured(tq_multi* h, void* stream);
 /* Block until the last launch is done, on whichever stream it was queued.
  * TQ_ERR_CUDA also when a kernel of a launch gave up waiting (tq_index_synchronize). */
 int tq_multi_synchronize(tq_multi* h);
-/* Chosen configuration; tuned_ms receives up to *n_tuned candidate timings
+/* Chosen configuration; n_items counts the work items of the persistent launch and
+ * each batch that runs the single-index kernels as one; tuned_ms receives up to *n_tuned candidate timings
  * (on return *n_tuned = candidates timed). */
 int tq_multi_config(tq_multi* h, long long* range_vectors, int* ctas, size_t* n_items, size_t* smem_bytes,
                     double* tuned_ms, size_t* n_tuned);

@@ -13,12 +13,12 @@
 // id asc) top-k are those of the flat search, so results equal the per-index
 // search bit for bit.
 //
-// The autotuner times candidates on the planned workload itself (CUDA events,
-// one untimed and one timed run each), in three passes: the vector-range
-// length of a work item, the resident CTAs per SM, and how many of the
-// heaviest index batches run the single-index scan kernels (inside the same
-// graph) instead of the persistent launch, with that range length and with short
-// ranges for the rest; then it captures the graph.
+// The autotuner times candidates on the planned batch sizes with pseudo-random
+// queries (CUDA events, after an untimed run where kernels or scratch are new), in
+// three passes: the vector-range length of a work item, the resident CTAs per SM,
+// and how many of the heaviest index batches run the single-index scan kernels
+// (inside the same graph) instead of the persistent launch, with that range length
+// and with short ranges for the rest; then it captures the graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,6 +32,22 @@
 #include "tq_bucket.h"
 #include "tq_index_impl.h"
 #include "tq_kernels.h"
+
+namespace {
+
+// Planning queries: row r's values spread over [-1, 1) by a multiplicative hash. Not
+// zeros: every score would equal the threshold sample's and fill the one-hot scan's
+// lists, which no real query does and the lookup scan hardly feels.
+__global__ void fill_queries_kernel(float* __restrict__ q, unsigned long long n) {
+  const unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  unsigned long long h = (i + 1ull) * 0x9e3779b97f4a7c15ull;
+  h ^= h >> 32;
+  h *= 0xd6e8feb86659fd93ull;
+  q[i] = static_cast<float>(static_cast<int>(h >> 32)) * 4.656612873077393e-10f;
+}
+
+}  // namespace
 
 struct tq_multi {
   vcb::WaitStatus status;  // of the direct batches
@@ -288,18 +304,19 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
       h->d_q[i]->reserve(std::max<size_t>(nq[i], 1) * h->idx[i]->dim * 4);
       h->d_s[i]->reserve(std::max<size_t>(nq[i] * h->ke[i], 1) * 4);
       h->d_i[i]->reserve(std::max<size_t>(nq[i] * h->ke[i], 1) * 8);
-      vcb::check(cudaMemsetAsync(h->d_q[i]->get(), 0, std::max<size_t>(nq[i], 1) * h->idx[i]->dim * 4, h->stream),
-                 "cudaMemsetAsync");
+      const size_t values = std::max<size_t>(nq[i], 1) * h->idx[i]->dim;
+      fill_queries_kernel<<<static_cast<unsigned>((values + 255) / 256), 256, 0, h->stream>>>(h->d_q[i]->as<float>(),
+                                                                                              values);
+      vcb::check(cudaGetLastError(), "query fill kernel");
     }
-    // Autotuner, two passes over the planned workload itself: the item range
-    // length at the most resident CTAs, then the resident CTAs per SM at that
-    // length. Each candidate: one untimed run (grows scratch, loads kernels),
-    // one timed run (CUDA events).
+    // Autotuner: the item range length at the most resident CTAs, then the resident
+    // CTAs per SM at that length. Each candidate: one untimed run (grows scratch,
+    // loads kernels), one timed run (CUDA events).
     h->tuned_ms.clear();
     long long best_rv = 8192;
+    double best = -1.0;
     if (autotune) {
       const long long ranges[] = {4096, 8192, 16384, 32768};
-      double best = -1.0;
       for (long long rv : ranges) {
         h->build_items(rv);
         h->ctas = h->sms * std::max(1, vcb::multi_scan_ctas_per_sm(h->smem, h->any3));
@@ -316,7 +333,7 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
     const int per_sm = std::max(1, vcb::multi_scan_ctas_per_sm(h->smem, h->any3));
     int best_c = per_sm;
     if (autotune && per_sm > 1) {
-      double best = -1.0;
+      best = -1.0;
       for (int c = 1; c <= per_sm; ++c) {
         h->ctas = h->sms * c;
         const double ms = h->time_ms(1);
@@ -345,24 +362,25 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
         const int ps = std::max(1, vcb::multi_scan_ctas_per_sm(h->smem, h->any3));
         h->ctas = h->sms * std::min(best_c, ps);
       };
-      set_direct(0, best_rv);
-      double best = h->time_ms(3);
-      size_t best_d = 0;
+      size_t best_d = 0, best_tried = 0;
       long long best_d_rv = best_rv;
       // The range length above suits all batches; what is left of them may be a few
-      // light ones that it cuts into fewer items than SMs, so short ranges are tried
-      // too (eight indexes of 20k to 440k vectors: the launch left with the lightest,
+      // light ones that it cuts into fewer items than CTAs, so short ranges are tried
+      // then (eight indexes of 20k to 440k vectors: the launch left with the lightest,
       // 33 queries x 20,913, was five items of 613 us; four of them in short ranges
       // take 362 us, the whole search 2.64 -> 2.23 ms).
       constexpr long long kShortRange = 1024;
-      // The lightest of several batches always stays with the persistent launch.
-      const size_t most = m > 1 ? m - 1 : 1;
-      for (size_t d : {size_t{1}, size_t{2}, size_t{4}, size_t{8}, size_t{16}, most}) {
-        if (d > most) continue;
+      for (size_t d : {size_t{1}, size_t{2}, size_t{4}, size_t{8}, size_t{16}, m - 1, m}) {
+        if (d > m || d <= best_tried) continue;
+        best_tried = d;
         for (long long rv : {best_rv, kShortRange}) {
+          if (rv != best_rv && (h->items.empty() || h->items.size() >= static_cast<size_t>(h->ctas))) break;
           set_direct(d, rv);
           h->time_ms(1);
-          const double ms = h->time_ms(3);  // candidates differ by less than single runs do
+          double ms = h->time_ms(1);
+          // Candidates differ by less than single runs do: the median of three for those
+          // in reach.
+          if (ms < 1.2 * best) ms = h->time_ms(3);
           h->tuned_ms.push_back(ms);
           if (ms < best) {
             best = ms;
@@ -370,12 +388,16 @@ int tq_multi_plan(tq_multi* h, const size_t* nq, const size_t* k, int autotune) 
             best_d_rv = rv;
           }
         }
-        if (d == most) break;
       }
       set_direct(best_d, best_d_rv);
     }
     h->capture();
     h->status.check();  // the runs so far are complete
+    for (size_t i = 0; i < m; ++i) {
+      vcb::check(cudaMemsetAsync(h->d_q[i]->get(), 0, std::max<size_t>(nq[i], 1) * h->idx[i]->dim * 4, h->stream),
+                 "cudaMemsetAsync");
+    }
+    vcb::check(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
     h->planned = true;
   });
 }
@@ -434,7 +456,7 @@ int tq_multi_config(tq_multi* h, long long* range_vectors, int* ctas, size_t* n_
     require(h->planned, TQ_ERR_STATE, "plan() first");
     if (range_vectors) *range_vectors = h->range_vectors;
     if (ctas) *ctas = h->ctas;
-    if (n_items) *n_items = h->items.size();
+    if (n_items) *n_items = h->items.size() + h->n_direct;
     if (smem_bytes) *smem_bytes = h->smem;
     if (n_tuned) {
       const size_t cap = *n_tuned;
