@@ -50,7 +50,7 @@ const char* tq_version(void);
 
 /* Free the device memory that the library keeps for its own later allocations.
  * Blocks of 1 MiB and more of closed indexes and outgrown buffers stay with the
- * process, at most 2 GiB over all devices (the oldest are freed first; all are when
+ * process, at most 2 GiB over all devices (all are freed when
  * an allocation of the library fails or a server starts). A program that leaves the
  * GPU to another allocator or process calls this after closing its indexes. */
 int tq_trim(void);

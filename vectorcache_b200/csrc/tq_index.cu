@@ -92,9 +92,9 @@ void* BlockCache::take(size_t bytes, size_t* capacity, int* device) {
   if (bytes >= kMinBlock) {
     std::lock_guard<std::mutex> lock(mu_);
     size_t best = blocks_.size();
-    for (size_t i = 0; i < blocks_.size(); ++i) {  // the smallest that fits, at most a quarter larger
+    for (size_t i = 0; i < blocks_.size(); ++i) {  // the smallest that fits, at most a sixteenth larger
       const Block& b = blocks_[i];
-      if (b.device != *device || b.capacity < *capacity || b.capacity > *capacity + *capacity / 4) continue;
+      if (b.device != *device || b.capacity < *capacity || b.capacity > *capacity + *capacity / 16) continue;
       if (best == blocks_.size() || b.capacity < blocks_[best].capacity) best = i;
     }
     if (best < blocks_.size()) {
@@ -139,13 +139,14 @@ void BlockCache::give(void* ptr, size_t capacity, int device) noexcept {
     {
       std::lock_guard<std::mutex> lock(mu_);
       try {
-        blocks_.push_back({ptr, capacity, device});
+        blocks_.push_back({ptr, capacity, device, ++given_});
         total_ += capacity;
         kept = true;
         while (total_ > kLimit) {
-          out.push_back(blocks_.front().ptr);
-          total_ -= blocks_.front().capacity;
-          blocks_.erase(blocks_.begin());
+          const size_t i = victim();
+          out.push_back(blocks_[i].ptr);
+          total_ -= blocks_[i].capacity;
+          blocks_.erase(blocks_.begin() + static_cast<std::ptrdiff_t>(i));
         }
       } catch (...) {  // no host memory for the list: ptr is freed below
       }
@@ -154,6 +155,21 @@ void BlockCache::give(void* ptr, size_t capacity, int device) noexcept {
   }
   if (!kept) cudaFree(ptr);
   if (keep && prev != device) cudaSetDevice(prev);
+}
+
+size_t BlockCache::victim() const noexcept {
+  if (given_ - blocks_.front().given > kStale) return 0;
+  size_t best = 0;
+  bool fits = false;  // blocks_[best] makes room by itself
+  for (size_t i = 0; i < blocks_.size(); ++i) {
+    const bool enough = total_ - blocks_[i].capacity <= kLimit;
+    const bool smaller = blocks_[i].capacity < blocks_[best].capacity;
+    if (enough ? !fits || smaller : !fits && !smaller) {
+      best = i;
+      fits = enough;
+    }
+  }
+  return best;
 }
 
 void BlockCache::trim() noexcept {
