@@ -247,7 +247,7 @@ void do_add_device(tq_index* h, const float* d_x, size_t n, cudaStream_t s) {
   check_aligned(d_x, "vectors");
   if (h->prepared) {
     h->encode_append(d_x, n, s);
-    h->reserve_onehot();
+    h->reserve_scratch();
     return;
   }
   // Stage on the device until prepare(), like gpu::FlatIndex::add.
@@ -436,7 +436,7 @@ int tq_index_prepare(tq_index* h) {
     require(h->staged_n > 0, TQ_ERR_STATE, "prepare with empty index");
     vcb::DeviceGuard g(h->device);
     h->encode_append(h->d_staged.as<float>(), h->staged_n, h->stream);
-    h->reserve_onehot();
+    h->reserve_scratch();
     h->sync();
     h->staged_n = 0;
     h->d_staged.release();

@@ -395,19 +395,33 @@ struct tq_index {
     n += count;
   }
 
-  // Scratch of one-hot batches of up to 64 queries (about 30 MB), for indexes of 512 MiB
-  // of codes and more, while the encode kernels run: a first search of 16 queries over
-  // 10M x 768 waited 1.0 to 4.4 ms for cudaMalloc otherwise. Smaller indexes reserve it
-  // with the first search that needs it.
-  void reserve_onehot() {
+  // Sums and arrival counters of a batch-split scan of m queries.
+  size_t split_sums(const vcb::ScanPlan& plan, size_t m) const {
+    return m * static_cast<size_t>(plan.split_batches) * cap;
+  }
+  size_t split_counters(const vcb::ScanPlan& plan, size_t m) const {
+    return (m + plan.q_per_cta - 1) / plan.q_per_cta * ((n + vcb::kScanBlockVectors - 1) / vcb::kScanBlockVectors);
+  }
+
+  // Scratch of small batches, for indexes of 512 MiB of codes and more, while the encode
+  // kernels run: of one-hot batches of up to 64 queries (about 30 MB) and of one- and
+  // two-query split scans (24 MB at 1M x 1536). A first search of 16 queries over
+  // 10M x 768 waited 1.0 to 4.4 ms for cudaMalloc otherwise, one query over 1M x 1536
+  // 0.4 to 16 ms. Smaller indexes reserve it with the first search that needs it.
+  void reserve_scratch() {
     constexpr size_t kFromBytes = size_t{512} << 20;
-    vcb::OneHotPlan p;
-    if (d_onehot.get() || n * nbg < kFromBytes ||
-        !vcb::plan_onehot(static_cast<long long>(n), 64, static_cast<int>(nbg), static_cast<int>(bits), 64, sms, &p)) {
-      return;
-    }
+    if (n * nbg < kFromBytes) return;
+    const long long rows = static_cast<long long>(n);
+    const int groups = static_cast<int>(nbg), width = static_cast<int>(bits);
     try {
-      d_onehot.reserve(vcb::onehot_scratch(p, 64, static_cast<int>(nbg)).bytes);
+      vcb::OneHotPlan p;
+      if (!d_onehot.get() && vcb::plan_onehot(rows, 64, groups, width, 64, sms, &p)) {
+        d_onehot.reserve(vcb::onehot_scratch(p, 64, groups).bytes);
+      }
+      vcb::ScanPlan plan;
+      if (!d_partial.get() && vcb::plan_scan(rows, 2, groups, 10, sms, &plan, 0, width) && plan.split_batches > 1) {
+        d_partial.reserve((split_sums(plan, 2) + split_counters(plan, 2)) * 4);
+      }
     } catch (const std::exception&) {  // no room: the search that needs it reports it
       cudaGetLastError();
     }
@@ -502,9 +516,7 @@ struct tq_index {
       if (plan.split_batches > 1 && sc.partial) {
         // Batch sums, then one arrival counter per (query group, block),
         // zeroed for this launch.
-        const size_t sums = m * static_cast<size_t>(plan.split_batches) * cap;
-        const size_t counters = static_cast<size_t>((m + plan.q_per_cta - 1) / plan.q_per_cta) *
-                                ((n + vcb::kScanBlockVectors - 1) / vcb::kScanBlockVectors);
+        const size_t sums = split_sums(plan, m), counters = split_counters(plan, m);
         sc.partial->reserve((sums + counters) * 4);
         a.partial = sc.partial->as<uint32_t>();
         a.partial_stride = static_cast<long long>(cap);
