@@ -207,8 +207,9 @@ def test_probe_counts_per_query_decide_by_their_pairs(nb_queries, many):
 
 @pytest.mark.parametrize("n,nq,k", [
     (2048, 3, 1), (2048, 2, 32),   # one list: fewer candidates than lanes, as many
-    (16384, 1, 32),                # 256 candidates: the most that one warp merges
-    (16385, 2, 32), (18433, 1, 29),  # one list more
+    (16384, 1, 32), (16385, 2, 32), (18433, 1, 29),
+    (65536, 1, 8), (65537, 1, 8),  # 256 candidates: the most that one warp merges; one list more
+    (65536, 2, 9),                 # the first k of the CTA's merge
     (524288, 1, 1), (524289, 1, 1),
 ])
 @pytest.mark.parametrize("zeros", [False, True])

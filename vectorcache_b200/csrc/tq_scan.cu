@@ -96,6 +96,47 @@ struct RegTopK {
       if (better(cs, ci, thr_s, thr_i)) insert(cs, ci, k, lane);
     }
   }
+
+  // offer() for candidates with arbitrary ids (merging candidate lists).
+  __device__ __forceinline__ void offer_ids(const float (&sc)[8], const uint32_t (&id)[8], unsigned valid, int k,
+                                            int lane) {
+    unsigned pass = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if ((valid >> j & 1u) && better(sc[j], id[j], thr_s, thr_i)) pass |= 1u << j;
+    }
+    if (!(thr_s > -INFINITY)) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (pass >> j & 1u) mx = fmaxf(mx, sc[j]);
+      }
+      const float bound = warp_kth_largest(mx, k, lane);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if ((pass >> j & 1u) && sc[j] < bound) pass &= ~(1u << j);
+      }
+    }
+    unsigned any = __ballot_sync(full_mask(), pass != 0);
+    while (any) {
+      const int src = __ffs(any) - 1;
+      const int my_j = __ffs(pass) - 1;
+      float my_s = sc[0];
+      uint32_t my_i = id[0];
+#pragma unroll
+      for (int j = 1; j < 8; ++j) {
+        if (j == my_j) {
+          my_s = sc[j];
+          my_i = id[j];
+        }
+      }
+      const float cs = __shfl_sync(full_mask(), my_s, src);
+      const uint32_t ci = __shfl_sync(full_mask(), my_i, src);
+      if (lane == src) pass &= pass - 1;
+      any = __ballot_sync(full_mask(), pass != 0);
+      if (better(cs, ci, thr_s, thr_i)) insert(cs, ci, k, lane);
+    }
+  }
 };
 
 // Staged code stream: group rows per slot, and slots per warp by queries per
@@ -560,75 +601,6 @@ __device__ __forceinline__ uint32_t score_key(float s) {
 // ranges): 150 -> 20 us against sorting 1024 candidates at a time.
 constexpr int kMergeRank = 512;
 constexpr int kMergeDirect = 64;  // candidates that need no bound
-constexpr int kMergeOneWarp = 256;  // candidates that one warp merges by itself (k <= 32)
-
-// The best kout of at most kMergeOneWarp candidates, kout <= 32, by one warp: as in
-// merge_kernel, the lanes' best scores giving the bound, but without barriers, which cost
-// more than the other warps bring here: one query over 50k x 128, k = 2 to 5 (50 to 125
-// candidates) 29.0 us by the whole CTA, 27.0 by one warp; 200k x 128 3-bit, k = 1 29.4 and
-// 26.3. (A kernel of one-warp CTAs of its own: no faster.)
-// buf_s, s_rank: kMergeOneWarp entries.
-__device__ __forceinline__ void merge_one_warp(const MergeArgs& a, long long qi, int total, const float* cs,
-                                               const uint32_t* ci, float* buf_s, unsigned long long* s_rank, int lane) {
-  constexpr int kEach = kMergeOneWarp / kWarp;
-  const int kout = a.k_out;
-  float sc[kEach];
-  uint32_t id[kEach];
-#pragma unroll
-  for (int u = 0; u < kEach; ++u) {
-    const int at = u * kWarp + lane;
-    sc[u] = at < total ? cs[at] : -INFINITY;
-    id[u] = at < total ? ci[at] : 0u;
-  }
-  uint32_t bound = 0u;
-#pragma unroll
-  for (int u = 0; u < kEach; ++u) {
-    if (sc[u] > -INFINITY) bound = max(bound, score_key(sc[u]));
-  }
-#pragma unroll
-  for (int size = 2; size <= kWarp; size <<= 1) {
-#pragma unroll
-    for (int step = size >> 1; step > 0; step >>= 1) {
-      const uint32_t o = __shfl_xor_sync(full_mask(), bound, step);
-      const bool lower = (lane & step) == 0, desc = (lane & size) == 0;
-      bound = lower == desc ? max(bound, o) : min(bound, o);
-    }
-  }
-  bound = max(1u, __shfl_sync(full_mask(), bound, kout - 1));
-  int n = 0;
-#pragma unroll
-  for (int u = 0; u < kEach; ++u) {
-    const uint32_t key = score_key(sc[u]);
-    const bool take = sc[u] > -INFINITY && key >= bound;
-    const unsigned votes = __ballot_sync(full_mask(), take);
-    if (take) {
-      const int at = n + __popc(votes & ((1u << lane) - 1u));
-      buf_s[at] = sc[u];
-      s_rank[at] = (static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(~id[u]);
-    }
-    n += __popc(votes);
-  }
-  const int padded = (n + 7) / 8 * 8;  // the padding ranks behind everything
-  if (lane < padded - n) s_rank[n + lane] = 0ull;
-  __syncwarp();
-  for (int t = lane; t < n; t += kWarp) {
-    const unsigned long long key = s_rank[t];
-    int rank = 0;
-    for (int j = 0; j < padded; j += 8) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u) rank += s_rank[j + u] >= key + (j + u < t ? 0ull : 1ull) ? 1 : 0;
-    }
-    if (rank < kout) {
-      a.out_score[qi * kout + rank] = buf_s[t];
-      a.out_id[qi * kout + rank] = static_cast<uint64_t>(static_cast<uint32_t>(~static_cast<uint32_t>(key)));
-    }
-  }
-  if (lane >= n && lane < kout) {
-    a.out_score[qi * kout + lane] = 0.f;
-    a.out_id[qi * kout + lane] = a.pad_id;
-  }
-}
-
 __global__ void __launch_bounds__(kMergeThreads) merge_kernel(MergeArgs a) {
   __shared__ float buf_s[kMergeCap];
   __shared__ uint32_t buf_i[kMergeCap];
@@ -646,10 +618,6 @@ __global__ void __launch_bounds__(kMergeThreads) merge_kernel(MergeArgs a) {
   const float* cs = a.cand_score + qi * stride;
   const uint32_t* ci = a.cand_id + qi * stride;
   const int kout = a.k_out;
-  if (total <= kMergeOneWarp && kout <= kWarp) {
-    if (tid < kWarp) merge_one_warp(a, qi, static_cast<int>(total), cs, ci, buf_s, s_rank, lane);
-    return;
-  }
   if (tid == 0) n_new = 0;
   uint32_t bound = 1u;  // every score above -inf
   float v[kAhead];
@@ -821,6 +789,40 @@ __global__ void __launch_bounds__(kMergeThreads) merge_kernel(MergeArgs a) {
     const bool have = t < nbest;
     a.out_score[qi * kout + t] = have ? best_s[t] : 0.f;
     a.out_id[qi * kout + t] = have ? static_cast<uint64_t>(best_i[t]) : a.pad_id;
+  }
+}
+
+// Few results of few candidates (lists only): one warp per query, insertions into a
+// register top-k. merge_kernel's bound, ranks and barriers pay from more of them on.
+// Kernel times, merge_kernel / here: one query over 200k x 128, k = 1 (98 candidates)
+// 4.4 / 2.4 us; over 50k x 128, k = 3 (75) 4.2 / 2.9; over 100k x 64, k = 5 (245) 4.5 / 3.2;
+// a search is 2 us longer or shorter by it (one query over 50k x 128, k = 3 29.7 / 27.7).
+constexpr int kMergeFew = 256;  // candidates
+constexpr int kMergeFewK = 8;   // results
+__global__ void __launch_bounds__(kWarp) merge_few_kernel(MergeArgs a) {
+  const int lane = static_cast<int>(threadIdx.x), kout = a.k_out, total = a.n_lists * a.k;
+  const long long qi = blockIdx.x;
+  const long long first = qi * static_cast<long long>(a.list_stride ? a.list_stride : a.n_lists) * a.k;
+  float sc[8];
+  uint32_t id[8];
+  unsigned ok = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int at = lane * 8 + j;
+    sc[j] = -INFINITY;
+    id[j] = 0xffffffffu;
+    if (at < total) {
+      sc[j] = a.cand_score[first + at];
+      id[j] = a.cand_id[first + at];
+      if (sc[j] > -INFINITY) ok |= 1u << j;
+    }
+  }
+  RegTopK top;
+  top.offer_ids(sc, id, ok, kout, lane);
+  if (lane < kout) {
+    const bool have = top.s > -INFINITY;
+    a.out_score[qi * kout + lane] = have ? top.s : 0.f;
+    a.out_id[qi * kout + lane] = have ? static_cast<uint64_t>(top.i) : a.pad_id;
   }
 }
 
@@ -1084,6 +1086,10 @@ cudaError_t launch_scan(const ScanArgs& a, const ScanPlan& plan, cudaStream_t st
 
 cudaError_t launch_merge(const MergeArgs& a, cudaStream_t stream) {
   if (a.nq == 0 || a.k_out == 0) return cudaSuccess;
+  if (!a.entry_count && a.k_out <= kMergeFewK && static_cast<long long>(a.n_lists) * a.k <= kMergeFew) {
+    merge_few_kernel<<<static_cast<unsigned>(a.nq), kWarp, 0, stream>>>(a);
+    return cudaGetLastError();
+  }
   merge_kernel<<<static_cast<unsigned>(a.nq), kMergeThreads, 0, stream>>>(a);
   return cudaGetLastError();
 }
