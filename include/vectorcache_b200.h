@@ -186,8 +186,8 @@ int tq_index_dense_scores(tq_index* h, const float* queries, size_t nq, uint32_t
 int tq_index_replay_count(const tq_index* h, uint64_t* count);
 
 /* The lookup scan's plan for a search of nq queries with this k, which batches
- * that the tensor cores take (tq_onehot.cu: above 64 queries over 8,192 vectors
- * and more, smaller ones by an estimate) do not run: queries per
+ * that the tensor cores take (tq_onehot.cu: by an estimate of both scans, from
+ * 8,192 vectors on) do not run: queries per
  * CTA, vector ranges (one CTA per query group and range), vectors per range
  * (a multiple of the 2048-vector scan block), and the number of 256-group
  * batches a one- or two-query scan splits into (1: no split), and the

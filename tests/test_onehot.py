@@ -1,9 +1,8 @@
 """Batches of queries on the tensor cores (tq_onehot.cu) against the CPU oracle,
 bit for bit: ids and scores of the top k at the edges of its tiles (256 vectors,
 32-query steps up to 192, 8 byte groups per stage, 256 per flush batch) and of
-its lists (k up to 64, up to 256), with equal scores across tiles. Batches above
-64 queries always run there; smaller ones by an estimate (k > 32 from three
-queries on). Bucketed passes of at least 16 pairs per bucket against passes
+its lists (k up to 64, up to 256), with equal scores across tiles. Which batches
+run there is an estimate (k > 32 from three queries on nearly always). Bucketed passes of at least 16 pairs per bucket against passes
 small enough for the lookup scan."""
 import numpy as np
 import pytest
@@ -225,3 +224,15 @@ def test_merge_of_few_candidates(oracle, n, nq, k, zeros):
     assert np.array_equal(res.ids, want_i)
     assert np.array_equal(res.scores.view(np.uint32), want_s.view(np.uint32))
     idx.close()
+
+
+@pytest.mark.parametrize("dim,bits,n,nq,k", [
+    (24, 2, 40001, 200, 1),      # 6 byte groups, one vector in the last tile, k = 1
+    (64, 3, 50000, 130, 3),
+    (8, 4, 100000, 66, 32),
+    (8, 4, 8192, 66, 1),         # the lookup scan: the smallest batch and k above 64 queries
+    (64, 3, 16384, 66, 3),
+    (768, 2, 8192, 600, 1),
+])
+def test_batches_above_64_queries_equal_the_oracle(oracle, dim, bits, n, nq, k):
+    check(oracle, dim, bits, n, nq, k)

@@ -1073,13 +1073,26 @@ int choose_ranges(long long q_tiles, long long tiles, int pairs) {
 // 20k x 768 4-bit 4 queries 125 / 85; one query of k = 100 over 1M x 1536 551 / 1137,
 // of k = 33 over 3M x 384 398 / 896, two of k = 48 over 8,192 x 128 58 / 39.
 bool onehot_pays(long long n, long long nq, int nbg, int bits, int k, int sms) {
-  // Above 64 queries here everywhere: the smallest indexes are launches on both sides
-  // (lookups / here, 65 queries of k = 10: 8,192 x 64 4-bit 47.6 / 43.5 us, 3-bit
-  // 45.6 / 43.2, 8,192 x 128 3-bit 48.1 / 48.6, 32,768 x 64 3-bit 48.6 / 49.0; 96 to 512
-  // queries over 8k to 100k vectors of 64 to 1536 dims 0.98 to 19.8 times).
-  if (nq > Config<kSmall>::kCols) return true;
   const long long pairs = sms / 2, tiles = (n + kPairVectors - 1) / kPairVectors;
   const double blocks = static_cast<double>((n + kScanBlockVectors - 1) / kScanBlockVectors);
+  if (nq > Config<kSmall>::kCols) {
+    if (k > 32) return true;
+    // Whole searches, fitted to 4,536 of them (66 to 600 queries, k 1 to 32, 8k to 100k
+    // vectors of 8 to 768 dims): the side it picks is 0.4 % above the faster one on
+    // average, more than 10 % in 68. Small indexes are launches on both sides, and the
+    // lookups' grow with k: lookups / here, 128 queries over 8,192 x 64 3-bit, k = 1
+    // 31.3 / 45.6 us, k = 5 34.4 / 47.3; 66 over 16,384 x 64 3-bit, k = 3 33.4 / 46.8.
+    const long long q_tiles = (nq + kMaxN - 1) / kMaxN;
+    const double share = static_cast<double>(((nq + q_tiles - 1) / q_tiles + 31) / 32 * 32) / kMaxN;
+    const double waves = std::max(0.0, static_cast<double>((nq + 3) / 4) * blocks / (2.0 * sms) - 0.5);
+    const double stages = static_cast<double>((nbg + (bits == 3 ? 15 : 7)) / (bits == 3 ? 16 : 8));
+    const double lookups = 22.6 + nbg * (bits == 3 ? 0.128 : 0.226) +
+                           waves * (nbg * (bits == 3 ? 0.151 : 0.259) + 10.2 + 1.6 * k) + 1.9 * k + 0.106 * blocks;
+    const double here = 36.7 + (bits == 3 ? 4.1 : 0.0) +
+                        static_cast<double>((q_tiles * tiles + pairs - 1) / pairs) * share * (0.374 * stages + 3.14) +
+                        0.085 * k + 0.019 * static_cast<double>(nq) + 0.72 * stages;
+    return lookups > here;
+  }
   const double stages = static_cast<double>((nbg + (bits == 3 ? 31 : 15)) / (bits == 3 ? 32 : 16));
   const double scan = static_cast<double>((tiles + pairs - 1) / pairs) * stages * (bits == 3 ? 0.56 : 0.43);
   const double here = 25.0 + scan;
