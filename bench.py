@@ -662,6 +662,7 @@ def run_ours(args, world, rank, local):
     for v in variants:
         v.pop("_top", None)
 
+    rl = scan_roofline(prof, args, nbg, achieved, peak, peak_kind)
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": "queries/s", "n_gpus": world, "steps": args.steps,
@@ -675,7 +676,7 @@ def run_ours(args, world, rank, local):
                 "recall_queries": nr, "l2": "inputs larger than L2 (codes %.0f MB per shard)"
                                            % (args.n * (nbg + 4) / 1e6),
                 "parallelism": f"shard{world}" if world > 1 else "single",
-                "scan_plan": plan,
+                "scan_plan": plan if rl["kernel"] == "scan_kernel" else None,
                 "encode_vectors_per_s": encode_vps, "prepare_ms": prepare_ms,
                 "kernel_ms_per_step": {"prep": prof["prep_ms"] / args.steps, "scan": prof["scan_ms"] / args.steps,
                                        "merge": prof["merge_ms"] / args.steps},
@@ -685,7 +686,7 @@ def run_ours(args, world, rank, local):
                                     "peak": peak, "frac": encode_bytes / (encode_kernels_ms / 1e3) / 1e9 / peak},
                 "latency_ms": latency,
             },
-            "roofline": {**scan_roofline(prof, args, nbg, achieved, peak, peak_kind), "traffic": tr,
+            "roofline": {**rl, "traffic": tr,
                          "bytes_per_launch": bytes_per_launch, "ms_per_launch": scan_ms_avg,
                          "share_of_kernel_time": prof["scan_ms"] / total_kernel_ms if total_kernel_ms else None,
                          "nibble_lookups_per_s": lookups * args.steps / (prof["scan_ms"] / 1e3)
