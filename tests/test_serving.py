@@ -219,3 +219,18 @@ def test_a_tight_budget_serves_with_less_scratch(indexes):
     assert np.array_equal(got[1], want.ids)
     assert np.array_equal(got[0].view(np.uint32), want.scores.view(np.uint32))
     srv.close()
+
+
+def test_served_flat_batches_in_passes_of_a_tile(indexes):
+    # Above 192 queries a served flat batch runs as even passes on the tensor cores.
+    flat, _, db, _ = indexes
+    srv = vcb.Server(max_slots=2, max_batch=600)
+    target = srv.add_flat(flat, 40)
+    srv.start()
+    for nq, k in ((70, 10), (193, 40), (600, 10), (577, 33)):
+        q = db[:nq] + 0.25
+        s, i, _ = srv.submit(target, q, k).wait()
+        want = flat.search(q, k)
+        assert np.array_equal(i, want.ids), nq
+        assert np.array_equal(s.view(np.uint32), want.scores.view(np.uint32)), nq
+    srv.close()

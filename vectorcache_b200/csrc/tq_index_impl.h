@@ -201,7 +201,7 @@ struct FlatScratch {
   DeviceBuffer* cand_s;
   DeviceBuffer* cand_i;
   DeviceBuffer* partial = nullptr;  // nullptr: the scan does not split
-  long long range_cap = 0;          // > 0: at most this many vectors per scan CTA
+  long long range_cap = 0;          // > 0: at most this many vectors per scan CTA, one query tile per one-hot launch
   DeviceBuffer* onehot = nullptr;   // nullptr: batches stay on the lookup scan
   unsigned* status = nullptr;       // WaitStatus::word of the search's owner
 };
@@ -211,9 +211,8 @@ struct FlatScratchStore {
   DeviceBuffer luts, qf, cand_s, cand_i, partial, onehot;
   long long range_cap = 0;  // see FlatScratch::range_cap
   unsigned* status = nullptr;
-  // Searches that bound a CTA's vectors (the server's) keep the lookup scan:
-  // the one-hot kernel holds its SMs for the whole search.
-  FlatScratch ref() { return {&luts, &qf, &cand_s, &cand_i, &partial, range_cap, range_cap > 0 ? nullptr : &onehot, status}; }
+  bool lean = false;  // the lookup scan alone
+  FlatScratch ref() { return {&luts, &qf, &cand_s, &cand_i, &partial, range_cap, lean ? nullptr : &onehot, status}; }
   void bind(ScratchArena* a) {
     for (DeviceBuffer* b : {&luts, &qf, &cand_s, &cand_i, &partial, &onehot}) b->bind(a);
   }
@@ -481,6 +480,11 @@ struct tq_index {
         onehot = vcb::plan_onehot(static_cast<long long>(n), static_cast<long long>(m), static_cast<int>(nbg),
                                   static_cast<int>(bits), static_cast<int>(k_eff), sms, &oh);
         if (onehot) fit = vcb::onehot_pass(oh, static_cast<long long>(m));
+        if (onehot && sc.range_cap > 0) {  // evenly: no small last pass with a plan of its own
+          const long long left = static_cast<long long>(m);
+          const long long passes = (left + vcb::kOneHotServedPass - 1) / vcb::kOneHotServedPass;
+          fit = std::min(fit, (left + passes - 1) / passes);
+        }
       }
       prep_queries(d_q + q0 * dim, m, s, nullptr, sc);
       if (onehot) {

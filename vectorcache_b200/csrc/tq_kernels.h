@@ -237,6 +237,13 @@ bool plan_onehot(long long n, long long nq, int nbg, int bits, int k, int sms, O
 // its sample within 128 MiB (at least one full tile).
 constexpr size_t kOneHotListBytes = size_t{1} << 30;
 constexpr long long kOneHotMaxPass = 32768;
+// Searches that bound a CTA's work (the server's): the kernel holds its SMs until it
+// ends, so a launch takes one tile of queries (a few ms over 10M x 768 3-bit) and other
+// streams' kernels get in between. Bursts of 1 to 256 queries, 30 % of them over 10M x
+// 768 3-bit, the others bucketed, lookup scan / here: at 6,000 q/s bucketed p99 100 / 7.0
+// ms, flat p99 309 / 10 ms; 15,000 q/s offered, 7,662 / 16,745 served. 80 % flat at
+// 12,000 q/s: bucketed p99 3937 / 12.3 ms (13.4 with all queries in one launch).
+constexpr long long kOneHotServedPass = 192;
 long long onehot_pass(const OneHotPlan& p, long long nq);
 // Device scratch of a pass, one block: running lists and sample scores (one region),
 // published scores and ids, compact LUTs, floors.

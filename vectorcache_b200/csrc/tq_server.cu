@@ -44,9 +44,9 @@
 
 namespace {
 
-// Vectors per scan CTA of a served flat search: a 10M x 768 3-bit scan of 128
-// queries then runs in CTAs of a few ms, so bucketed batches on the
-// high-priority stream wait at most that long for an SM.
+// Vectors per lookup-scan CTA of a served flat search, and with it one query tile per
+// one-hot launch: flat searches then run in CTAs (launches) of a few ms, so bucketed
+// batches on the high-priority stream wait about that long for an SM.
 constexpr long long kServingRangeVectors = 65536;
 
 int64_t now_ns() {
@@ -168,9 +168,11 @@ struct tq_server {
   vcb::ScratchArena sizer;            // measure-mode arena of the dry runs
   vcb::FlatScratchStore sizer_flat;   // scratch the dry runs size
   vcb::BucketScratch* sizer_bkt = nullptr;
+  bool all_lean = false;              // the budget holds lean batches only
   uint64_t memory_waits = 0;          // batches that waited for arena memory
   uint64_t blocked_head = 0;          // id of the request heading a waiting batch (0: none)
   size_t blocked_nq = 0, blocked_need = 0;
+  bool blocked_lean = false;
 
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
@@ -204,9 +206,13 @@ struct tq_server {
   }
 
   // Exact scratch bytes of a batch: the same host code with no device work,
-  // its scratch buffers drawing placeholder pieces from a measuring arena.
-  size_t batch_need(const Target& t, size_t nq, size_t k, size_t n_probe) {
+  // its scratch buffers drawing placeholder pieces from a measuring arena. Lean
+  // batches keep the lookup scan: bucketed ones need the least then, and flat ones
+  // what they always did.
+  size_t batch_need(const Target& t, size_t nq, size_t k, size_t n_probe, bool lean) {
     sizer.reset(nullptr, 0, true);
+    sizer_flat.lean = lean;
+    vcb::bucket_scratch_lean(sizer_bkt, lean);
     sizer_flat.bind(&sizer);
     vcb::bucket_scratch_bind(sizer_bkt, &sizer);
     struct DryRun {
@@ -215,6 +221,15 @@ struct tq_server {
     } dry;
     run_search(t, nullptr, nq, k, n_probe, nullptr, nullptr, nullptr, sizer_flat, *sizer_bkt);
     return sizer.used;
+  }
+
+  // What admission takes for a batch: lean where the arena holds only that.
+  size_t admitted_need(const Target& t, size_t nq, size_t k, size_t n_probe, bool* lean) {
+    *lean = all_lean;
+    const size_t need = batch_need(t, nq, k, n_probe, all_lean);
+    if (all_lean || need <= arena_bytes) return need;
+    *lean = true;
+    return batch_need(t, nq, k, n_probe, true);
   }
 
   void stop() {
@@ -320,11 +335,13 @@ struct tq_server {
     Request* r0 = b.front();
     const Target& t = targets[r0->target];
     size_t need = 0;
+    bool lean = false;
     if (blocked_head == r0->id && blocked_nq == nq) {
       need = blocked_need;  // sized while it waited
+      lean = blocked_lean;
     } else {
       try {
-        need = batch_need(t, nq, r0->k, r0->n_probe);
+        need = admitted_need(t, nq, r0->k, r0->n_probe, &lean);
       } catch (const std::exception& ex) {
         unqueue(b);
         fail_batch(b, TQ_ERR_CUDA, ex.what());
@@ -336,7 +353,7 @@ struct tq_server {
       b.resize(1);
       nq = r0->nq;
       try {
-        need = batch_need(t, nq, r0->k, r0->n_probe);
+        need = admitted_need(t, nq, r0->k, r0->n_probe, &lean);
       } catch (const std::exception& ex) {
         unqueue(b);
         fail_batch(b, TQ_ERR_CUDA, ex.what());
@@ -356,6 +373,7 @@ struct tq_server {
       blocked_head = r0->id;
       blocked_nq = nq;
       blocked_need = need;
+      blocked_lean = lean;
       return false;
     }
     blocked_head = 0;
@@ -366,6 +384,8 @@ struct tq_server {
     sl.region.reset(static_cast<unsigned char*>(arena.get()) + off, need, false);
     sl.flat.bind(&sl.region);
     vcb::bucket_scratch_bind(sl.bkt, &sl.region);
+    sl.flat.lean = lean;
+    vcb::bucket_scratch_lean(sl.bkt, lean);
     arena_peak = std::max(arena_peak, pool.used());
     try {
       launch(sl);
@@ -504,31 +524,32 @@ struct tq_server {
     resident_bytes = total_b - free_b;  // indexes, kernels, context and the slots' buffers
     // The scratch a full batch needs at the largest k and n_probe (and one- and
     // two-query batches, which may take the batch-split scan) has to fit the budget;
-    // bucketed batches leave the one-hot scan and its larger regions where only that
-    // fits.
+    // batches are lean where only that fits.
     sizer_flat.range_cap = kServingRangeVectors;
     sizer_bkt = vcb::bucket_scratch_new();
-    auto largest = [&](bool every_k) {
+    auto largest = [&](bool lean, bool every_k) {
       size_t need = 0;
       for (const Target& t : targets) {
-        for (size_t m : {max_batch, std::min<size_t>(max_batch, 2), size_t{1}}) {
-          for (size_t k = every_k ? 1 : t.max_k; k <= t.max_k; ++k) need = std::max(need, batch_need(t, m, k, t.max_probe));
+        for (size_t m : {max_batch, std::min<size_t>(max_batch, 192), std::min<size_t>(max_batch, 64),
+                         std::min<size_t>(max_batch, 2), size_t{1}}) {
+          for (size_t k = every_k ? 1 : t.max_k; k <= t.max_k; ++k) {
+            need = std::max(need, batch_need(t, m, k, t.max_probe, lean));
+          }
         }
       }
       return need;
     };
     const size_t room = budget > resident_bytes ? budget - resident_bytes : 0;
-    const bool lean = largest(false) > room;
-    vcb::bucket_scratch_lean(sizer_bkt, lean);
-    for (auto& sl : slots) vcb::bucket_scratch_lean(sl->bkt, lean);
-    const size_t least = largest(false);
+    const size_t roomy = largest(false, false), leanest = largest(true, false);
+    all_lean = roomy > room && leanest <= room;
+    const size_t least = std::min(roomy, leanest);
     if (least > room || room == 0) {
       vcb::fail(TQ_ERR_OUT_OF_MEMORY, "the HBM budget does not hold the resident indexes plus the scratch of one "
                                       "full batch (" + std::to_string(resident_bytes + least) + " bytes needed)");
     }
     // The arena holds a batch of any admissible k (a k below an index's re-rank depth
     // needs buffers that max_k may not).
-    max_need = largest(true);
+    max_need = largest(all_lean, true);
     arena_bytes = std::min(budget - resident_bytes, max_slots * max_need);
     arena_bytes = arena_bytes / vcb::ScratchArena::kAlign * vcb::ScratchArena::kAlign;
     arena.reserve(arena_bytes);
@@ -711,7 +732,8 @@ int tq_server_batch_bytes(tq_server* h, int target, size_t nq, size_t k, size_t 
     require(k >= 1 && k <= t.max_k, TQ_ERR_INVALID_ARGUMENT, "k must be in [1, max_k of the index]");
     vcb::DeviceGuard g(h->device);
     std::lock_guard<std::mutex> lk(h->mu);
-    *bytes = h->batch_need(t, nq, k, t.flat ? 0 : (n_probe ? n_probe : t.max_probe));
+    bool lean = false;
+    *bytes = h->admitted_need(t, nq, k, t.flat ? 0 : (n_probe ? n_probe : t.max_probe), &lean);
   });
 }
 
