@@ -52,7 +52,8 @@ const char* tq_version(void);
  * Blocks of 1 MiB and more of closed indexes and outgrown buffers stay with the
  * process, at most 2 GiB over all devices (all are freed when
  * an allocation of the library fails or a server starts). A program that leaves the
- * GPU to another allocator or process calls this after closing its indexes. */
+ * GPU to another allocator or process calls this after closing its indexes (kept
+ * blocks do not count in a running server's budget). */
 int tq_trim(void);
 
 /* ---- host-side tables (same values as the reference's setup code) -------- */

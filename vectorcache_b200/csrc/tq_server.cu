@@ -465,7 +465,7 @@ struct tq_server {
     std::normal_distribution<float> nd;
     for (float& v : warm) v = nd(rng);
     {
-      // Full-size and two-query searches per index with throwaway scratch:
+      // Full-size and small searches per index with throwaway scratch:
       // kernels are loaded on their first launch, and that device memory is
       // resident, not part of the scratch arena.
       vcb::DeviceBuffer q, sc_s, sc_i;
@@ -482,11 +482,14 @@ struct tq_server {
       vcb::check(cudaMemcpy(q.get(), warm.data(), m * max_dim * 4, cudaMemcpyHostToDevice), "H2D");
       for (const Target& t : targets) {
         if (t.flat) {
-          t.flat->search_device(q.as<float>(), m, t.max_k, sc_s.as<float>(), sc_i.as<uint64_t>(),
-                                std::min(t.max_k, t.flat->n), nullptr, fs.ref());
-          // one- and two-query searches may take the batch-split scan kernels
-          t.flat->search_device(q.as<float>(), std::min<size_t>(m, 2), t.max_k, sc_s.as<float>(),
-                                sc_i.as<uint64_t>(), std::min(t.max_k, t.flat->n), nullptr, fs.ref());
+          // Up to 64 queries take other one-hot kernels, one and two may take the
+          // batch-split scan; the list kernels follow k (to 32, to 64, above).
+          for (size_t nq : {m, std::min<size_t>(m, 64), std::min<size_t>(m, 2)}) {
+            for (size_t k : {t.max_k, std::min<size_t>(t.max_k, 64), std::min<size_t>(t.max_k, 32)}) {
+              t.flat->search_device(q.as<float>(), nq, k, sc_s.as<float>(), sc_i.as<uint64_t>(),
+                                    std::min(k, t.flat->n), nullptr, fs.ref());
+            }
+          }
         } else {
           const vcb::LearnedProbe lp{t.mlp, t.coverage, t.min_conf};
           vcb::bucketed_search_with(t.bkt, q.as<float>(), m, t.max_k, t.max_probe, t.mlp ? &lp : nullptr,
@@ -518,10 +521,15 @@ struct tq_server {
       slots.push_back(std::move(sl));
     }
     slot_bytes = max_batch * (max_dim * 4 + max_k * 12);
-    size_t free_b = 0, total_b = 0;
-    vcb::BlockCache::get().trim();  // what it holds counts as free
-    vcb::check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-    resident_bytes = total_b - free_b;  // indexes, kernels, context and the slots' buffers
+    size_t room = 0;
+    auto measure = [&] {
+      size_t free_b = 0, total_b = 0;
+      vcb::BlockCache::get().trim();  // what it holds counts as free
+      vcb::check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+      resident_bytes = total_b - free_b;  // indexes, kernels, context and the slots' buffers
+      room = budget > resident_bytes ? budget - resident_bytes : 0;
+    };
+    measure();
     // The scratch a full batch needs at the largest k and n_probe (and one- and
     // two-query batches, which may take the batch-split scan) has to fit the budget;
     // batches are lean where only that fits.
@@ -539,8 +547,16 @@ struct tq_server {
       }
       return need;
     };
-    const size_t room = budget > resident_bytes ? budget - resident_bytes : 0;
     const size_t roomy = largest(false, false), leanest = largest(true, false);
+    if (std::min(roomy, leanest) > room) {
+      // The indexes' own scratch of small batches (reserve_scratch), which serving does not use.
+      for (const Target& t : targets) {
+        if (!t.flat) continue;
+        t.flat->d_onehot.release();
+        t.flat->d_partial.release();
+      }
+      measure();
+    }
     all_lean = roomy > room && leanest <= room;
     const size_t least = std::min(roomy, leanest);
     if (least > room || room == 0) {
