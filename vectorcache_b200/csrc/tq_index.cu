@@ -122,17 +122,17 @@ void* BlockCache::take(size_t bytes, size_t* capacity, int* device) {
 // ends the capture with an error, whichever thread it runs on; cudaFree is refused by a
 // global-mode capture only. That a free waits was measured with 256 bytes, 512 KiB and
 // 8 MiB behind 1.7 s of queued products.
-static bool wait_for_device() {
+bool BlockCache::wait_for_device() noexcept {
   void* p = nullptr;
   return cudaMalloc(&p, 256) == cudaSuccess && cudaFree(p) == cudaSuccess;
 }
 
-void BlockCache::give(void* ptr, size_t capacity, int device) noexcept {
+void BlockCache::give(void* ptr, size_t capacity, int device, bool known_idle) noexcept {
   int prev = device;
   const bool keep = capacity >= kMinBlock && capacity <= kLimit && cudaGetDevice(&prev) == cudaSuccess &&
                     (prev == device || cudaSetDevice(device) == cudaSuccess);
   bool kept = false;
-  const bool idle = keep && wait_for_device();
+  const bool idle = keep && (known_idle || wait_for_device());
   if (keep && !idle) cudaGetLastError();  // not the next launch's error
   if (idle) {
     std::vector<void*> out;
@@ -439,8 +439,8 @@ int tq_index_prepare(tq_index* h) {
     h->reserve_scratch();
     h->sync();
     h->staged_n = 0;
-    h->d_staged.release();
-    h->d_flat.release();
+    h->d_staged.release(true);  // adds and this call waited for their uses
+    h->d_flat.release(true);
     h->prepared = true;
   });
 }

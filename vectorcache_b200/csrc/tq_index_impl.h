@@ -83,7 +83,10 @@ class BlockCache {
   static BlockCache& get();
   // A block of at least `bytes` on the current device; *capacity and *device say what it is.
   void* take(size_t bytes, size_t* capacity, int* device);
-  void give(void* ptr, size_t capacity, int device) noexcept;
+  // known_idle: the caller has waited for the block's uses.
+  void give(void* ptr, size_t capacity, int device, bool known_idle) noexcept;
+  // Waits for the current device's queued work; about 10 us on an idle one.
+  static bool wait_for_device() noexcept;
   void trim() noexcept;
 
  private:
@@ -143,8 +146,8 @@ class DeviceBuffer {
     bytes_ = bytes;
     return ptr_;
   }
-  void release() {
-    if (ptr_ && !arena_) BlockCache::get().give(ptr_, capacity_, device_);
+  void release(bool known_idle = false) {
+    if (ptr_ && !arena_) BlockCache::get().give(ptr_, capacity_, device_, known_idle);
     ptr_ = nullptr;
     bytes_ = 0;
   }
@@ -279,6 +282,15 @@ struct tq_index {
       cudaEventDestroy(t.stop);
     }
     for (auto e : event_pool) cudaEventDestroy(e);
+    // One wait for all of them (searches may be queued on other streams).
+    if (vcb::BlockCache::wait_for_device()) {
+      for (vcb::DeviceBuffer* b : {&d_codes, &d_alpha, &d_staged, &d_flat, &d_queries, &d_luts, &d_qf, &d_cand_s,
+                                   &d_cand_i, &d_out_s, &d_out_i, &d_qrot, &d_partial, &d_onehot}) {
+        b->release(true);
+      }
+    } else {
+      cudaGetLastError();  // each buffer then waits, or frees, for itself
+    }
   }
 
   cudaEvent_t take_event() {
